@@ -306,56 +306,392 @@ __device__ bool decode_block(const uint8_t* src, uint32_t n, uint8_t* dst, uint6
   return true;
 }
 
-__global__ void __launch_bounds__(kWarps * 32) k_lz4_decode(const Lz4Frame* __restrict__ frames, uint32_t n_frames,
-                                                            int32_t* err) {
-  const uint32_t warp = blockIdx.x * kWarps + (threadIdx.x >> 5);
-  for (uint32_t fi = warp; fi < n_frames; fi += gridDim.x * kWarps) {
-    const Lz4Frame fr = frames[fi];
-    const uint8_t* s = fr.src;
-    const uint64_t n = fr.src_len;
-    bool ok = n >= 7 && le32(s) == 0x184D2204u;
-    uint64_t pos = 0, o = 0;
-    bool block_sum = false, content_sum = false;
-    if (ok) {
-      const uint8_t flg = s[4], bd = s[5];
-      block_sum = flg & 0x10;
-      content_sum = flg & 0x04;
-      pos = 6 + ((flg & 0x08) ? 8 : 0) + ((flg & 0x01) ? 4 : 0);
-      ok = (flg >> 6) == 1 && (bd & 0x8F) == 0 && n > pos &&
-           s[pos] == (uint8_t)((xxh32_short(s + 4, (uint32_t)(pos - 4)) >> 8) & 0xFF);
-      pos++;
-    }
-    while (ok) {
-      if (n - pos < 4) {
-        ok = false;
-        break;
-      }
-      const uint32_t bs = le32(s + pos);
-      pos += 4;
-      if (bs == 0) break;  // end mark
-      const uint32_t sz = bs & 0x7FFFFFFFu;
-      if (sz > n - pos || (block_sum && n - pos - sz < 4)) {
-        ok = false;
-        break;
-      }
-      if (bs & 0x80000000u) {  // stored
-        if (sz > fr.dst_len - o) {
-          ok = false;
-          break;
+// ---- frames decoded block by block ---------------------------------------------------------
+// A block is a serial chain (each token says where the next one is, each match may copy what the
+// last one wrote).  One warp per frame followed it from global memory: 5.3 ms for a map output of
+// three wide record batches (100 frames, 1.4 MB decoded), most SMs idle; one warp per block, staged
+// in shared memory: 261 us, still the chain (about 1000 sequences of 500 cycles).  The frames the
+// splitter writes hold independent blocks of at most kLz4MaxBlock bytes, so here
+//   k_lz4_blocks  gives every block a CTA that follows no chain: where the next token would be is
+//                 computed for every byte position at once, the positions reached from the first
+//                 are marked by pointer doubling (about ten rounds), the sequences' sizes are
+//                 scanned, and every output byte's source is followed to a literal by pointer
+//                 jumping.  Bound by instruction issue and shared memory (43 KiB: five CTAs per SM).
+//                 Where a block's bytes go depends on the sizes of the blocks before it, so they
+//                 go to a slot of their own
+//   k_lz4_place   adds up the sizes and moves slots (and stored blocks) to their place
+// A frame that is anything else (blocks that reach back into earlier ones, larger blocks, more
+// blocks than slots, malformed) is decoded as a whole by one warp of k_lz4_place.
+constexpr uint32_t kNoSlot = 0xffffffffu;      // the block cannot be decoded on its own
+constexpr int kDT = 256;                       // threads per block
+constexpr int kPer = kLz4MaxBlock / kDT;       // byte positions per thread
+constexpr uint32_t kInStage = kLz4MaxBlock + 64;   // + the phase of its first byte
+constexpr uint32_t kMaxSeq = kLz4MaxBlock / 4 + 1; // every match yields four bytes or more
+constexpr uint32_t kSeqRoom = (kMaxSeq + 1 + 7) & ~7u;
+constexpr uint32_t kPtrRoom = kLz4MaxBlock + 2 * (kLz4MaxBlock / 32);
+constexpr size_t kDecodeSmem = kInStage + 2 * kPtrRoom + 4 * 2 * kSeqRoom;
+static_assert(kLz4MaxBlock == kDT * 32, "a mark word per thread");
+static_assert(kDecodeSmem <= 46 * 1024, "five CTAs per SM, no opt-in");
+// index of output byte o in the pointer array: a thread's 32 bytes start in a bank of their own
+__device__ __forceinline__ uint32_t swz(uint32_t o) { return o + 2 * (o >> 5); }
+
+// Reads and checks a frame's header; false when malformed.  *pos: its first block.
+__device__ bool frame_header(const uint8_t* s, uint64_t n, uint64_t* pos, bool* block_sum, bool* content_sum) {
+  if (n < 7 || le32(s) != 0x184D2204u) return false;
+  const uint8_t flg = s[4], bd = s[5];
+  *block_sum = flg & 0x10;
+  *content_sum = flg & 0x04;
+  const uint64_t p = 6 + ((flg & 0x08) ? 8 : 0) + ((flg & 0x01) ? 4 : 0);
+  if (!((flg >> 6) == 1 && (bd & 0x8F) == 0 && n > p && s[p] == (uint8_t)((xxh32_short(s + 4, (uint32_t)(p - 4)) >> 8) & 0xFF)))
+    return false;
+  *pos = p + 1;
+  return true;
+}
+
+// The sequence at position `at` of the staged block in[0, n): its literals, and its match (ml 0:
+// the block ends with the literals).  Returns the position after it, or kNoSlot when it is cut off or
+// longer than `cap`.
+__device__ __forceinline__ uint32_t parse_seq(const uint8_t* in, uint32_t n, uint32_t cap, uint32_t at, uint32_t* lit,
+                                              uint32_t* lpos, uint32_t* ml) {
+  const uint32_t token = in[at];
+  uint32_t p = at + 1, l = token >> 4, b;
+  if (l == 15) {
+    do {
+      if (p >= n) return kNoSlot;
+      b = in[p++];
+      l += b;
+    } while (b == 255 && l <= cap);
+  }
+  if (l > n - p || l > cap) return kNoSlot;
+  *lit = l;
+  *lpos = p;
+  *ml = 0;
+  p += l;
+  if (p == n) return p;
+  if (n - p < 2) return kNoSlot;
+  p += 2;
+  uint32_t m = token & 15;
+  if (m == 15) {
+    do {
+      if (p >= n) return kNoSlot;
+      b = in[p++];
+      m += b;
+    } while (b == 255 && m <= cap);
+  }
+  if (m + 4 > cap) return kNoSlot;
+  *ml = m + 4;
+  return p;
+}
+
+// Exclusive scan of x over the CTA; *total gets the sum.
+__device__ __forceinline__ uint32_t cta_exscan(uint32_t x, uint32_t* warp_sum, uint32_t* total) {
+  uint32_t inc = x;
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t y = __shfl_up_sync(kFull, inc, o);
+    if (lane_id() >= o) inc += y;
+  }
+  __syncthreads();  // earlier reads of warp_sum
+  if (lane_id() == 31) warp_sum[threadIdx.x >> 5] = inc;
+  __syncthreads();
+  uint32_t before = 0, all = 0;
+  for (int w = 0; w < kDT / 32; w++) {
+    const uint32_t v = warp_sum[w];
+    if (w < (int)(threadIdx.x >> 5)) before += v;
+    all += v;
+  }
+  *total = all;
+  return before + inc - x;
+}
+
+// Decodes the block staged at `in` (n >= 1 bytes) on its own, by the whole CTA, into `out` (global,
+// 16-byte aligned, room for cap bytes rounded up to 16); returns its size, or kNoSlot when it is
+// malformed, longer than `cap` or reaches back before its first byte.
+__device__ uint32_t decode_staged(const uint8_t* in, uint32_t n, uint32_t cap, uint16_t* ptr, uint16_t* seq,
+                                  uint32_t* marks, uint32_t* warp_sum, uint8_t* out) {
+  const uint32_t t = threadIdx.x;
+  uint16_t* start = seq;                 // first output byte of each sequence
+  uint16_t* mst = seq + kSeqRoom;        // its first match byte
+  uint16_t* lpos = seq + 2 * kSeqRoom;   // its literals in the input
+  uint16_t* offs = seq + 3 * kSeqRoom;   // its match offset
+  uint32_t lit, lp, ml;
+  // where a sequence at each position would end: n the block's end, 0xffff nowhere
+  uint16_t* J = ptr;
+  for (uint32_t q = t; q < n; q += kDT) J[q] = (uint16_t)parse_seq(in, n, cap, q, &lit, &lp, &ml);
+  marks[t] = t == 0 ? 1u : 0u;
+  __syncthreads();
+  // J jumps 2^r sequences and the first 2^r are marked: until the first one's jump ends the block
+  while (J[0] < n) {
+    uint32_t nj[kPer / 2];
+#pragma unroll
+    for (int j = 0; j < kPer; j++) {
+      const uint32_t q = j * kDT + t;
+      if (j * kDT >= (int)n) break;
+      uint32_t v = 0;
+      if (q < n) {
+        v = J[q];
+        if (v < n) {
+          if ((marks[q >> 5] >> (q & 31)) & 1u) atomicOr(&marks[v >> 5], 1u << (v & 31));
+          v = J[v];
         }
-        for (uint32_t i = lane_id(); i < sz; i += 32) fr.dst[o + i] = s[pos + i];
-        o += sz;
-      } else {
-        ok = decode_block(s + pos, sz, fr.dst, fr.dst_len, &o);
       }
-      pos += sz + (block_sum ? 4 : 0);
-      __syncwarp();
+      if (j & 1) nj[j >> 1] |= v << 16;
+      else nj[j >> 1] = v;
     }
-    // (content checksums are skipped, not verified)
-    if (ok && content_sum && n - pos < 4) ok = false;
-    if (!(ok && o == fr.dst_len) && lane_id() == 0) atomicOr(err, 1);
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < kPer; j++) {
+      const uint32_t q = j * kDT + t;
+      if (j * kDT >= (int)n) break;
+      if (q < n) J[q] = (uint16_t)(nj[j >> 1] >> (16 * (j & 1)));
+    }
+    __syncthreads();
+  }
+  if (J[0] != n) return kNoSlot;
+  // the marked positions in order
+  uint32_t nseq, total;
+  uint32_t k = cta_exscan(__popc(marks[t]), warp_sum, &nseq);
+  if (nseq > kMaxSeq) return kNoSlot;
+  for (uint32_t m = marks[t]; m; m &= m - 1) lpos[k++] = (uint16_t)(32 * t + __ffs(m) - 1);
+  __syncthreads();
+  // sizes, output starts, offsets: a thread takes sequences [k0, k1)
+  const uint32_t per = (nseq + kDT - 1) / kDT;
+  const uint32_t k0 = min(nseq, t * per), k1 = min(nseq, k0 + per);
+  uint32_t sum = 0;
+  for (k = k0; k < k1; k++) {
+    parse_seq(in, n, cap, lpos[k], &lit, &lp, &ml);
+    lpos[k] = (uint16_t)lp;
+    start[k] = (uint16_t)(lit + ml);  // at most 2 * cap
+    mst[k] = (uint16_t)lit;
+    offs[k] = ml ? (uint16_t)((uint32_t)in[lp + lit] | (uint32_t)in[lp + lit + 1] << 8) : (uint16_t)0;
+    sum += lit + ml;
+  }
+  uint32_t o = cta_exscan(sum, warp_sum, &total);
+  if (total > cap) return kNoSlot;
+  bool bad = false;
+  for (k = k0; k < k1; k++) {
+    const uint32_t len = start[k], l = mst[k];
+    start[k] = (uint16_t)o;
+    mst[k] = (uint16_t)(o + l);
+    if (len > l) bad |= offs[k] == 0 || offs[k] > o + l;
+    o += len;
+  }
+  if (t == 0) start[nseq] = (uint16_t)total;
+  if (__syncthreads_or(bad)) return kNoSlot;
+  // every output byte's source: a literal (bit 15 and its input position) or an earlier output byte
+  {
+    const uint32_t o0 = 32 * t, o1 = min(total, o0 + 32);
+    if (o0 < o1) {
+      uint32_t lo = 0, hi = nseq;  // start[lo] <= o0 < start[hi]
+      while (hi - lo > 1) {
+        const uint32_t mid = (lo + hi) >> 1;
+        if (start[mid] <= o0) lo = mid;
+        else hi = mid;
+      }
+      uint32_t s0 = start[lo], s1 = start[lo + 1], m0 = mst[lo], l0 = lpos[lo], f0 = offs[lo];
+      for (o = o0; o < o1; o++) {
+        while (o >= s1) {
+          lo++;
+          s0 = s1;
+          s1 = start[lo + 1];
+          m0 = mst[lo];
+          l0 = lpos[lo];
+          f0 = offs[lo];
+        }
+        uint32_t v;
+        if (o < m0) {
+          v = 0x8000u | (l0 + o - s0);
+        } else {
+          // byte d of a match repeats byte d mod offset of its source run
+          uint32_t d = o - m0;
+          if (d >= f0) d %= f0;
+          v = m0 - f0 + d;
+        }
+        ptr[swz(o)] = (uint16_t)v;
+      }
+    }
+  }
+  __syncthreads();
+  // every source followed to its literal (a pointer read while its owner moves it on is an
+  // earlier one of the same chain: still right)
+  for (;;) {
+    bool more = false;
+    for (uint32_t q = t; q < total; q += kDT) {
+      uint32_t v = ptr[swz(q)];
+      if (!(v & 0x8000u)) {
+        v = ptr[swz(v)];
+        ptr[swz(q)] = (uint16_t)v;
+        more |= !(v & 0x8000u);
+      }
+    }
+    if (!__syncthreads_or(more)) break;
+  }
+  for (uint32_t w = t; w < (total + 3) >> 2; w += kDT) {
+    // (bytes past the end come from whatever the array holds there, an index inside the stage)
+    const uint32_t i = swz(4 * w);
+    const uint32_t a = *reinterpret_cast<const uint32_t*>(ptr + i), b = *reinterpret_cast<const uint32_t*>(ptr + i + 2);
+    const uint32_t x = in[a & 0x1fff] | (uint32_t)in[(a >> 16) & 0x1fff] << 8 | (uint32_t)in[b & 0x1fff] << 16 |
+                       (uint32_t)in[(b >> 16) & 0x1fff] << 24;
+    reinterpret_cast<uint32_t*>(out)[w] = x;
+  }
+  return total;
+}
+
+// One CTA per (frame, block ordinal): block `i` of frame `fi` into slot frames[fi].slot0 + i.
+__global__ void __launch_bounds__(kDT, 5) k_lz4_blocks(const Lz4Frame* __restrict__ frames, const uint32_t* __restrict__ frame_of,
+                                                       Lz4Slot* __restrict__ slots, uint8_t* __restrict__ slot_mem) {
+  extern __shared__ __align__(16) uint8_t dsm[];
+  __shared__ uint32_t marks[kDT];
+  __shared__ uint32_t warp_sum[kDT / 32];
+  const uint32_t g = blockIdx.x;
+  const Lz4Frame fr = frames[frame_of[g]];
+  const uint32_t i = g - fr.slot0;
+  const uint8_t* s = fr.src;
+  const uint64_t n = fr.src_len;
+  Lz4Slot sl{0, 0, kNoSlot, 0};  // a bad frame, or a block that cannot be decoded on its own
+  uint64_t pos = 0;
+  bool block_sum = false, content_sum = false;
+  bool ok = n < (1ull << 31) && frame_header(s, n, &pos, &block_sum, &content_sum);
+  uint32_t sz = 0;
+  bool stored = false;
+  for (uint32_t b = 0; ok; b++) {  // (every thread walks the headers: uniform loads)
+    if (n - pos < 4) {
+      ok = false;
+      break;
+    }
+    const uint32_t bs = le32(s + pos);
+    pos += 4;
+    if (bs == 0) {  // end mark: fewer than i + 1 blocks
+      sl.size = 0;
+      sl.state = 1;
+      ok = false;
+      break;
+    }
+    sz = bs & 0x7FFFFFFFu;
+    stored = bs & 0x80000000u;
+    if (sz > n - pos || (block_sum && n - pos - sz < 4)) {
+      ok = false;
+      break;
+    }
+    if (b == i) break;
+    pos += sz + (block_sum ? 4 : 0);
+  }
+  if (ok && i + 1 == fr.n_slots) {  // the last slot: the end mark must follow
+    const uint64_t after = pos + sz + (block_sum ? 4 : 0);
+    if (n - after < 4 || le32(s + after) != 0) ok = false;
+  }
+  if (ok) {
+    sl.pos = (uint32_t)pos;
+    if (stored) {
+      sl.size = sz;
+      sl.state = 2;
+    } else if (sz > 0 && sz <= kLz4MaxBlock) {
+      // the aligned 16-byte words that hold the block (they stay inside the stream's allocation)
+      const uint8_t* src = s + pos;
+      const uint32_t phase = (uint32_t)(reinterpret_cast<uintptr_t>(src) & 15);
+      const uint4* a = reinterpret_cast<const uint4*>(src - phase);
+      const uint32_t nw = (phase + sz + 15) >> 4;
+      for (uint32_t q = threadIdx.x; q < nw; q += kDT) reinterpret_cast<uint4*>(dsm)[q] = __ldg(a + q);
+      __syncthreads();
+      const uint32_t slot = lz4_slot_bytes(fr.dst_len);
+      uint16_t* ptr = reinterpret_cast<uint16_t*>(dsm + kInStage);
+      sl.size = decode_staged(dsm + phase, sz, slot, ptr, ptr + kPtrRoom, marks, warp_sum,
+                              slot_mem + fr.mem0 + (size_t)i * slot);
+      if (sl.size != kNoSlot) sl.state = 3;
+    }
+  }
+  if (threadIdx.x == 0) slots[g] = sl;
+}
+
+// n bytes from src to dst by one warp, in aligned 16- or 4-byte words of dst.
+__device__ void warp_copy(uint8_t* dst, const uint8_t* src, uint32_t n) {
+  const uint32_t lane = lane_id();
+  const uint32_t W = ((reinterpret_cast<uintptr_t>(src) ^ reinterpret_cast<uintptr_t>(dst)) & 15) == 0 ? 16u : 4u;
+  const uint32_t head = min(n, (uint32_t)(-reinterpret_cast<intptr_t>(dst) & (W - 1)));
+  if (lane < head) dst[lane] = src[lane];
+  dst += head;
+  src += head;
+  n -= head;
+  const uint32_t nv = n / W;
+  if (W == 16) {
+    const uint4* a = reinterpret_cast<const uint4*>(src);
+#pragma unroll 8
+    for (uint32_t q = lane; q < nv; q += 32) reinterpret_cast<uint4*>(dst)[q] = __ldg(a + q);
+  } else {
+    // a funnel shift of two aligned source words, each holding bytes of [src, src + n)
+    const uint32_t sh = (uint32_t)(reinterpret_cast<uintptr_t>(src) & 3) * 8;
+    const uint32_t* a = reinterpret_cast<const uint32_t*>(src - (sh >> 3));
+    const uint32_t up = sh ? 1u : 0u;
+#pragma unroll 8
+    for (uint32_t q = lane; q < nv; q += 32)
+      reinterpret_cast<uint32_t*>(dst)[q] = __funnelshift_r(__ldg(a + q), __ldg(a + q + up), sh);
+  }
+  for (uint32_t q = nv * W + lane; q < n; q += 32) dst[q] = src[q];
+}
+
+// The whole frame by one warp, its blocks in order (matches may reach back into earlier ones).
+__device__ bool decode_frame(const Lz4Frame& fr) {
+  const uint8_t* s = fr.src;
+  const uint64_t n = fr.src_len;
+  uint64_t pos = 0, o = 0;
+  bool block_sum = false, content_sum = false;
+  bool ok = frame_header(s, n, &pos, &block_sum, &content_sum);
+  while (ok) {
+    if (n - pos < 4) return false;
+    const uint32_t bs = le32(s + pos);
+    pos += 4;
+    if (bs == 0) break;  // end mark
+    const uint32_t sz = bs & 0x7FFFFFFFu;
+    if (sz > n - pos || (block_sum && n - pos - sz < 4)) return false;
+    if (bs & 0x80000000u) {  // stored
+      if (sz > fr.dst_len - o) return false;
+      for (uint32_t i = lane_id(); i < sz; i += 32) fr.dst[o + i] = s[pos + i];
+      o += sz;
+    } else {
+      ok = decode_block(s + pos, sz, fr.dst, fr.dst_len, &o);
+    }
+    pos += sz + (block_sum ? 4 : 0);
     __syncwarp();
   }
+  // (content checksums are skipped, not verified)
+  if (ok && content_sum && n - pos < 4) ok = false;
+  return ok && o == fr.dst_len;
+}
+
+__global__ void __launch_bounds__(kWarps * 32) k_lz4_place(const Lz4Frame* __restrict__ frames,
+                                                           const uint32_t* __restrict__ frame_of, uint32_t n_slots,
+                                                           const Lz4Slot* __restrict__ slots,
+                                                           const uint8_t* __restrict__ slot_mem, int32_t* err) {
+  const uint32_t g = blockIdx.x * kWarps + (threadIdx.x >> 5);
+  if (g >= n_slots) return;
+  const uint32_t lane = lane_id();
+  const Lz4Frame fr = frames[frame_of[g]];
+  const uint32_t i = g - fr.slot0;
+  // the frame's blocks: any that could not be decoded on its own, their sizes before this one
+  uint64_t before = 0, total = 0;
+  bool bad = false;
+  for (uint32_t q0 = 0; q0 < fr.n_slots; q0 += 32) {
+    const uint32_t q = q0 + lane;
+    const uint32_t sz = q < fr.n_slots ? slots[fr.slot0 + q].size : 0u;
+    bad |= __any_sync(kFull, sz == kNoSlot);
+    uint64_t t = sz, p = q < i ? sz : 0u;
+    for (int x = 16; x; x >>= 1) {
+      t += __shfl_xor_sync(kFull, t, x);
+      p += __shfl_xor_sync(kFull, p, x);
+    }
+    total += t;
+    before += p;
+  }
+  bad = bad || total != fr.dst_len;
+  // a frame with a content checksum is checked for it by decode_frame
+  if (bad || (fr.src_len > 4 && (fr.src[4] & 0x04))) {
+    if (i != 0) return;
+    const bool ok = decode_frame(fr);
+    if (!ok && lane == 0) atomicOr(err, 1);
+    return;
+  }
+  const Lz4Slot sl = slots[g];
+  if (sl.state == 2) warp_copy(fr.dst + before, fr.src + sl.pos, sl.size);
+  else if (sl.state == 3) warp_copy(fr.dst + before, slot_mem + fr.mem0 + (size_t)i * lz4_slot_bytes(fr.dst_len), sl.size);
 }
 
 int sm_count() {
@@ -387,11 +723,13 @@ cudaError_t launch_lz4_compress(const Lz4Chunk* chunks, uint32_t n_chunks, uint3
   return cudaGetLastError();
 }
 
-cudaError_t launch_lz4_decode(const Lz4Frame* frames, uint32_t n_frames, int32_t* err, cudaStream_t st) {
-  if (n_frames == 0) return cudaSuccess;
-  const uint32_t need = (n_frames + kWarps - 1) / kWarps;
-  const uint32_t cap = (uint32_t)sm_count() * 16;
-  k_lz4_decode<<<need < cap ? need : cap, kWarps * 32, 0, st>>>(frames, n_frames, err);
+cudaError_t launch_lz4_decode(const Lz4Frame* frames, const uint32_t* frame_of, uint32_t n_slots, Lz4Slot* slots,
+                              uint8_t* slot_mem, int32_t* err, cudaStream_t st) {
+  if (n_slots == 0) return cudaSuccess;
+  k_lz4_blocks<<<n_slots, kDT, kDecodeSmem, st>>>(frames, frame_of, slots, slot_mem);
+  const cudaError_t e = cudaGetLastError();
+  if (e != cudaSuccess) return e;
+  k_lz4_place<<<(n_slots + kWarps - 1) / kWarps, kWarps * 32, 0, st>>>(frames, frame_of, n_slots, slots, slot_mem, err);
   return cudaGetLastError();
 }
 

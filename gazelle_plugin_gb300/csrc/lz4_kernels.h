@@ -26,7 +26,24 @@ struct Lz4Frame {  // one frame to decode: src_len bytes into exactly dst_len by
   uint64_t src_len;
   uint8_t* dst;
   uint64_t dst_len;
+  uint32_t slot0;    // its first block slot
+  uint32_t n_slots;  // its slots (lz4_frame_slots)
+  uint64_t mem0;     // where the slots' memory starts (lz4_slot_bytes each)
 };
+
+struct Lz4Slot {  // one block of a frame
+  uint32_t pos;    // its payload inside the frame
+  uint32_t pad;
+  uint32_t size;   // decoded bytes, or 0xffffffff: not decodable on its own
+  uint32_t state;  // 0: see size, 1: no such block, 2: stored, 3: decoded into its slot
+};
+
+// Block slots for a frame of dst_len bytes: blocks of kLz4MaxBlock bytes, and three shorter ones
+// inside it (an offsets buffer starts with its own first offset, a batch may continue from an
+// earlier device pass); a frame with more blocks is decoded by one warp.
+inline uint32_t lz4_frame_slots(uint64_t dst_len) {
+  return (uint32_t)((dst_len + kLz4MaxBlock - 1) / kLz4MaxBlock) + 3;
+}
 
 // Warps of the compression grid (each needs kLz4Slot bytes of scratch).
 uint32_t lz4_compress_warps();
@@ -38,7 +55,19 @@ cudaError_t launch_lz4_compress(const Lz4Chunk* chunks, uint32_t n_chunks, uint3
                                 uint8_t* out, unsigned long long* out_used, unsigned long long out_cap,
                                 Lz4Block* res, int32_t* err, cudaStream_t st);
 
-// Decodes every frame; *err gets bit 0 for a malformed frame or a size that differs.
-cudaError_t launch_lz4_decode(const Lz4Frame* frames, uint32_t n_frames, int32_t* err, cudaStream_t st);
+// Memory of one block slot of a frame of dst_len bytes (16-byte units; no block is longer).
+#ifdef __CUDACC__
+__host__ __device__
+#endif
+inline uint32_t lz4_slot_bytes(uint64_t dst_len) {
+  return dst_len < kLz4MaxBlock ? ((uint32_t)dst_len + 15u) & ~15u : kLz4MaxBlock;
+}
+
+// Decodes every frame; *err gets bit 0 for a malformed frame or a size that differs.  frame_of[g]:
+// the frame of slot g (n_slots of them, every frame's in a row); `slots` and `slot_mem`
+// are scratch.  The sources' allocations start and end on 16-byte
+// boundaries.
+cudaError_t launch_lz4_decode(const Lz4Frame* frames, const uint32_t* frame_of, uint32_t n_slots, Lz4Slot* slots,
+                              uint8_t* slot_mem, int32_t* err, cudaStream_t st);
 
 }  // namespace gz

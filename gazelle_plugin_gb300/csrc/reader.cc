@@ -358,26 +358,46 @@ Status PartitionReader::AddStream(const uint8_t* data, int64_t len) {
   }
   images_.push_back(d);
   arenas_.push_back(nullptr);
-  if (!frames.empty()) {
-    // compressed buffers: every LZ4 frame decoded by the device into the stream's arena
+  if (!frames.empty() && d != nullptr) {  // (batches without rows leave no image)
+    // compressed buffers: every LZ4 frame decoded by the device into the stream's arena; the
+    // jobs, the frame of every block slot, the error word and the slots lie in front of it
     std::vector<Lz4Frame> jobs;
-    for (const FrameRef& f : frames)
-      jobs.push_back(Lz4Frame{nullptr, (uint64_t)f.src_len, nullptr, (uint64_t)f.dst_len});
-    const size_t jb = AlignUp(sizeof(Lz4Frame) * jobs.size(), 256);
-    st = Cuda(cudaMallocAsync(reinterpret_cast<void**>(&arena), jb + 256 + AlignUp((size_t)arena_bytes, 256), stream_),
+    std::vector<uint32_t> frame_of;
+    size_t slot_bytes = 0;
+    for (const FrameRef& f : frames) {
+      const uint32_t ns = lz4_frame_slots((uint64_t)f.dst_len);
+      jobs.push_back(Lz4Frame{nullptr, (uint64_t)f.src_len, nullptr, (uint64_t)f.dst_len, (uint32_t)frame_of.size(), ns,
+                              slot_bytes});
+      slot_bytes += (size_t)ns * lz4_slot_bytes((uint64_t)f.dst_len);
+      frame_of.resize(frame_of.size() + ns, (uint32_t)jobs.size() - 1);
+    }
+    const size_t jb = AlignUp(sizeof(Lz4Frame) * jobs.size(), 256), fb = AlignUp(4 * frame_of.size(), 256),
+                 sb = AlignUp(sizeof(Lz4Slot) * frame_of.size(), 256);
+    const size_t head = jb + fb + 256 + sb;
+    st = Cuda(cudaMallocAsync(reinterpret_cast<void**>(&arena), head + AlignUp((size_t)arena_bytes, 256), stream_),
               "cudaMallocAsync(decode)");
     if (!st.ok()) return st;
-    arenas_.back() = arena + jb + 256;
+    uint8_t* slot_mem = nullptr;
+    st = Cuda(cudaMallocAsync(reinterpret_cast<void**>(&slot_mem), std::max<size_t>(slot_bytes, 256), stream_),
+              "cudaMallocAsync(decode)");
+    if (!st.ok()) return st;
+    arenas_.back() = arena + head;
     for (size_t i = 0; i < jobs.size(); i++) {
       jobs[i].src = d + frames[i].src;
       jobs[i].dst = arenas_.back() + frames[i].dst;
     }
-    int32_t* d_err = reinterpret_cast<int32_t*>(arena + jb);
+    std::vector<uint8_t> up(jb + fb + 4, 0);  // with the error word, zero
+    memcpy(up.data(), jobs.data(), sizeof(Lz4Frame) * jobs.size());
+    memcpy(up.data() + jb, frame_of.data(), 4 * frame_of.size());
+    int32_t* d_err = reinterpret_cast<int32_t*>(arena + jb + fb);
     int32_t err = 0;
-    st = Cuda(cudaMemcpyAsync(arena, jobs.data(), sizeof(Lz4Frame) * jobs.size(), cudaMemcpyHostToDevice, stream_), "H2D");
-    if (st.ok()) st = Cuda(cudaMemsetAsync(d_err, 0, 4, stream_), "memset");
-    if (st.ok()) st = Cuda(launch_lz4_decode(reinterpret_cast<const Lz4Frame*>(arena), (uint32_t)jobs.size(), d_err, stream_),
-                           "k_lz4_decode");
+    st = Cuda(cudaMemcpyAsync(arena, up.data(), up.size(), cudaMemcpyHostToDevice, stream_), "H2D");
+    if (st.ok())
+      st = Cuda(launch_lz4_decode(reinterpret_cast<const Lz4Frame*>(arena), reinterpret_cast<const uint32_t*>(arena + jb),
+                                  (uint32_t)frame_of.size(), reinterpret_cast<Lz4Slot*>(arena + jb + fb + 256), slot_mem,
+                                  d_err, stream_),
+                "k_lz4_blocks");
+    cudaFreeAsync(slot_mem, stream_);
     if (st.ok()) st = Cuda(cudaMemcpyAsync(&err, d_err, 4, cudaMemcpyDeviceToHost, stream_), "D2H");
     // the decoded offsets bound each batch's characters (and a nested node's child entries): for
     // each, the 4-byte words of its first and last offset (low word, then high word of a 64-bit one)
@@ -411,7 +431,7 @@ Status PartitionReader::AddStream(const uint8_t* data, int64_t len) {
         }
     std::vector<int32_t> ends(where.size());
     if (st.ok() && !where.empty()) st = Cuda(gather_words(where.data(), ends.data(), where.size(), stream_), "offsets");
-    if (st.ok()) st = Cuda(cudaStreamSynchronize(stream_), "k_lz4_decode");
+    if (st.ok()) st = Cuda(cudaStreamSynchronize(stream_), "k_lz4_place");
     if (!st.ok()) return st;
     if (err) return Status::Error(GZ_INVALID, "a compressed buffer is not a valid LZ4 frame of its stated length");
     size_t e = 0;

@@ -176,3 +176,122 @@ def test_gpu_compressed_size_of_first_batch():
     body = len(data) - 8 - 8 - meta_len  # continuation + length prefix, EOS at the end
     assert R.batches_compressed(data) == [True]
     assert abs(cs_lz4 - body) <= 0.01 * body + 64
+
+
+def _lz4_block(rng, n, lits, mls, offs, history=b""):
+    """A random LZ4 block of `n` decoded bytes and those bytes: sequences of literal lengths drawn from
+    `lits`, match lengths from `mls` and offsets from `offs` (clipped to what precedes, `history`
+    included), a literal tail."""
+    out, blk = bytearray(history), bytearray()
+    base = len(history)
+
+    def ext(x):
+        return b"" if x < 15 else b"\xff" * ((x - 15) // 255) + bytes([(x - 15) % 255])
+
+    while True:
+        lit, ml = int(rng.choice(lits)), int(rng.choice(mls))
+        if len(out) == 0:
+            lit = max(lit, 1)
+        if len(out) - base + lit + ml + 5 > n:
+            break
+        data = rng.integers(0, 256, lit, dtype=np.uint8).tobytes()
+        off = min(int(rng.choice(offs)), len(out) + lit)
+        blk += bytes([(min(lit, 15) << 4) | min(ml - 4, 15)]) + ext(lit) + data + off.to_bytes(2, "little") + ext(ml - 4)
+        out += data
+        for _ in range(ml):
+            out.append(out[-off])
+    lit = n - (len(out) - base)
+    data = rng.integers(0, 256, lit, dtype=np.uint8).tobytes()
+    blk += bytes([min(lit, 15) << 4]) + ext(lit) + data
+    return bytes(blk), bytes(out[base:]) + data
+
+
+def _lz4_frame(blocks):
+    """Frame of (payload, stored) blocks, as the splitter's frames are: independent blocks, no checksums."""
+    f = b"\x04\x22\x4d\x18\x60\x40" + bytes([(O.xxh32(b"\x60\x40") >> 8) & 255])
+    for b, stored in blocks:
+        f += (len(b) | (0x80000000 if stored else 0)).to_bytes(4, "little") + b
+    return f + bytes(4)
+
+
+def _read_values_frame(frame, n):
+    """The reader's value bytes of an int64 column of n bytes whose values buffer is `frame` (put over
+    a longer frame of stored blocks; what follows a frame's end mark is not read)."""
+    from gazelle_plugin_gb300 import workloads as W
+    # the values' own bytes do not matter: they mark where the frame has to go
+    plain = np.frombuffer(b"\xa5" * n, np.uint8)
+    msg = bytearray(encode_lz4_stored(n // 8, [(n // 8, 0)], [np.zeros(0, np.uint8), plain]))
+    at = msg.index(b"\x04\x22\x4d\x18")
+    assert at + len(frame) <= len(msg)
+    msg[at:at + len(frame)] = frame
+    r = S.PartitionReader([W.Field("v", "int64", False)])
+    try:
+        r.addStream(bytes(msg))
+        r.finish()
+        return r.column_to_host(0)[2].tobytes()
+    finally:
+        r.close()
+
+
+FRAME_SHAPES = {
+    # sizes of the blocks, whether each is stored, and what their sequences look like
+    "short sequences": ([8192, 8192, 3000], "ccc", range(0, 6), range(4, 12), range(1, 4000)),
+    "overlapping matches": ([8192, 104], "cc", range(0, 3), range(4, 70), range(1, 40)),
+    "long lengths": ([8192, 8184], "cc", [0, 14, 15, 16, 269, 270, 271, 600], [4, 18, 19, 20, 273, 274, 900], range(1, 9000)),
+    "window edges": ([8192], "c", range(10, 18), range(14, 22), range(1, 300)),
+    "pieces of a spanning batch": ([4, 8192, 1001, 8192, 3], "scscs", range(0, 9), range(4, 30), range(1, 2000)),
+    "one short block": ([40], "c", range(0, 3), range(4, 6), range(1, 9)),
+    "more blocks than slots": ([96] * 40, "c" * 40, range(0, 3), range(4, 9), range(1, 90)),
+    "blocks over 8 KiB": ([20000, 65536], "cc", range(0, 9), range(4, 60), range(1, 65000)),
+    "blocks that reach back": ([8192, 8192, 800], "lll", range(0, 6), range(4, 30), range(1, 20000)),
+}
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("shape", list(FRAME_SHAPES))
+def test_gpu_decoder_frame_shapes(shape):
+    sizes, kinds, lits, mls, offs = FRAME_SHAPES[shape]
+    for seed in range(4):
+        rng = np.random.default_rng(seed)
+        want, blocks = b"", []
+        for n, kind in zip(sizes, kinds):
+            if kind == "s":
+                b = d = rng.integers(0, 256, n, dtype=np.uint8).tobytes()
+            else:
+                b, d = _lz4_block(rng, n, list(lits), list(mls), list(offs), want if kind == "l" else b"")
+            blocks.append((b, kind == "s"))
+            want += d
+        pad = -len(want) % 8
+        if pad:
+            want += bytes(pad)
+            blocks.append((bytes(pad), True))
+        frame = _lz4_frame(blocks)
+        assert O.lz4f_decompress(frame, len(want)) == want
+        assert _read_values_frame(frame, len(want)) == want
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("how", ["offset 0", "offset before the frame", "cut block", "short", "long", "no end mark", "header"])
+def test_gpu_decoder_malformed_frames(how):
+    n = 8192 + 800
+    rng = np.random.default_rng(3)
+    b1, d1 = _lz4_block(rng, 8192, [3], [6], [100])
+    b2, d2 = _lz4_block(rng, 800, [3], [6], [100])
+    if how == "offset 0":
+        b2 = b2[:4] + b"\x00\x00" + b2[6:]  # token, 3 literals, offset
+    elif how == "offset before the frame":
+        b1 = b1[:4] + b"\xff\xff" + b1[6:]
+    elif how == "cut block":
+        b2 = b2[:5]
+    elif how == "short":
+        b2 = _lz4_block(rng, 792, [3], [6], [100])[0]
+    elif how == "long":
+        b2 = _lz4_block(rng, 808, [3], [6], [100])[0]
+    frame = _lz4_frame([(b1, False), (b2, False)])
+    if how == "no end mark":
+        frame = frame[:-4] + (0x7fffffff).to_bytes(4, "little")
+    elif how == "header":
+        frame = frame[:6] + bytes([frame[6] ^ 1]) + frame[7:]
+    with pytest.raises(S.SplitterError) as e:
+        _read_values_frame(frame, n)
+    assert e.value.status == S.GZ_INVALID
