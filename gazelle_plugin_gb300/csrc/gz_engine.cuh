@@ -38,6 +38,21 @@ enum KeyKind : int32_t { KEY_I32 = 0, KEY_I64 = 1, KEY_I8 = 2, KEY_I16 = 3, KEY_
 enum Partitioner : int32_t { PART_HASH = 0, PART_RR = 1, PART_RANGE = 2 };
 enum ColKind : int32_t { COL_FIXED = 0, COL_BOOL = 1, COL_BINARY = 2 };
 
+// Spark pmod(h, P) from one 32-bit high product (64-bit products are the slow half of the integer
+// pipe): |h| <= 2^31, so with l = ceil(log2 P) and m = floor(2^(31 + l) / P) + 1 (below 2^32 for P > 1)
+// the quotient is (|h| * m) >> (31 + l) (Granlund & Montgomery, "Division by invariant integers using
+// multiplication", 1994, for 31-bit dividends; m * P - 2^(31 + l) is at most P, and equal to it only
+// for powers of two, where 2^31 divides as well).
+struct PmodDiv {
+  uint32_t P, m, shift;  // shift: l - 1
+};
+inline PmodDiv make_pmod(uint32_t P) {
+  uint32_t l = 0;
+  while ((uint64_t(1) << l) < P) l++;
+  if (P <= 1) return PmodDiv{1, 0, 0};
+  return PmodDiv{P, (uint32_t)((uint64_t(1) << (31 + l)) / P + 1), l - 1};
+}
+
 // Static description of the split, copied to the device once at make.
 struct SchemaDesc {
   int32_t P;
@@ -49,7 +64,8 @@ struct SchemaDesc {
   int32_t prefer_spill;
   int32_t partitioner;  // Partitioner
   uint64_t quirk_mask;  // array columns a with array_idx_[a] < fixed_width_col_cnt_ (splitter.cc:878-886)
-  uint64_t pmod_magic;  // floor((2^64 - 1) / P) + 1, for the pmod without a divide
+  uint64_t pmod_magic;  // floor((2^64 - 1) / P) + 1, for the round-robin selection's modulus
+  uint32_t pmod_m, pmod_shift;  // the hash's pmod (PmodDiv)
   int32_t key_col[kMaxKeys];
   int32_t key_kind[kMaxKeys];
   int32_t arr_col[kMaxCols];    // schema index of array column a

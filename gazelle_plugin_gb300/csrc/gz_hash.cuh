@@ -5,6 +5,8 @@
 #pragma once
 #include <stdint.h>
 
+#include "gz_engine.cuh"
+
 namespace gz {
 namespace hash {
 
@@ -56,17 +58,18 @@ __device__ __forceinline__ int32_t hash_bytes(const uint8_t* p, int32_t len, int
   return (int32_t)fmix32(h1, (uint32_t)len);
 }
 
-// Spark pmod(h, P) without a hardware divide: Lemire, Kaser & Kurz, "Faster remainder by
+// a mod d without a hardware divide, any 32-bit a: Lemire, Kaser & Kurz, "Faster remainder by
 // direct computation" (2019): a mod d = hi64((M * a) mod 2^64 * d) with M = floor(2^64-1 / d) + 1.
 __device__ __forceinline__ uint32_t fastmod_u32(uint32_t a, uint32_t d, unsigned long long M) {
   const unsigned long long low = M * (unsigned long long)a;
   return (uint32_t)__umul64hi(low, (unsigned long long)d);
 }
-__device__ __forceinline__ uint32_t fast_pmod(int32_t h, uint32_t P, unsigned long long M) {
-  if (P == 1) return 0;
-  if (h >= 0) return fastmod_u32((uint32_t)h, P, M);
-  const uint32_t r = fastmod_u32(0u - (uint32_t)h, P, M);
-  return r == 0 ? 0 : P - r;
+// Spark pmod(h, P).
+__device__ __forceinline__ uint32_t pmod_div(int32_t h, const PmodDiv& d) {
+  if (d.P == 1) return 0;
+  const uint32_t a = h < 0 ? 0u - (uint32_t)h : (uint32_t)h;
+  const uint32_t r = a - (__umulhi(a, d.m) >> d.shift) * d.P;
+  return h < 0 && r != 0 ? d.P - r : r;
 }
 
 __device__ __forceinline__ bool get_bit(const uint8_t* bits, uint32_t i) {

@@ -135,6 +135,7 @@ __global__ void __launch_bounds__(kHashThreads) k_hash_count(const SchemaDesc sd
   }
   __syncthreads();
   const unsigned long long M = sd.pmod_magic;
+  const PmodDiv pmod{(uint32_t)P, sd.pmod_m, sd.pmod_shift};
   const int part = sd.partitioner;
   bool bad = false;
   bool bad_pid = false;
@@ -230,7 +231,7 @@ __global__ void __launch_bounds__(kHashThreads) k_hash_count(const SchemaDesc sd
 #pragma unroll
   for (int u = 0; u < kHashRows; u++) {
     if (part == PART_HASH) {
-      p[u] = fast_pmod(h[u], (uint32_t)P, M);
+      p[u] = pmod_div(h[u], pmod);
     } else if (part == PART_RR) {
       // the selection runs on from row to row and batch to batch, wrapping at P
       p[u] = fastmod_u32(fd.rr_base + tile.frow0 + i0 + u, (uint32_t)P, M);

@@ -166,6 +166,9 @@ Status Splitter::Init(const std::string& short_name, std::vector<Field> fields, 
   sd_.prefer_spill = opts_.prefer_spill ? 1 : 0;
   sd_.partitioner = partitioner_;
   sd_.pmod_magic = P_ > 1 ? UINT64_MAX / (uint64_t)P_ + 1 : 0;
+  const PmodDiv pd = make_pmod((uint32_t)P_);
+  sd_.pmod_m = pd.m;
+  sd_.pmod_shift = pd.shift;
   for (int a = 0; a < n_array_; a++) {
     const int ci = array_idx_[a];
     if (a >= first_stream_) {  // a nested column's stream: list-like, rows from its slot

@@ -160,3 +160,55 @@ def test_static_scratch_rejects_oversized_call():
     st = _entry()(0, P, cols, 1, rows, dummy.data_ptr(), dummy.data_ptr(), None)
     assert st == S.GZ_INVALID
     assert "static scratch" in _last_error()
+
+
+@pytest.fixture(scope="module")
+def many_keys():
+    """One batch with a key of every width, nulls in all, and the Spark hash's ids by P."""
+    n = 70001
+    rng = np.random.default_rng(7)
+    schema = [W.Field(f"k{i}", t) for i, t in enumerate(("int64", "int32", "int16", "int8", "bool", "float64"))]
+    bufs = []
+    for f in schema:
+        v = rng.standard_normal(n) if f.type == "float64" else rng.integers(0, 2 if f.type == "bool" else 120, n)
+        bufs += W._column(rng, f, n, v, 0.2)
+    batch = W.Batch(n, bufs)
+    ids = {}
+
+    def pids(P):
+        if P not in ids:
+            ids[P] = _oracle_pids(schema, list(range(len(schema))), P, batch)
+        return ids[P]
+
+    return schema, batch, pids
+
+
+# both sides of every line of the dispatch: rows of one cluster block, of a cluster, of two launches;
+# histograms of 512- and 1024-thread blocks, of one block per SM, in the scratch
+@pytest.mark.parametrize("P", [1, 8, 2048, 2049, 12288, 12289, 24577, 57344, 57345])
+@pytest.mark.parametrize("shift", [0, 1])
+def test_static_ids_and_counts_over_sizes(many_keys, P, shift):
+    schema, batch, pids = many_keys
+    cols = (GzKeyColumn * len(schema))()
+    hold = []
+    for j, f in enumerate(schema):
+        valid, vals = batch.buffers[2 * j].view(np.uint8), batch.buffers[2 * j + 1].view(np.uint8)
+        w = W.BYTE_WIDTH.get(f.type, 1) * shift  # values one element off the allocation's alignment
+        t = torch.from_numpy(np.concatenate([np.zeros(w, np.uint8), vals])).cuda()
+        m = torch.from_numpy(np.concatenate([np.zeros(shift, np.uint8), valid])).cuda()
+        hold += [t, m]
+        cols[j].type, cols[j].values, cols[j].validity = f.code, t.data_ptr() + w, m.data_ptr() + shift
+    for n in (1, 3, 1023, 1024, 1025, 8192, 8193, 32767, 32768, 32769, batch.num_rows):
+        if -(-n // TILE_ROWS) * P > MAX_COUNTERS:
+            continue
+        out = torch.full((n + 1 + shift,), -1, dtype=torch.int16, device="cuda")
+        counts = torch.full((P,), -1, dtype=torch.int64, device="cuda")
+        st = _entry()(0, P, cols, len(schema), n, out.data_ptr() + 2 * shift, counts.data_ptr(),
+                      torch.cuda.current_stream().cuda_stream)
+        assert st == 0, _last_error()
+        got = out.cpu().numpy().view(np.uint16)
+        want = pids(P)[:n]
+        assert np.array_equal(got[shift:shift + n], want), (n, P)
+        assert got[shift + n] == 0xFFFF  # nothing past the last row
+        assert np.array_equal(counts.cpu().numpy(), np.bincount(want, minlength=P)), (n, P)
+    del hold
