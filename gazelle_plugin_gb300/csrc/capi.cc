@@ -342,9 +342,9 @@ GzStatus gz_split_stop(int64_t handle, GzSplitResult* out) {
 GzStatus gz_split_data(int64_t handle, uint8_t* dst, int64_t* out_size) {
   auto e = Lookup(handle);
   if (!e) return GZ_INVALID;
-  const auto& d = e->splitter->DataBytes();
-  if (out_size) *out_size = (int64_t)d.size();
-  if (dst && !d.empty()) memcpy(dst, d.data(), d.size());
+  const gz::Splitter& sp = *e->splitter;
+  if (out_size) *out_size = sp.DataSize();
+  if (dst && sp.DataSize() > 0) memcpy(dst, sp.DataBytes(), (size_t)sp.DataSize());
   return GZ_OK;
 }
 

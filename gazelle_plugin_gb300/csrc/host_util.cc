@@ -204,6 +204,7 @@ class CopyPool {
 namespace {
 
 struct ForJob {
+  std::function<void(size_t)> own;  // Background's function
   const std::function<void(size_t)>* fn;
   size_t n;
   std::atomic<size_t> next{0};
@@ -281,6 +282,17 @@ void ParallelFor(size_t n, const std::function<void(size_t)>& fn, int max_helper
   job->Work();
   std::unique_lock<std::mutex> lk(job->mu);
   job->cv.wait(lk, [&] { return job->done.load() == n; });
+}
+
+void Background(int threads, const std::function<void()>& fn) {
+  ForPool& pool = ForPool::Get();
+  const int n = std::min(threads, pool.workers());
+  if (n <= 0) return;
+  auto job = std::make_shared<ForJob>();
+  job->own = [fn](size_t) { fn(); };
+  job->fn = &job->own;
+  job->n = (size_t)n;
+  pool.Post(job, n);
 }
 
 void ParallelCopy(const std::vector<CopyJob>& jobs, size_t total_bytes) {

@@ -40,4 +40,8 @@ void ParallelCopy(const std::vector<CopyJob>& jobs, size_t total_bytes);
 // every fn(i) has returned.  Items are claimed one at a time, so long and short items balance.
 void ParallelFor(size_t n, const std::function<void(size_t)>& fn, int max_helpers = 15);
 
+// Starts fn on up to `threads` threads of that pool and returns at once; fn runs at most that often
+// (not at all while the pool is busy), possibly after the caller is done: it owns what it uses.
+void Background(int threads, const std::function<void()>& fn);
+
 }  // namespace gz

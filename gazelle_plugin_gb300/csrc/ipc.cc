@@ -191,7 +191,7 @@ int64_t AppendLz4Buffer(int64_t uncompressed_len, const std::vector<Lz4BlockRef>
     uint8_t* w = m + 15 + 4 * i;
     Put<uint32_t>(w, blocks[i].size | (blocks[i].stored ? 0x80000000u : 0u));
     pieces->push_back(Chunk{w, 4});
-    if (blocks[i].size) pieces->push_back(Chunk{blocks[i].data, (int64_t)blocks[i].size});
+    if (blocks[i].size) pieces->push_back(Chunk{blocks[i].data, (int64_t)blocks[i].size, blocks[i].dev});
     total += 4 + blocks[i].size;
   }
   pieces->push_back(Chunk{m + 15 + 4 * nb, 4});  // end mark (zeros)

@@ -90,6 +90,7 @@ struct Lz4BlockRef {
   const uint8_t* data;
   uint32_t size;
   bool stored;
+  bool dev = false;  // `data` is device memory
 };
 
 // Appends the bytes of one compressed IPC body buffer to `pieces`: the int64 uncompressed length,

@@ -154,7 +154,7 @@ __device__ uint32_t compress_block(const uint8_t* src, uint32_t n, uint16_t* tab
 __global__ void __launch_bounds__(kCWarps * 32, 8)
 k_lz4_compress(const Lz4Chunk* __restrict__ chunks, uint32_t n_chunks, uint32_t* next, uint8_t* scratch,
                uint8_t* out, unsigned long long* out_used, unsigned long long out_cap, Lz4Block* res,
-               int32_t* err) {
+               bool skip_stored, int32_t* err) {
   extern __shared__ __align__(16) uint8_t csm[];
   const uint32_t warp = threadIdx.x >> 5;
   uint8_t* sbuf = csm + (size_t)warp * (kStage + (2u << kHashLog));
@@ -186,6 +186,11 @@ k_lz4_compress(const Lz4Chunk* __restrict__ chunks, uint32_t n_chunks, uint32_t*
     }
     const bool stored = size >= n;  // a plain copy, or no gain: the block is stored as it is
     if (stored) size = n;
+    if (stored && skip_stored) {
+      if (lane_id() == 0) res[c] = Lz4Block{0, n, 1u};
+      __syncwarp();
+      continue;
+    }
     unsigned long long pos = 0;
     if (lane_id() == 0) pos = atomicAdd(out_used, (unsigned long long)((size + 15) & ~15u));
     pos = __shfl_sync(kFull, pos, 0);
@@ -710,7 +715,7 @@ uint32_t lz4_compress_warps() { return (uint32_t)sm_count() * 8 * kCWarps; }
 
 cudaError_t launch_lz4_compress(const Lz4Chunk* chunks, uint32_t n_chunks, uint32_t* next, uint8_t* scratch,
                                 uint8_t* out, unsigned long long* out_used, unsigned long long out_cap,
-                                Lz4Block* res, int32_t* err, cudaStream_t st) {
+                                Lz4Block* res, bool skip_stored, int32_t* err, cudaStream_t st) {
   if (n_chunks == 0) return cudaSuccess;
   const uint32_t grid = lz4_compress_warps() / kCWarps;
   static bool attr = false;
@@ -719,7 +724,7 @@ cudaError_t launch_lz4_compress(const Lz4Chunk* chunks, uint32_t n_chunks, uint3
     if (e != cudaSuccess) return e;
     attr = true;
   }
-  k_lz4_compress<<<grid, kCWarps * 32, kCompressSmem, st>>>(chunks, n_chunks, next, scratch, out, out_used, out_cap, res, err);
+  k_lz4_compress<<<grid, kCWarps * 32, kCompressSmem, st>>>(chunks, n_chunks, next, scratch, out, out_used, out_cap, res, skip_stored, err);
   return cudaGetLastError();
 }
 

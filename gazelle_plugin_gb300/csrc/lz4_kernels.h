@@ -50,10 +50,11 @@ uint32_t lz4_compress_warps();
 
 // Compresses every chunk into the arena `out` (out_cap bytes; *out_used is the bump counter,
 // *next the work counter, both zero at launch); res[c] tells where chunk c went.  *err gets bit
-// 0 when the arena ran out.
+// 0 when the arena ran out.  skip_stored: a chunk that does not shrink takes no room (its input is
+// its payload).
 cudaError_t launch_lz4_compress(const Lz4Chunk* chunks, uint32_t n_chunks, uint32_t* next, uint8_t* scratch,
                                 uint8_t* out, unsigned long long* out_used, unsigned long long out_cap,
-                                Lz4Block* res, int32_t* err, cudaStream_t st);
+                                Lz4Block* res, bool skip_stored, int32_t* err, cudaStream_t st);
 
 // Memory of one block slot of a frame of dst_len bytes (16-byte units; no block is longer).
 #ifdef __CUDACC__

@@ -15,6 +15,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <functional>
 #include <memory>
 #include <string>
 #include <vector>
@@ -87,7 +88,8 @@ class Splitter {
   int64_t TotalComputePidTime() const { return total_compute_pid_time_; }
   const std::vector<int64_t>& PartitionLengths() const { return partition_lengths_; }
   const std::vector<int64_t>& RawPartitionLengths() const { return raw_partition_lengths_; }
-  const std::vector<uint8_t>& DataBytes() const { return data_bytes_; }
+  const uint8_t* DataBytes() const { return data_bytes_.get(); }
+  int64_t DataSize() const { return data_size_; }
   int32_t num_partitions() const { return P_; }
   bool stopped() const { return stopped_; }
 
@@ -239,11 +241,27 @@ class Splitter {
   // `device_view`: body ranges point at the pass outputs where they are (HBM, or pinned host
   // memory the device reads; Chunk::dev set) for the device to compress or copy, bit regions at
   // their host copies (h_bits); otherwise everything points at the host copies (h_out).
-  Status BuildSegment(int p, const Segment& s, SegMsg* msg, bool device_view = false) const;
-  // Compressed Stop: body ranges of every record batch through the device (LZ4 blocks for
-  // batches above batch_compress_threshold rows, plain copies for the others) into one arena,
-  // which is then copied to pinned host memory; fills every message's header and pieces.
-  Status CompressBodies(std::vector<std::vector<SegMsg>>* msgs);
+  // `encode`: fill the header and pieces too (a compressed batch's are filled by CompressBodies).
+  Status BuildSegment(int p, const Segment& s, SegMsg* msg, bool device_view = false, bool encode = true) const;
+  // Compressed Stop: body ranges of every record batch above batch_compress_threshold rows through
+  // the device (LZ4 blocks) into one arena; fills every message's header and pieces.  With
+  // `emit` the arena (compress_mem_) stays on the device and what was not compressed where it is;
+  // otherwise everything (the other batches as plain copies) goes through the arena to pinned
+  // host memory.
+  Status CompressBodies(std::vector<std::vector<SegMsg>>* msgs, bool emit);
+  // The data file's `total` bytes put together by the device (k_emit): partition p's from start[p]
+  // on, each the schema message, its messages and the end-of-stream marker.
+  Status EmitData(const std::vector<std::vector<SegMsg>>& msgs, const std::vector<uint8_t>& schema_msg,
+                  const std::vector<int64_t>& start, int64_t total);
+  Status EmitWindows(const std::vector<std::vector<SegMsg>>& msgs, const std::vector<uint8_t>& schema_msg,
+                     const std::vector<int64_t>& start, int64_t total, int64_t W, int fd, uint8_t* map,
+                     const std::function<bool(size_t)>& ready);
+  Status WriteData(const std::vector<std::vector<SegMsg>>& msgs, const std::vector<uint8_t>& schema_msg,
+                   const std::vector<int64_t>& start, int64_t total);
+  bool EmitAtStop() const;
+  bool coherent_ = false;       // the device reads and writes pageable host memory
+  bool emit_at_stop_ = false;   // Stop has begun and the device puts the data file together
+  uint8_t* compress_mem_ = nullptr;
   uint32_t SplitBatchSize(int32_t num_rows, const std::vector<const uint8_t*>& host_offsets,
                           bool* complete);
 
@@ -406,7 +424,8 @@ class Splitter {
   double kernel_ms_[4] = {0, 0, 0, 0};
   size_t timed_flushes_ = 0;
   std::vector<int64_t> partition_lengths_, raw_partition_lengths_;
-  std::vector<uint8_t> data_bytes_;
+  std::unique_ptr<uint8_t[]> data_bytes_;  // without a data file: its bytes
+  int64_t data_size_ = 0;
 };
 
 // Split calls of several tasks at once (task i: n_batches[i] batches of n_bufs[i] buffers, its
