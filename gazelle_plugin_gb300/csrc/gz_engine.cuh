@@ -102,6 +102,12 @@ struct HostCopy {
   uint64_t bytes;
 };
 
+// Descriptors passed as kernel parameters: a call's buffers (a 16-column batch has 34).
+constexpr uint32_t kGatherArgs = 128;
+struct GatherArgs {
+  HostCopy job[kGatherArgs];
+};
+
 // bits of FlushDesc::err
 constexpr int32_t kErrEmitOverflow = 1;
 constexpr int32_t kErrBadOffsets = 2;

@@ -130,7 +130,6 @@ PartitionReader::~PartitionReader() {
     cudaStreamSynchronize(stream_);
     cudaStreamDestroy(stream_);
   }
-  PinnedRelease(PinnedBlock{reinterpret_cast<uint8_t*>(jobs_), jobs_bytes_});
 }
 
 // Walks the messages of one stream: an optional schema message, record batches, then the
@@ -326,35 +325,29 @@ Status PartitionReader::AddStream(const uint8_t* data, int64_t len) {
   std::vector<FrameRef> frames;
   int64_t arena_bytes = 0;
   const int idx = (int)images_.size();
-  Status st = ParseStream(data, len, idx, &bs, &frames, &arena_bytes);
-  if (!st.ok()) return st;
-  st = Cuda(cudaSetDevice(device_), "cudaSetDevice");
+  Status st = Cuda(cudaSetDevice(device_), "cudaSetDevice");
   if (!st.ok()) return st;
   uint8_t* d = nullptr;
   uint8_t* arena = nullptr;
-  if (!bs.empty()) {
+  if (len > 0) {
     st = Cuda(cudaMallocAsync(reinterpret_cast<void**>(&d), AlignUp((size_t)len, 256), stream_), "cudaMallocAsync(stream)");
     if (!st.ok()) return st;
-    // the caller's bytes are read before the call returns: by the device itself where it walks
-    // the host page tables (many CTAs reading 256 KiB pieces over the coherent link), else by a copy
+    // the caller's bytes are read before the call returns, and while the host parses them: by the
+    // device itself where it walks the host page tables, else by a copy
     if (direct_) {
-      const size_t piece = 256u << 10;
-      const size_t n = ((size_t)len + piece - 1) / piece;
-      if (jobs_cap_ < n) {
-        PinnedRelease(PinnedBlock{reinterpret_cast<uint8_t*>(jobs_), jobs_bytes_});
-        const PinnedBlock b = PinnedAcquire(sizeof(HostCopy) * n);
-        if (!b.ptr) return Status::Error(GZ_OOM, "pinned host memory for copy descriptors");
-        jobs_ = reinterpret_cast<HostCopy*>(b.ptr);
-        jobs_bytes_ = b.cap;
-        jobs_cap_ = b.cap / sizeof(HostCopy);
-      }
-      for (size_t i = 0; i < n; i++)
-        jobs_[i] = HostCopy{data + i * piece, d + i * piece, std::min<uint64_t>(piece, (uint64_t)len - i * piece)};
-      st = Cuda(launch_gather(jobs_, (uint32_t)n, stream_), "k_gather");
+      const HostCopy job{data, d, (uint64_t)len};
+      st = Cuda(launch_gather_args(&job, 1, nullptr, nullptr, 0, stream_), "k_gather");
     } else {
       st = Cuda(cudaMemcpyAsync(d, data, (size_t)len, cudaMemcpyHostToDevice, stream_), "H2D stream");
     }
-    if (!st.ok()) return st;
+    if (st.ok()) st = ParseStream(data, len, idx, &bs, &frames, &arena_bytes);
+    if (!st.ok() || bs.empty()) {  // nothing to keep
+      const Status read = Cuda(cudaStreamSynchronize(stream_), "H2D stream");
+      cudaFreeAsync(d, stream_);
+      d = nullptr;
+      if (st.ok()) st = read;
+      if (!st.ok()) return st;
+    }
   }
   images_.push_back(d);
   arenas_.push_back(nullptr);

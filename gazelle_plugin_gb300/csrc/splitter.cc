@@ -323,9 +323,11 @@ Status Splitter::Init(const std::string& short_name, std::vector<Field> fields, 
   }
   if (direct_) {
     jobs_cap_ = size_t(1) << 20;  // 24 MiB of descriptors: a refill waits for the device
-    const PinnedBlock b = PinnedAcquire(jobs_cap_ * sizeof(HostCopy));
+    const PinnedBlock b = PinnedAcquire(jobs_cap_ * sizeof(HostCopy) + 64);
     if (!b.ptr) return Status::Error(GZ_OOM, "pinned host memory for the gather descriptors");
     h_jobs_ = reinterpret_cast<HostCopy*>(b.ptr);
+    h_reads_ = reinterpret_cast<uint32_t*>(b.ptr + jobs_cap_ * sizeof(HostCopy));
+    *h_reads_ = 0;
     h_jobs_bytes_ = b.cap;
   }
   {
@@ -339,7 +341,7 @@ Status Splitter::Init(const std::string& short_name, std::vector<Field> fields, 
   const size_t state_bytes = AlignUp(sizeof(uint32_t) * P_, 256) * 2 +
                              AlignUp(sizeof(unsigned long long) * P_, 256) +
                              AlignUp(sizeof(uint32_t) * (size_t)std::max(n_str_, 1) * P_, 256) +
-                             256 * 3;
+                             256 * 4;
   st = Cuda(cudaMallocAsync(reinterpret_cast<void**>(&d_state_), state_bytes, stream_), "cudaMallocAsync(state)");
   if (!st.ok()) return st;
   st = Cuda(cudaMemsetAsync(d_state_, 0, state_bytes, stream_), "cudaMemset(state)");
@@ -351,7 +353,8 @@ Status Splitter::Init(const std::string& short_name, std::vector<Field> fields, 
   st_sb_ = reinterpret_cast<uint32_t*>(q); q += AlignUp(sizeof(uint32_t) * (size_t)std::max(n_str_, 1) * P_, 256);
   st_ihn_ = reinterpret_cast<unsigned long long*>(q); q += 256;
   d_err_ = reinterpret_cast<int32_t*>(q); q += 256;
-  d_call_ = reinterpret_cast<uint32_t*>(q);
+  d_call_ = reinterpret_cast<uint32_t*>(q); q += 256;
+  d_reads_ = reinterpret_cast<uint32_t*>(q);
   for (int i = 0; i < 2; i++) {
     st = Cuda(cudaEventCreateWithFlags(&stage_ev_[i], cudaEventDisableTiming), "cudaEventCreate");
     if (!st.ok()) return st;
@@ -506,7 +509,9 @@ Status Splitter::SplitMany(int32_t n_batches, const int32_t* rows, const int64_t
 Status Splitter::LaunchGather() {
   const size_t n = jobs_end_ - jobs_begin_;
   if (n == 0) return Status::OK();
-  Status st = Cuda(launch_gather(h_jobs_ + jobs_begin_, (uint32_t)n, cstream_), "k_gather");
+  Status st = Cuda(n <= kGatherArgs ? launch_gather_args(h_jobs_ + jobs_begin_, (uint32_t)n, d_reads_, nullptr, 0, cstream_)
+                                    : launch_gather(h_jobs_ + jobs_begin_, (uint32_t)n, cstream_),
+                   "k_gather");
   jobs_begin_ = jobs_end_;
   gather_pending_bytes_ = 0;
   return st;
@@ -519,9 +524,17 @@ Status Splitter::FinishHostReads() {
   return st.ok() ? WaitHostReads() : st;
 }
 
-// Launches the queued host reads and marks their end; WaitHostReads waits for that mark.
+// Launches the queued host reads and marks their end; WaitHostReads waits for that mark: the word that
+// a single launch (a plain split call's) writes itself, else an event.
 Status Splitter::StartHostReads() {
   if (!direct_ || jobs_end_ == 0) return Status::OK();
+  if (jobs_begin_ == 0 && jobs_end_ <= kGatherArgs) {
+    Status st = Cuda(launch_gather_args(h_jobs_, (uint32_t)jobs_end_, d_reads_, h_reads_, ++reads_seq_, cstream_), "k_gather");
+    jobs_begin_ = jobs_end_;
+    gather_pending_bytes_ = 0;
+    reads_marked_ = reads_word_ = st.ok();
+    return st;
+  }
   Status st = LaunchGather();
   if (!st.ok()) return st;
   st = Cuda(cudaEventRecord(gather_ev_, cstream_), "event");
@@ -533,8 +546,22 @@ Status Splitter::StartHostReads() {
 Status Splitter::WaitHostReads() {
   if (!reads_marked_) return Status::OK();
   reads_marked_ = false;
-  Status st = Cuda(cudaEventSynchronize(gather_ev_), "host reads");
-  if (!st.ok()) return st;
+  Status st;
+  if (reads_word_) {
+    reads_word_ = false;
+    for (uint32_t polls = 1; __atomic_load_n(h_reads_, __ATOMIC_ACQUIRE) != reads_seq_; polls++) {
+      if (polls % 4096) continue;
+      // taking long: a failed launch never writes the word
+      const cudaError_t e = cudaStreamQuery(cstream_);
+      if (e == cudaSuccess) break;
+      if (e != cudaErrorNotReady) return Cuda(e, "host reads");
+      cudaGetLastError();
+      std::this_thread::yield();
+    }
+  } else {
+    st = Cuda(cudaEventSynchronize(gather_ev_), "host reads");
+    if (!st.ok()) return st;
+  }
   jobs_begin_ = jobs_end_ = 0;
   return Status::OK();
 }

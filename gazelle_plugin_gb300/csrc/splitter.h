@@ -220,7 +220,11 @@ class Splitter {
   Status SplitOne(int32_t num_rows, const int64_t* addrs, const int64_t* sizes, int32_t n);
   Status LaunchGather();
   Status FinishHostReads();
-  bool reads_marked_ = false;  // gather_ev_ marks host reads not yet waited for
+  bool reads_marked_ = false;  // gather_ev_, or h_reads_, marks host reads not yet waited for
+  bool reads_word_ = false;    // it is h_reads_: the last k_gather_args writes reads_seq_ there
+  uint32_t* h_reads_ = nullptr;  // (pinned, behind h_jobs_)
+  uint32_t* d_reads_ = nullptr;  // its count of finished blocks
+  uint32_t reads_seq_ = 0;
   Status PinnedMeta(size_t bytes, uint32_t** out);
   Status Flush();
   Status SyncAndCheck();

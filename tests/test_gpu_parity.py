@@ -455,3 +455,29 @@ def test_split_group_of_tasks_equals_per_task_calls():
         w.stop(h, P)
         assert w.data(h) == O.run_oracle(sch, bs, P, keys).data
         w.close(h)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n_cols", [60, 61, 64])
+def test_host_reads_of_few_and_many_buffers_per_call(n_cols):
+    """A call's host reads go in one launch with their descriptors as kernel parameters up to 128 buffers
+    (two per int column with nulls) and through the descriptor ring above; buffers from one byte to
+    several pieces, at every 16-byte phase of the source."""
+    rng = np.random.default_rng(n_cols)
+    schema = [W.Field("k", "int64", False)] + [W.Field(f"c{i}", ("int8", "int32", "int64")[i % 3]) for i in range(n_cols - 1)]
+    keep, batches = [], []
+    for n in (1, 9, 4097, 20011, 32768):
+        bufs = []
+        for i, f in enumerate(schema):
+            cols = W._column(rng, f, n, rng.integers(-100, 100, n), 0.0 if i == 0 else 0.3)
+            for b in cols:
+                w = 1 if b is cols[0] else W.BYTE_WIDTH[f.type]
+                shift = (w * int(rng.integers(0, 16 // w))) if b.nbytes else 0
+                room = np.zeros(b.nbytes + shift + 64, np.uint8)
+                at = (-room.ctypes.data) % 16 + shift
+                room[at:at + b.nbytes] = b.view(np.uint8)
+                keep.append(room)
+                bufs.append(room[at:at + b.nbytes])
+        batches.append(W.Batch(n, bufs))
+    res, data = S.split_batches(schema, batches, 16, [0])
+    assert data == O.run_oracle(schema, batches, 16, [0]).data
