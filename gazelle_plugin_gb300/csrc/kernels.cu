@@ -1651,14 +1651,12 @@ __global__ void __launch_bounds__(256) k_gather_args(const __grid_constant__ Gat
     for (uint64_t j = threadIdx.x; j < to - from; j += 256) dst[j] = src[j];
   }
   if (flag == nullptr) return;
-  __syncthreads();  // every load of the block has returned: its value has been stored
-  if (threadIdx.x == 0) {
-    __threadfence_system();
-    if (atomicAdd(done, 1u) == n_pieces - 1) {
-      *done = 0;  // for the next launch on this stream
-      __threadfence_system();
-      *flag = seq;
-    }
+  // Every load of the block has returned: the store of its value has been issued.  That is all the
+  // host waits for (the stores' readers come later on the stream), so nothing is fenced.
+  __syncthreads();
+  if (threadIdx.x == 0 && atomicAdd(done, 1u) == n_pieces - 1) {
+    *done = 0;  // for the next launch on this stream
+    *flag = seq;
   }
 }
 

@@ -1,6 +1,6 @@
 // sm_103a kernels of the reduce-side read (PartitionReader): the record batches of a partition's
 // IPC streams, already in HBM, concatenated into one set of Arrow columns.  Three job lists, each
-// job at most a few hundred KB so that one CTA per job keeps every SM busy:
+// job at most 64 KB so that one CTA per job keeps every SM busy:
 //   byte jobs   values of fixed-width columns and characters of binary columns, copied
 //   offset jobs binary offsets (int32, or int64 of the large types) rebased:
 //               out[i] = in[i] - in[0] + (the batch's first character)
@@ -9,6 +9,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "copy.cuh"
 #include "read_kernels.h"
 
 namespace gz {
@@ -16,47 +17,6 @@ namespace gz {
 namespace {
 
 constexpr int kThreads = 256;
-
-template <typename V>
-__device__ __forceinline__ void copy_words(const uint8_t* src, uint8_t* dst, uint64_t n) {
-  constexpr uint32_t W = sizeof(V);
-  const uint64_t lead = (W - (reinterpret_cast<uintptr_t>(src) & (W - 1))) & (W - 1);
-  const uint64_t head = n < lead ? n : lead;
-  if (threadIdx.x < head) dst[threadIdx.x] = src[threadIdx.x];
-  const uint64_t nv = (n - head) / W;
-  const V* sv = reinterpret_cast<const V*>(src + head);
-  V* dv = reinterpret_cast<V*>(dst + head);
-  for (uint64_t i = threadIdx.x; i < nv; i += kThreads) dv[i] = sv[i];
-  for (uint64_t j = head + nv * W + threadIdx.x; j < n; j += kThreads) dst[j] = src[j];
-}
-
-__global__ void __launch_bounds__(kThreads) k_read_bytes(const ByteJob* __restrict__ jobs, uint32_t n_jobs) {
-  for (uint32_t b = blockIdx.x; b < n_jobs; b += gridDim.x) {
-    const ByteJob job = jobs[b];
-    const uintptr_t phase = reinterpret_cast<uintptr_t>(job.src) ^ reinterpret_cast<uintptr_t>(job.dst);
-    if ((phase & 15) == 0) copy_words<uint4>(job.src, job.dst, job.bytes);
-    else if ((phase & 7) == 0) copy_words<uint2>(job.src, job.dst, job.bytes);
-    else if ((phase & 3) == 0) copy_words<uint32_t>(job.src, job.dst, job.bytes);
-    else
-      for (uint64_t j = threadIdx.x; j < job.bytes; j += kThreads) job.dst[j] = job.src[j];
-  }
-}
-
-__global__ void __launch_bounds__(kThreads) k_read_offsets(const OffsetJob* __restrict__ jobs, uint32_t n_jobs) {
-  for (uint32_t b = blockIdx.x; b < n_jobs; b += gridDim.x) {
-    const OffsetJob job = jobs[b];
-    if (job.wide) {
-      const int64_t* src = static_cast<const int64_t*>(job.src);
-      int64_t* dst = static_cast<int64_t*>(job.dst);
-      for (uint32_t i = threadIdx.x; i < job.n; i += kThreads) dst[i] = src[i] + job.add;
-    } else {
-      const int32_t* src = static_cast<const int32_t*>(job.src);
-      int32_t* dst = static_cast<int32_t*>(job.dst);
-      const int32_t add = (int32_t)job.add;
-      for (uint32_t i = threadIdx.x; i < job.n; i += kThreads) dst[i] = src[i] + add;
-    }
-  }
-}
 
 // Bits [start, start + len) of `src` (len <= 32) as the low bits of a word.  Reads only the 4-byte
 // words that hold those bits.
@@ -68,19 +28,43 @@ __device__ __forceinline__ uint32_t extract_bits(const uint32_t* src, uint64_t s
   return len == 32 ? v : v & ((1u << len) - 1);
 }
 
-__global__ void __launch_bounds__(kThreads) k_read_bits(const BitJob* __restrict__ jobs, uint32_t n_jobs) {
-  for (uint32_t b = blockIdx.x; b < n_jobs; b += gridDim.x) {
-    const BitJob job = jobs[b];
-    if (job.nbits == 0) continue;
-    const uint64_t d0 = job.dst_bit, d1 = job.dst_bit + job.nbits;
-    const uint64_t w0 = d0 >> 5, w1 = (d1 - 1) >> 5;
-    for (uint64_t w = w0 + threadIdx.x; w <= w1; w += kThreads) {
-      const uint64_t lo = w * 32 > d0 ? w * 32 : d0;
-      const uint64_t hi = w * 32 + 32 < d1 ? w * 32 + 32 : d1;
-      const uint32_t len = (uint32_t)(hi - lo);
-      const uint32_t bits = job.src ? extract_bits(job.src, job.src_bit + (lo - d0), len)
-                                    : (len == 32 ? 0xffffffffu : (1u << len) - 1);
-      if (bits) atomicOr(job.dst + w, bits << (uint32_t)(lo - w * 32));
+// The three lists in one launch: blocks take the byte jobs first, then the offset jobs, then the bit jobs.
+// Bound by HBM (every byte read and written once).  A record batch's buffers meet the column at any
+// byte offset (characters) or element (values): the characters moved byte by byte before, in a launch of
+// their own.  READ_NOTE
+__global__ void __launch_bounds__(kThreads) k_read(const ReadJobs jobs) {
+  const uint32_t n = jobs.n_bytes + jobs.n_offs + jobs.n_bits;
+  for (uint32_t b = blockIdx.x; b < n; b += gridDim.x) {
+    if (b < jobs.n_bytes) {
+      const ByteJob job = jobs.bytes[b];
+      copy_bytes<kThreads>(job.dst, job.src, (uint32_t)job.bytes, threadIdx.x);
+    } else if (b < jobs.n_bytes + jobs.n_offs) {
+      const OffsetJob job = jobs.offs[b - jobs.n_bytes];
+      if (job.wide) {
+        const int64_t* src = static_cast<const int64_t*>(job.src);
+        int64_t* dst = static_cast<int64_t*>(job.dst);
+#pragma unroll 4
+        for (uint32_t i = threadIdx.x; i < job.n; i += kThreads) dst[i] = src[i] + job.add;
+      } else {
+        const int32_t* src = static_cast<const int32_t*>(job.src);
+        int32_t* dst = static_cast<int32_t*>(job.dst);
+        const int32_t add = (int32_t)job.add;
+#pragma unroll 8
+        for (uint32_t i = threadIdx.x; i < job.n; i += kThreads) dst[i] = src[i] + add;
+      }
+    } else {
+      const BitJob job = jobs.bits[b - jobs.n_bytes - jobs.n_offs];
+      if (job.nbits == 0) continue;
+      const uint64_t d0 = job.dst_bit, d1 = job.dst_bit + job.nbits;
+      const uint64_t w0 = d0 >> 5, w1 = (d1 - 1) >> 5;
+      for (uint64_t w = w0 + threadIdx.x; w <= w1; w += kThreads) {
+        const uint64_t lo = w * 32 > d0 ? w * 32 : d0;
+        const uint64_t hi = w * 32 + 32 < d1 ? w * 32 + 32 : d1;
+        const uint32_t len = (uint32_t)(hi - lo);
+        const uint32_t bits = job.src ? extract_bits(job.src, job.src_bit + (lo - d0), len)
+                                      : (len == 32 ? 0xffffffffu : (1u << len) - 1);
+        if (bits) atomicOr(job.dst + w, bits << (uint32_t)(lo - w * 32));
+      }
     }
   }
 }
@@ -120,15 +104,10 @@ cudaError_t gather_words(const int32_t* const* src, int32_t* out, size_t n, cuda
   return e;
 }
 
-cudaError_t launch_read_jobs(const ByteJob* bytes, uint32_t n_bytes, const OffsetJob* offs, uint32_t n_offs,
-                             const BitJob* bits, uint32_t n_bits, cudaStream_t st) {
-  if (n_bytes) k_read_bytes<<<grid_for(n_bytes), kThreads, 0, st>>>(bytes, n_bytes);
-  cudaError_t e = cudaGetLastError();
-  if (e != cudaSuccess) return e;
-  if (n_offs) k_read_offsets<<<grid_for(n_offs), kThreads, 0, st>>>(offs, n_offs);
-  e = cudaGetLastError();
-  if (e != cudaSuccess) return e;
-  if (n_bits) k_read_bits<<<grid_for(n_bits), kThreads, 0, st>>>(bits, n_bits);
+cudaError_t launch_read_jobs(const ReadJobs& jobs, cudaStream_t st) {
+  const uint32_t n = jobs.n_bytes + jobs.n_offs + jobs.n_bits;
+  if (n == 0) return cudaSuccess;
+  k_read<<<grid_for(n), kThreads, 0, st>>>(jobs);
   return cudaGetLastError();
 }
 

@@ -31,8 +31,14 @@ struct BitJob {  // bits [src_bit, src_bit + nbits) of src (all ones when src is
 // enqueues: the caller synchronises `st` before reading out).
 cudaError_t gather_words(const int32_t* const* src, int32_t* out, size_t n, cudaStream_t st);
 
-// Runs the three job lists on `st` (the job arrays in device memory).
-cudaError_t launch_read_jobs(const ByteJob* bytes, uint32_t n_bytes, const OffsetJob* offs, uint32_t n_offs,
-                             const BitJob* bits, uint32_t n_bits, cudaStream_t st);
+struct ReadJobs {  // the job lists, in device memory
+  const ByteJob* bytes;
+  const OffsetJob* offs;
+  const BitJob* bits;
+  uint32_t n_bytes, n_offs, n_bits;
+};
+
+// Runs the three job lists on `st` in one launch (a byte job: less than 4 GB).
+cudaError_t launch_read_jobs(const ReadJobs& jobs, cudaStream_t st);
 
 }  // namespace gz

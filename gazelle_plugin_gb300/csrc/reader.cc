@@ -576,7 +576,7 @@ Status PartitionReader::Finish(int64_t* rows, int32_t* n_batches) {
   std::vector<ByteJob> bj;
   std::vector<OffsetJob> oj;
   std::vector<BitJob> tj;
-  constexpr uint64_t kChunk = 256u << 10;   // bytes per byte job
+  constexpr uint64_t kChunk = 64u << 10;    // bytes per byte job
   constexpr uint64_t kBitChunk = 1u << 20;  // bits per bit job
   auto add_bytes = [&](const uint8_t* src, uint8_t* dst, uint64_t n) {
     for (uint64_t x = 0; x < n; x += kChunk) bj.push_back(ByteJob{src + x, dst + x, std::min(kChunk, n - x)});
@@ -699,10 +699,11 @@ Status PartitionReader::Finish(int64_t* rows, int32_t* n_batches) {
   if (!st.ok()) return st;
   st = Cuda(cudaMemcpyAsync(dj, hj.data(), hj.size(), cudaMemcpyHostToDevice, stream_), "H2D jobs");
   if (st.ok())
-    st = Cuda(launch_read_jobs(reinterpret_cast<const ByteJob*>(dj), (uint32_t)bj.size(),
-                               reinterpret_cast<const OffsetJob*>(dj + jb), (uint32_t)oj.size(),
-                               reinterpret_cast<const BitJob*>(dj + jb + jo), (uint32_t)tj.size(), stream_),
-              "reader kernels");
+    st = Cuda(launch_read_jobs(ReadJobs{reinterpret_cast<const ByteJob*>(dj), reinterpret_cast<const OffsetJob*>(dj + jb),
+                                        reinterpret_cast<const BitJob*>(dj + jb + jo), (uint32_t)bj.size(),
+                                        (uint32_t)oj.size(), (uint32_t)tj.size()},
+                               stream_),
+              "k_read");
   cudaFreeAsync(dj, stream_);
   if (!st.ok()) return st;
   // the stream images and decoded buffers are no longer needed
@@ -714,7 +715,7 @@ Status PartitionReader::Finish(int64_t* rows, int32_t* n_batches) {
     if (p) cudaFreeAsync(p, stream_);
     p = nullptr;
   }
-  st = Cuda(cudaStreamSynchronize(stream_), "reader kernels");
+  st = Cuda(cudaStreamSynchronize(stream_), "k_read");
   if (!st.ok()) return st;
   out_nodes_.assign(F, {});
   for (size_t f = 0; f < F; f++) {
