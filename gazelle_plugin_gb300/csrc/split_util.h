@@ -45,19 +45,36 @@ inline int64_t OffAt(const uint8_t* off, int w, size_t r) {
 // Copies `nbits` bits from src (starting at bit `sbit`) to dst (starting at bit `dbit`);
 // dst bits outside the range are left as they are.
 inline void CopyBits(const uint8_t* src, uint64_t sbit, uint8_t* dst, uint64_t dbit, uint64_t nbits) {
-  for (uint64_t i = 0; i < nbits; i++) {
+  // bit by bit up to a byte of dst, then whole bytes (each from at most two of src), then the rest
+  auto one = [&](uint64_t i) {
     const uint64_t s = sbit + i, d = dbit + i;
     const uint8_t b = (src[s >> 3] >> (s & 7)) & 1;
     if (b) dst[d >> 3] |= (uint8_t)(1u << (d & 7));
     else dst[d >> 3] &= (uint8_t)~(1u << (d & 7));
+  };
+  uint64_t i = 0;
+  for (; i < nbits && ((dbit + i) & 7); i++) one(i);
+  const uint32_t sh = (uint32_t)((sbit + i) & 7);
+  const uint8_t* s = src + ((sbit + i) >> 3);
+  uint8_t* d = dst + ((dbit + i) >> 3);
+  const uint64_t nb = (nbits - i) >> 3;
+  if (sh == 0) {
+    if (nb) memcpy(d, s, (size_t)nb);
+  } else {
+    for (uint64_t k = 0; k < nb; k++) d[k] = (uint8_t)(s[k] >> sh | s[k + 1] << (8 - sh));
   }
+  for (i += nb << 3; i < nbits; i++) one(i);
 }
 
 inline int64_t CountZeros(const uint8_t* bits, int64_t n) {
-  int64_t ones = 0;
-  int64_t full = n >> 3;
-  for (int64_t i = 0; i < full; i++) ones += __builtin_popcount(bits[i]);
-  for (int64_t i = full * 8; i < n; i++) ones += (bits[i >> 3] >> (i & 7)) & 1;
+  int64_t ones = 0, i = 0;
+  for (; i + 64 <= n; i += 64) {
+    uint64_t w;
+    memcpy(&w, bits + (i >> 3), 8);
+    ones += __builtin_popcountll(w);
+  }
+  for (; i + 8 <= n; i += 8) ones += __builtin_popcount(bits[i >> 3]);
+  for (; i < n; i++) ones += (bits[i >> 3] >> (i & 7)) & 1;
   return n - ones;
 }
 

@@ -21,6 +21,7 @@
 #include "emit_kernels.h"
 #include "gz_kernels.h"
 #include "lz4_kernels.h"
+#include "stream_pool.h"
 #include "host_util.h"
 #include "split_util.h"
 #include "tune.h"
@@ -285,33 +286,22 @@ Status Splitter::Init(const std::string& short_name, std::vector<Field> fields, 
   (void)dummy;
   Status st = Cuda(cudaSetDevice(device_), "cudaSetDevice");
   if (!st.ok()) return st;
+  st = Cuda(AcquireStreams(device_, &streams_set_), "cudaStreamCreate");
+  if (!st.ok()) return st;
+  cstream_ = streams_set_.c;
+  pstream_ = streams_set_.p;
+  stream_ = streams_set_.s;
+  hstream_ = streams_set_.h;
+  ostream_ = streams_set_.o;
   {
-    // host reads, then the plan kernels, get the higher priorities: their few CTAs are
-    // scheduled ahead of the remaining CTAs of a running k_scatter; k_hash_count gets the lowest,
-    // so it takes the SMs k_scatter leaves idle instead of delaying it
-    int least = 0, greatest = 0;
-    cudaDeviceGetStreamPriorityRange(&least, &greatest);
-    st = Cuda(cudaStreamCreateWithPriority(&cstream_, cudaStreamNonBlocking, greatest), "cudaStreamCreate");
-    if (!st.ok()) return st;
-    st = Cuda(cudaStreamCreateWithPriority(&pstream_, cudaStreamNonBlocking, std::min(greatest + 1, least)),
-              "cudaStreamCreate");
-    if (!st.ok()) return st;
-    st = Cuda(cudaStreamCreateWithPriority(&stream_, cudaStreamNonBlocking, std::min(greatest + 2, least)),
-              "cudaStreamCreate");
-    if (!st.ok()) return st;
-    st = Cuda(cudaStreamCreateWithPriority(&hstream_, cudaStreamNonBlocking, least), "cudaStreamCreate");
-    if (!st.ok()) return st;
+    static_assert(2 + kScratchBufs + 2 + kTabBufs == StreamSet::kEvents, "an event each");
+    const cudaEvent_t* e = streams_set_.ev;
+    hwait_ev_ = *e++;
+    gather_ev_ = *e++;
+    for (auto& x : scr_ev_) x = *e++;
+    for (auto& x : stage_ev_) x = *e++;
+    for (auto& x : tab_ev_) x = *e++;
   }
-  st = Cuda(cudaEventCreateWithFlags(&hwait_ev_, cudaEventDisableTiming), "cudaEventCreate");
-  if (!st.ok()) return st;
-  for (auto& e : scr_ev_) {
-    st = Cuda(cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "cudaEventCreate");
-    if (!st.ok()) return st;
-  }
-  st = Cuda(cudaStreamCreateWithFlags(&ostream_, cudaStreamNonBlocking), "cudaStreamCreate");
-  if (!st.ok()) return st;
-  st = Cuda(cudaEventCreateWithFlags(&gather_ev_, cudaEventDisableTiming), "cudaEventCreate");
-  if (!st.ok()) return st;
   {
     // kernels may dereference any host address when the device walks the host page tables
     // (a coherent CPU-GPU link): host inputs are then read by k_gather, no CPU copy
@@ -355,14 +345,6 @@ Status Splitter::Init(const std::string& short_name, std::vector<Field> fields, 
   d_err_ = reinterpret_cast<int32_t*>(q); q += 256;
   d_call_ = reinterpret_cast<uint32_t*>(q); q += 256;
   d_reads_ = reinterpret_cast<uint32_t*>(q);
-  for (int i = 0; i < 2; i++) {
-    st = Cuda(cudaEventCreateWithFlags(&stage_ev_[i], cudaEventDisableTiming), "cudaEventCreate");
-    if (!st.ok()) return st;
-  }
-  for (int i = 0; i < kTabBufs; i++) {
-    st = Cuda(cudaEventCreateWithFlags(&tab_ev_[i], cudaEventDisableTiming), "cudaEventCreate");
-    if (!st.ok()) return st;
-  }
   dev_off_.resize(n_str_);
   need_.assign(n_bufs_expected_ + 1, Need{nullptr, 0});
   host_off_.assign(n_str_, nullptr);
@@ -376,31 +358,22 @@ Status Splitter::Init(const std::string& short_name, std::vector<Field> fields, 
 }
 
 Splitter::~Splitter() {
-  if (cstream_) cudaStreamSynchronize(cstream_);
-  if (hstream_) cudaStreamSynchronize(hstream_);
-  if (stream_) cudaStreamSynchronize(stream_);
-  if (pstream_) cudaStreamSynchronize(pstream_);
-  if (ostream_) cudaStreamSynchronize(ostream_);
+  bool idle = true;
+  for (cudaStream_t st : {cstream_, hstream_, stream_, pstream_, ostream_})
+    if (st && cudaStreamSynchronize(st) != cudaSuccess) idle = false;
   for (auto& f : flushes_) {
     if (f.d_out) cudaFreeAsync(f.d_out, stream_);
-    for (auto& e : f.ev)
-      if (e) cudaEventDestroy(e);
+    for (auto& e : f.ev) ReleaseEvent(device_, e);
   }
   ReleaseHost();
   for (auto& c : meta_chunks_) PinnedRelease(c);
-  for (int i = 0; i < kTabBufs; i++) {
-    PinnedRelease(PinnedBlock{h_tables_[i], tables_cap_[i]});
-    if (tab_ev_[i]) cudaEventDestroy(tab_ev_[i]);
-  }
+  for (int i = 0; i < kTabBufs; i++) PinnedRelease(PinnedBlock{h_tables_[i], tables_cap_[i]});
   for (int i = 0; i < 2; i++) {
     PinnedRelease(PinnedBlock{h_stage_[i], h_stage_cap_});
     if (d_stage_[i]) cudaFreeAsync(d_stage_[i], stream_);
-    if (stage_ev_[i]) cudaEventDestroy(stage_ev_[i]);
   }
-  for (int i = 0; i < kScratchBufs; i++) {
+  for (int i = 0; i < kScratchBufs; i++)
     if (d_scratch_[i]) cudaFreeAsync(d_scratch_[i], stream_);
-    if (scr_ev_[i]) cudaEventDestroy(scr_ev_[i]);
-  }
   if (d_state_) cudaFreeAsync(d_state_, stream_);
   if (compress_mem_) cudaFreeAsync(compress_mem_, stream_);
   if (d_iota_ || !old_iota_.empty()) {
@@ -409,13 +382,9 @@ Splitter::~Splitter() {
     for (int32_t* o : old_iota_) cudaFree(o);
   }
   PinnedRelease(PinnedBlock{reinterpret_cast<uint8_t*>(h_jobs_), h_jobs_bytes_});
-  if (gather_ev_) cudaEventDestroy(gather_ev_);
-  if (pstream_) cudaStreamDestroy(pstream_);
-  if (hstream_) cudaStreamDestroy(hstream_);
-  if (hwait_ev_) cudaEventDestroy(hwait_ev_);
-  if (cstream_) cudaStreamDestroy(cstream_);
-  if (ostream_) cudaStreamDestroy(ostream_);
-  if (stream_) cudaStreamDestroy(stream_);
+  // (the frees above are all that is left on stream_; a set whose work failed is not used again)
+  if (idle) ReleaseStreams(&streams_set_);
+  else DestroyStreams(&streams_set_);
 }
 
 // CalculateSplitBatchSize (splitter.cc:800-853).  `host_offsets` (may hold nullptr) are the
@@ -1273,7 +1242,7 @@ Status Splitter::Flush() {
     }
   }
   for (auto& e : fr.ev) {
-    st = Cuda(cudaEventCreate(&e), "cudaEventCreate");
+    st = Cuda(AcquireEvent(device_, &e), "cudaEventCreate");
     if (!st.ok()) return st;
   }
   if (n_jobs) {  // the nested columns' row ranges and lengths, before anything reads them
@@ -1498,19 +1467,26 @@ void Splitter::DiskSpillStats(int64_t* out3) const {
 }
 
 Status Splitter::SyncAndCheck() {
-  Status st = Cuda(cudaStreamSynchronize(cstream_), "host reads");
+  for (cudaStream_t x : {cstream_, hstream_, pstream_}) {
+    Status st = Cuda(cudaStreamSynchronize(x), "device work");
+    if (!st.ok()) return st;
+  }
+  Status st = Cuda(cudaStreamSynchronize(ostream_), "partition data to host");
   if (!st.ok()) return st;
-  st = Cuda(cudaStreamSynchronize(hstream_), "device work");
-  if (!st.ok()) return st;
-  st = Cuda(cudaStreamSynchronize(stream_), "device work");
-  if (!st.ok()) return st;
-  st = Cuda(cudaStreamSynchronize(pstream_), "device work");
-  if (!st.ok()) return st;
-  st = Cuda(cudaStreamSynchronize(ostream_), "partition data to host");
+  // the error word and the partitions' open rows, behind everything that writes them
+  const size_t state = (size_t)(reinterpret_cast<uint8_t*>(st_sb_) - reinterpret_cast<uint8_t*>(st_base_));
+  if (!h_state_) {
+    uint32_t* m = nullptr;
+    st = PinnedMeta(256 + state, &m);
+    if (!st.ok()) return st;
+    h_state_ = reinterpret_cast<uint8_t*>(m);
+  }
+  st = Cuda(cudaMemcpyAsync(h_state_, d_err_, 4, cudaMemcpyDeviceToHost, stream_), "read error word");
+  if (st.ok()) st = Cuda(cudaMemcpyAsync(h_state_ + 256, st_base_, state, cudaMemcpyDeviceToHost, stream_), "D2H state");
+  if (st.ok()) st = Cuda(cudaStreamSynchronize(stream_), "device work");
   if (!st.ok()) return st;
   int32_t err = 0;
-  st = Cuda(cudaMemcpy(&err, d_err_, 4, cudaMemcpyDeviceToHost), "read error word");
-  if (!st.ok()) return st;
+  memcpy(&err, h_state_, 4);
   if (err & kErrTimeout) return Status::Error(GZ_TIMEOUT, "a device-side wait timed out");
   if (err & kErrBadOffsets)
     return Status::Error(GZ_INVALID, "binary offsets are decreasing or exceed the value buffer");
@@ -1542,7 +1518,9 @@ Status Splitter::ProcessFlushes() {
   const int words = kEmitFixedWords + nstr;
   for (; processed_flushes_ < flushes_.size(); processed_flushes_++) {
     const int32_t fi = (int32_t)processed_flushes_;
-    const FlushRec& f = flushes_[fi];
+    FlushRec& f = flushes_[fi];
+    f.zero_fb.assign(std::max(nstr, 1), 0);
+    f.last_fb.resize((size_t)P * std::max(nstr, 1));
     const uint32_t ne = f.emit_count(P, nstr);
     if (ne > f.emit_cap) return Status::Error(GZ_CUDA, "emission list overflow");
     const uint32_t* recs = f.emits(P, nstr);
@@ -1558,11 +1536,11 @@ Status Splitter::ProcessFlushes() {
       auto& v = by_p[p];
       std::sort(v.begin(), v.end(), [](const uint32_t* x, const uint32_t* y) { return x[1] < y[1]; });
       uint32_t frow0 = 0, vpos0 = 0;
-      std::vector<uint32_t> fb0(nstr, 0);
+      const uint32_t* fb0 = f.zero_fb.data();
       Segment& open = open_[p];
       for (const uint32_t* r : v) {
         const uint32_t frow1 = r[1];
-        std::vector<uint32_t> fb1(r + kEmitFixedWords, r + kEmitFixedWords + nstr);
+        const uint32_t* fb1 = r + kEmitFixedWords;  // (the pinned records live as long as the splitter)
         if (frow1 > frow0) open.pieces.push_back(Piece{fi, frow0, frow1, vpos0, fb0, fb1});
         vpos0 += (frow1 - frow0 + 63u) & ~63u;
         frow0 = frow1;
@@ -1578,7 +1556,7 @@ Status Splitter::ProcessFlushes() {
         open = Segment();
       }
       if (rows_f[p] > frow0) {
-        std::vector<uint32_t> fb1(nstr);
+        uint32_t* fb1 = f.last_fb.data() + (size_t)p * nstr;
         for (int k = 0; k < nstr; k++) fb1[k] = bytes_f[(size_t)k * P + p];
         open.pieces.push_back(Piece{fi, frow0, rows_f[p], vpos0, fb0, fb1});
       }
@@ -1880,12 +1858,9 @@ Status Splitter::Stop() {
   st = ProcessFlushes();
   if (!st.ok()) return st;
   // the open buffer of every partition is emitted at Stop (CacheRecordBatch(pid, true))
-  std::vector<uint32_t> base(P_);
-  std::vector<unsigned long long> hv(P_);
-  st = Cuda(cudaMemcpy(base.data(), st_base_, 4 * (size_t)P_, cudaMemcpyDeviceToHost), "D2H state");
-  if (!st.ok()) return st;
-  st = Cuda(cudaMemcpy(hv.data(), st_hv_, 8 * (size_t)P_, cudaMemcpyDeviceToHost), "D2H state");
-  if (!st.ok()) return st;
+  const uint32_t* base = reinterpret_cast<const uint32_t*>(h_state_ + 256);
+  const unsigned long long* hv = reinterpret_cast<const unsigned long long*>(
+      h_state_ + 256 + (reinterpret_cast<uint8_t*>(st_hv_) - reinterpret_cast<uint8_t*>(st_base_)));
   for (int p = 0; p < P_; p++) {
     Segment& open = open_[p];
     if (base[p] > 0) {
@@ -1928,6 +1903,8 @@ Status Splitter::Stop() {
   const std::vector<uint8_t> schema_msg = opts_.write_schema ? EncodeSchemaMessage(out_fields) : std::vector<uint8_t>();
   std::vector<std::vector<SegMsg>> msgs(P_);
   std::vector<Status> pst(P_);
+  // (a few small partitions are done sooner than helpers wake up)
+  const int helpers = stat_input_bytes_ < kEmitBytes && P_ <= 64 ? 0 : 15;
   ParallelFor((size_t)P_, [&](size_t pi) {
     const int p = (int)pi;
     const auto& segs = segments_[p];
@@ -1939,7 +1916,7 @@ Status Splitter::Stop() {
         return;
       }
     }
-  });
+  }, helpers);
   for (int p = 0; p < P_; p++)
     if (!pst[p].ok()) return pst[p];
   if (compressed) {
@@ -1979,9 +1956,13 @@ Status Splitter::Stop() {
   for (auto& v : segments_) stat_emitted_ += (int64_t)v.size();
   total_write_time_ += NowNs() - t0;
   stopped_ = true;
-  // the pinned copies are no longer needed
+  // the pinned copies are no longer needed, nor the messages (made by many threads, and freed so)
   ReleaseHost();
   ReleaseStaging();
+  ParallelFor((size_t)P_, [&](size_t p) {
+    std::vector<SegMsg>().swap(msgs[p]);
+    for (Segment& s : segments_[p]) std::vector<Piece>().swap(s.pieces);
+  }, helpers);
   return Status::OK();
 }
 
@@ -2015,18 +1996,25 @@ Status Splitter::WriteData(const std::vector<std::vector<SegMsg>>& msgs, const s
   }
   static const uint32_t kEos[2] = {0xFFFFFFFFu, 0u};  // WriteEOS (splitter.cc:166-172)
   std::vector<char> wrote(P_, 1);
-  ParallelFor((size_t)P_, [&](size_t pi) {
-    const int p = (int)pi;
-    if (msgs[p].empty()) return;
-    RangeWriter w(fd, mem, start[p]);
+  auto put = [&](RangeWriter& w, int p) {
+    if (msgs[p].empty()) return true;
     bool ok = w.Add(schema_msg.data(), (int64_t)schema_msg.size());
     for (const SegMsg& m : msgs[p]) {
       ok = ok && w.Add(m.header.data(), (int64_t)m.header.size());
       for (const Chunk& c : m.pieces) ok = ok && w.Add(c.data, c.len);
     }
-    ok = ok && w.Add(kEos, 8) && w.Flush();
-    wrote[p] = ok;
-  });
+    return ok && w.Add(kEos, 8);
+  };
+  if (total < kEmitBytes) {  // one writer: partitions lie behind one another
+    RangeWriter w(fd, mem, 0);
+    for (int p = 0; p < P_; p++) wrote[0] = wrote[0] && put(w, p);
+    wrote[0] = wrote[0] && w.Flush();
+  } else {
+    ParallelFor((size_t)P_, [&](size_t pi) {
+      RangeWriter w(fd, mem, start[pi]);
+      wrote[pi] = put(w, (int)pi) && w.Flush();
+    });
+  }
   bool ok = true;
   for (int p = 0; p < P_; p++) ok = ok && wrote[p];
   if (mapped && munmap(mapped, (size_t)total) != 0) ok = false;

@@ -25,6 +25,7 @@
 #include "host_util.h"
 #include "ipc.h"
 #include "schema_ipc.h"
+#include "stream_pool.h"
 
 namespace gz {
 
@@ -169,6 +170,7 @@ class Splitter {
     std::string spill_path;
     std::vector<size_t> off_values, off_bits, off_valid, off_chars;  // per array column, SIZE_MAX: none
     std::vector<size_t> off_cvalid;  // list columns: element validity bits (in the bit regions)
+    std::vector<uint32_t> zero_fb, last_fb;  // byte ranges' first start; [P][nstr] last ends
     uint32_t* h_meta = nullptr;         // pinned: rows_f, pstart, vstart, bytes_f, cstart, count, emit
     size_t bits_begin = 0, bits_end = 0;  // the bit regions (validity, bool values) in the output
     uint8_t* h_bits = nullptr;          // pinned copy of just the bit regions (compressed Stop)
@@ -192,7 +194,7 @@ class Splitter {
     int32_t flush;
     uint32_t frow0, frow1;  // flush-local rows of the partition
     uint32_t vpos0;         // flush-local validity bit of frow0
-    std::vector<uint32_t> fb0, fb1;  // flush-local byte range per binary column
+    const uint32_t *fb0, *fb1;  // flush-local byte range per binary column (in the pass's records)
   };
 
   struct Segment {  // one emitted record batch of one partition
@@ -322,6 +324,7 @@ class Splitter {
 
   // device
   int device_ = 0;
+  StreamSet streams_set_;            // the streams and events below
   cudaStream_t stream_ = nullptr;
   uint8_t* d_state_ = nullptr;      // persistent partition state
   uint32_t* st_cap_ = nullptr;
@@ -331,6 +334,7 @@ class Splitter {
   unsigned long long* st_ihn_ = nullptr;
   int32_t* d_err_ = nullptr;
   uint32_t* d_call_ = nullptr;
+  uint8_t* h_state_ = nullptr;       // pinned: the error word, then (256 bytes on) st_base_, st_hv_
   // The pass schedule: k_hash_count (with its pass's table copies and clears) on hstream_, the
   // plan kernels on pstream_, k_scatter on stream_.  With device-resident inputs a pass's
   // k_scatter is queued only when the next pass is (or at a sync), after that pass's k_hash_count
