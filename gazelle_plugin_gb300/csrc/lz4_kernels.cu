@@ -6,13 +6,16 @@
 // buffer is written as an int64 uncompressed length followed by one LZ4 frame.  Here the
 // buffers are cut into chunks of at most 8 KiB, each staged in shared memory and compressed by
 // one warp into one LZ4 block (greedy single-candidate matching, hash table in shared memory:
-// every read of the match search is a shared-memory read; 12 KiB of shared memory per warp, 16
+// every read of the match search is a shared-memory read; 12 KiB of shared memory per warp, 18
 // warps per SM), and the host strings the blocks of a buffer into a frame (independent blocks,
-// 64 KiB maximum block size in the descriptor, no checksums).  The search is bound by its
-// dependent instruction chains, so its speed follows the warps per SM and the latency of its
-// reads: against 64 KiB blocks searched in global memory, the Stop compression of the wide
+// 64 KiB maximum block size in the descriptor, no checksums).  The search is bound by the
+// instructions of its dependent chains, so its speed follows the warps per SM and the instructions per
+// sequence: against 64 KiB blocks searched in global memory, the Stop compression of the wide
 // fact-table bodies runs 2.1x faster, for 1.9% more output (an 8 KiB history); 16 KiB blocks (8
-// warps per SM) were 1.0x, 8 KiB blocks with a 4096-entry table (12 warps) 1.5x.  The output is
+// warps per SM) were 1.0x, 8 KiB blocks with a 4096-entry table (12 warps) 1.5x.  117 thousand
+// instructions per block of the wide table's worded columns (94 MB: 2.6 ms, 51% of the issue slots)
+// fell to 1.55 ms with short sequences written by one store, positions of the last window looked up
+// again instead of read and hashed again, and chunks staged in 16-byte words from any phase.  The output is
 // a valid frame for any LZ4 frame decoder; it is not the same byte string the LZ4 library would
 // produce (the codec's output is not unique).
 //
@@ -36,21 +39,13 @@ constexpr unsigned kFull = 0xffffffffu;
 constexpr int kWarps = 4;  // warps per CTA
 constexpr int kHashLog = 11;
 constexpr int kCWarps = 2;                       // warps per CTA of the compressor
-constexpr uint32_t kStage = kLz4MaxBlock + 16;   // a warp's staged chunk (and a zero-padded word)
+constexpr int kCBlocks = 9;                      // resident CTAs per SM (shared memory)
+constexpr uint32_t kStage = kLz4MaxBlock + 32;   // a warp's staged chunk, at its source's 16-byte phase
 constexpr size_t kCompressSmem = (size_t)kCWarps * (kStage + (2u << kHashLog));
+constexpr uint32_t kAgain = 24;  // window positions from which a new window is read instead (12, 20, 28, 32: 3, 0, 0, 10% slower)
 constexpr uint16_t kEmpty = 0xffff;  // no position (position 65535 never starts a match)
 
 __device__ __forceinline__ uint32_t lane_id() { return threadIdx.x & 31; }
-
-// Little-endian 4 bytes at chunk position q: two aligned words of the source funnel-shifted.
-// Both words hold bytes of the same source buffer (q + 4 <= len).
-__device__ __forceinline__ uint32_t read32(const uint32_t* base, uint32_t sh0, uint32_t q) {
-  const uint32_t i = sh0 + q;
-  const uint32_t w0 = __ldg(base + (i >> 2));
-  if ((i & 3) == 0) return w0;
-  const uint32_t w1 = __ldg(base + (i >> 2) + 1);
-  return __funnelshift_r(w0, w1, (i & 3) * 8);
-}
 
 __device__ __forceinline__ uint32_t hash4(uint32_t v) { return (v * 2654435761u) >> (32 - kHashLog); }
 
@@ -83,36 +78,48 @@ __device__ uint32_t emit(uint8_t* dst, uint32_t o, const uint8_t* src, uint32_t 
   return o;
 }
 
-// Compresses src[0, n) (n <= 65536) into dst (room for n + n / 255 + 16 bytes); returns the
+// A sequence like emit's whose lengths fit its token: lane j writes byte j, with one store.
+__device__ __forceinline__ uint32_t emit_short(uint8_t* dst, uint32_t o, const uint8_t* src, uint32_t anchor, uint32_t lit,
+                                               uint32_t off, uint32_t ml) {
+  const uint32_t j = lane_id();
+  uint32_t b = lit << 4 | ml;
+  if (j > lit) b = j == lit + 1 ? off : off >> 8;
+  if (j - 1 < lit) b = src[anchor + j - 1];
+  if (j < lit + 3) dst[o + j] = (uint8_t)b;
+  return o + lit + 3;
+}
+
+// Compresses the staged src[0, n) (n <= kLz4MaxBlock) into dst (room for n + n / 255 + 16 bytes); returns the
 // block's size.  Positions are scanned 32 at a time: every lane hashes its position's 4 bytes and
 // looks up the last earlier position with that hash; the first lane whose candidate matches
 // starts the match, which the warp then extends 32 bytes at a time.  Table entries come only from
 // earlier windows (inserted after the lookups), so a candidate always precedes its position.
-// Little-endian 4 bytes at position q of a staged (word-aligned, shared-memory) chunk.
-__device__ __forceinline__ uint32_t read32_s(const uint32_t* sw, uint32_t q) {
-  const uint32_t w0 = sw[q >> 2];
-  return (q & 3) == 0 ? w0 : __funnelshift_r(w0, sw[(q >> 2) + 1], (q & 3) * 8);
-}
-
 __device__ uint32_t compress_block(const uint8_t* src, uint32_t n, uint16_t* table, uint8_t* dst) {
   const uint32_t lane = lane_id();
-  const uint32_t* sw = reinterpret_cast<const uint32_t*>(src);  // the staged chunk (word aligned)
+  const uint32_t ph = (uint32_t)(reinterpret_cast<uintptr_t>(src) & 3);
+  const uint32_t* sw = reinterpret_cast<const uint32_t*>(src - ph);
+  // little-endian 4 bytes at position q (q + 8 <= n)
+  auto read4 = [&](uint32_t q) {
+    const uint32_t i = ph + q;
+    return __funnelshift_r(sw[i >> 2], sw[(i >> 2) + 1], (i & 3) * 8);
+  };
   uint32_t o = 0, anchor = 0, p = 0;
   uint32_t misses = 0;  // windows in a row without a match
   if (n >= 13) {
-    for (uint32_t i = lane; i < (1u << kHashLog); i += 32) table[i] = kEmpty;
+    for (uint32_t i = lane; i < (1u << kHashLog) / 8; i += 32)
+      reinterpret_cast<uint4*>(table)[i] = make_uint4(~0u, ~0u, ~0u, ~0u);  // kEmpty: past every position
     __syncwarp();
     while (p + 12 <= n) {
       const uint32_t q = p + lane;
       const bool valid = q + 12 <= n;
       uint32_t v = 0, h = 0, cand = kEmpty;
       if (valid) {
-        v = read32_s(sw, q);
+        v = read4(q);
         h = hash4(v);
         cand = table[h];
       }
-      const bool ok = valid && cand != kEmpty && cand < q && read32_s(sw, cand) == v;
-      const unsigned m = __ballot_sync(kFull, ok);
+      bool ok = cand < q && read4(cand) == v;
+      unsigned m = __ballot_sync(kFull, ok);
       __syncwarp();
       if (m == 0) {
         if (valid) table[h] = (uint16_t)q;
@@ -125,33 +132,48 @@ __device__ uint32_t compress_block(const uint8_t* src, uint32_t n, uint16_t* tab
         continue;
       }
       misses = 0;
-      const uint32_t f = __ffs(m) - 1;
-      if (valid && lane <= f) table[h] = (uint16_t)q;  // positions up to the match start only
-      const uint32_t mq = p + f;
-      const uint32_t mc = __shfl_sync(kFull, cand, f);
-      __syncwarp();
-      uint32_t len = 4;
-      for (;;) {  // the match may end at n - 5 at the latest
-        const uint32_t a = mq + len + lane;
-        const bool eq = a + 5 < n && src[a] == src[mc + len + lane];
-        const unsigned ne = __ballot_sync(kFull, !eq);
-        if (ne == 0) {
-          len += 32;
-          continue;
+      const uint32_t base = p;
+      for (uint32_t first = 0;;) {
+        // the match of lane f, the first with one from position base + first on
+        const uint32_t f = __ffs(m) - 1;
+        if (valid && lane >= first && lane <= f) table[h] = (uint16_t)q;  // positions up to the match start only
+        const uint32_t mq = base + f;
+        const uint32_t mc = __shfl_sync(kFull, cand, f);
+        __syncwarp();
+        uint32_t len = 4;
+        for (;;) {  // the match may end at n - 5 at the latest
+          const uint32_t a = mq + len + lane;
+          const bool eq = a + 5 < n && src[a] == src[mc + len + lane];
+          const unsigned ne = __ballot_sync(kFull, !eq);
+          if (ne == 0) {
+            len += 32;
+            continue;
+          }
+          len += __ffs(ne) - 1;
+          break;
         }
-        len += __ffs(ne) - 1;
-        break;
+        const uint32_t lit = mq - anchor;
+        o = lit < 15 && len < 19 ? emit_short(dst, o, src, anchor, lit, mq - mc, len - 4)
+                                 : emit(dst, o, src, anchor, lit, mq - mc, len);
+        p = mq + len;
+        anchor = p;
+        // The next window starts at p; a match of a position both windows hold is its first match as well,
+        // found by looking those positions up again (their bytes and hashes are at hand)
+        first = p - base;
+        if (first >= kAgain) break;
+        cand = valid && lane >= first ? table[h] : kEmpty;
+        ok = cand < q && read4(cand) == v;
+        m = __ballot_sync(kFull, ok);
+        __syncwarp();
+        if (m == 0) break;
       }
-      o = emit(dst, o, src, anchor, mq - anchor, mq - mc, len);
-      p = mq + len;
-      anchor = p;
     }
   }
   o = emit(dst, o, src, anchor, n - anchor, 0, 0);
   return o;
 }
 
-__global__ void __launch_bounds__(kCWarps * 32, 8)
+__global__ void __launch_bounds__(kCWarps * 32, kCBlocks)
 k_lz4_compress(const Lz4Chunk* __restrict__ chunks, uint32_t n_chunks, uint32_t* next, uint8_t* scratch,
                uint8_t* out, unsigned long long* out_used, unsigned long long out_cap, Lz4Block* res,
                bool skip_stored, int32_t* err) {
@@ -169,19 +191,14 @@ k_lz4_compress(const Lz4Chunk* __restrict__ chunks, uint32_t n_chunks, uint32_t*
     const uint32_t n = ch.raw || ch.len <= kLz4MaxBlock ? ch.len : 0;  // the host cuts blocks to 64 KiB
     uint32_t size = n;
     if (!ch.raw) {
-      // the chunk into this warp's shared buffer (then zeros up to two words past its end)
-      const uintptr_t a = reinterpret_cast<uintptr_t>(ch.src);
-      if ((a & 15) == 0) {
-        const uint32_t nv = n >> 4;
-        for (uint32_t i = lane_id(); i < nv; i += 32)
-          reinterpret_cast<uint4*>(sbuf)[i] = __ldg(reinterpret_cast<const uint4*>(ch.src) + i);
-        for (uint32_t i = (nv << 4) + lane_id(); i < n; i += 32) sbuf[i] = __ldg(ch.src + i);
-      } else {
-        for (uint32_t i = lane_id(); i < n; i += 32) sbuf[i] = __ldg(ch.src + i);
-      }
-      if (lane_id() < 8) sbuf[n + lane_id()] = 0;
+      // the chunk into this warp's shared buffer: the aligned 16-byte words that hold it (each holds a
+      // byte of the chunk, so none is outside its allocation)
+      const uint32_t phase = (uint32_t)(reinterpret_cast<uintptr_t>(ch.src) & 15);
+      const uint4* a = reinterpret_cast<const uint4*>(ch.src - phase);
+#pragma unroll 4
+      for (uint32_t i = lane_id(); i < (phase + n + 15) >> 4; i += 32) reinterpret_cast<uint4*>(sbuf)[i] = __ldg(a + i);
       __syncwarp();
-      size = compress_block(sbuf, n, table, slot);
+      size = compress_block(sbuf + phase, n, table, slot);
       __syncwarp();
     }
     const bool stored = size >= n;  // a plain copy, or no gain: the block is stored as it is
@@ -711,7 +728,7 @@ int sm_count() {
 
 }  // namespace
 
-uint32_t lz4_compress_warps() { return (uint32_t)sm_count() * 8 * kCWarps; }
+uint32_t lz4_compress_warps() { return (uint32_t)sm_count() * kCBlocks * kCWarps; }
 
 cudaError_t launch_lz4_compress(const Lz4Chunk* chunks, uint32_t n_chunks, uint32_t* next, uint8_t* scratch,
                                 uint8_t* out, unsigned long long* out_used, unsigned long long out_cap,
