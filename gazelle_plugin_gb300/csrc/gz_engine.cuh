@@ -106,6 +106,7 @@ struct HostCopy {
 constexpr uint32_t kGatherArgs = 128;
 struct GatherArgs {
   HostCopy job[kGatherArgs];
+  uint32_t first[kGatherArgs];  // first block of each buffer
 };
 
 // bits of FlushDesc::err

@@ -1597,16 +1597,16 @@ __device__ __forceinline__ void gather_words(const uint8_t* src, uint8_t* dst, u
   const uint64_t nv = (n - head) / W;
   const V* sv = reinterpret_cast<const V*>(src + head);
   V* dv = reinterpret_cast<V*>(dst + head);
-  constexpr int U = 4;  // loads in flight per thread
-  uint64_t i = threadIdx.x;
-  for (; i + (U - 1) * 256 < nv; i += U * 256) {
+  constexpr int U = 4;  // loads in flight per thread, also in the last round
+  for (uint64_t i = threadIdx.x; i < nv; i += U * 256) {
     V v[U];
 #pragma unroll
-    for (int u = 0; u < U; u++) v[u] = sv[i + u * 256];
+    for (int u = 0; u < U; u++)
+      if (i + u * 256 < nv) v[u] = sv[i + u * 256];
 #pragma unroll
-    for (int u = 0; u < U; u++) dv[i + u * 256] = v[u];
+    for (int u = 0; u < U; u++)
+      if (i + u * 256 < nv) dv[i + u * 256] = v[u];
   }
-  for (; i < nv; i += 256) dv[i] = sv[i];
   for (uint64_t j = head + nv * W + threadIdx.x; j < n; j += 256) dst[j] = src[j];
 }
 
@@ -1626,19 +1626,21 @@ __global__ void __launch_bounds__(256) k_gather(const HostCopy* __restrict__ job
 
 // k_gather_args: a call's reads of up to kGatherArgs buffers, the descriptors in the kernel's
 // parameters.  The caller waits for it before every split returns, so it is bound by latency: each
-// buffer is cut into pieces of two rounds of a block's loads (k_gather gives a buffer to one block: seven
+// buffer is cut into pieces of one round of a block's loads (k_gather gives a buffer to one block: seven
 // rounds over the link for the 110 KB of a 4096-row batch's comments, after one more for its
 // descriptor), and the last block tells the host itself, through a word the caller polls (an event
 // behind the kernel costs its record, the semaphore and the wait).  One task's split of a 4096-row,
-// 737 KB batch: 21.8 us with k_gather and an event, 15.7 us now.
-__global__ void __launch_bounds__(256) k_gather_args(const __grid_constant__ GatherArgs a, uint32_t piece,
-                                                     uint32_t n_pieces, uint32_t* done, volatile uint32_t* flag,
-                                                     uint32_t seq) {
-  const HostCopy job = a.job[blockIdx.y];
+// 737 KB batch: 21.8 us with k_gather and an event, 14.5 us now; of 64 rows: 13.5 and 10.5.
+__global__ void __launch_bounds__(256) k_gather_args(const __grid_constant__ GatherArgs a, uint32_t n_jobs, uint32_t piece,
+                                                     uint32_t* done, volatile uint32_t* flag, uint32_t seq) {
+  // the buffer of this block's piece: the last one whose first piece is not after it
+  uint32_t j = 0;
+  for (uint32_t step = kGatherArgs / 2; step; step >>= 1)
+    if (j + step < n_jobs && a.first[j + step] <= blockIdx.x) j += step;
+  const HostCopy job = a.job[j];
   // pieces start at multiples of 16 bytes of the source
   const uint32_t ph = (uint32_t)(reinterpret_cast<uintptr_t>(job.src) & 15);
-  const uint64_t end = job.bytes + ph, lo = (uint64_t)blockIdx.x * piece;
-  if (lo >= end) return;
+  const uint64_t end = job.bytes + ph, lo = (uint64_t)(blockIdx.x - a.first[j]) * piece;
   const uint64_t from = lo > ph ? lo - ph : 0, to = (lo + piece < end ? lo + piece : end) - ph;
   const uint8_t* src = job.src + from;
   uint8_t* dst = job.dst + from;
@@ -1648,13 +1650,13 @@ __global__ void __launch_bounds__(256) k_gather_args(const __grid_constant__ Gat
   } else if ((phase & 3) == 0) {
     gather_words<uint32_t>(src, dst, to - from);
   } else {
-    for (uint64_t j = threadIdx.x; j < to - from; j += 256) dst[j] = src[j];
+    for (uint64_t i = threadIdx.x; i < to - from; i += 256) dst[i] = src[i];
   }
   if (flag == nullptr) return;
   // Every load of the block has returned: the store of its value has been issued.  That is all the
   // host waits for (the stores' readers come later on the stream), so nothing is fenced.
   __syncthreads();
-  if (threadIdx.x == 0 && atomicAdd(done, 1u) == n_pieces - 1) {
+  if (threadIdx.x == 0 && atomicAdd(done, 1u) == gridDim.x - 1) {
     *done = 0;  // for the next launch on this stream
     *flag = seq;
   }
@@ -1776,22 +1778,22 @@ cudaError_t launch_gather_args(const HostCopy* jobs, uint32_t n_jobs, uint32_t* 
                                cudaStream_t st) {
   if (n_jobs == 0 || n_jobs > kGatherArgs) return n_jobs ? cudaErrorInvalidValue : cudaSuccess;
   GatherArgs a;
-  uint64_t most = 0, total = 0;
+  uint64_t total = 0;
   for (uint32_t i = 0; i < n_jobs; i++) {
     a.job[i] = jobs[i];
-    const uint64_t n = jobs[i].bytes + (reinterpret_cast<uintptr_t>(jobs[i].src) & 15);
-    most = n > most ? n : most;
-    total += n;
+    total += jobs[i].bytes;
   }
-  // two rounds of four 16-byte loads per thread (a 737 KB batch: 17.2 us a call with one round, 15.7
-  // with two, 17.6 with four), longer pieces where there are blocks enough anyway (5.9 MB: 42 us with
-  // 48 blocks or more, 50 with 16)
-  uint32_t piece = 32u << 10;
+  // one round of four 16-byte loads per thread (a 737 KB batch: 14.5 us a call from 4 to 16 KB pieces,
+  // 15.2 at 32 KB with two loads a thread), longer pieces where there are blocks enough anyway (5.9 MB:
+  // 41 us with 48 blocks or more, 50 with 16)
+  uint32_t piece = 16u << 10;
   while (piece < (1u << 20) && total / piece > 128) piece <<= 1;
   uint32_t n = 0;
-  for (uint32_t i = 0; i < n_jobs; i++)
+  for (uint32_t i = 0; i < n_jobs; i++) {
+    a.first[i] = n;
     n += (uint32_t)((jobs[i].bytes + (reinterpret_cast<uintptr_t>(jobs[i].src) & 15) + piece - 1) / piece);
-  k_gather_args<<<dim3((unsigned)((most + piece - 1) / piece), n_jobs), 256, 0, st>>>(a, piece, n, done, flag, seq);
+  }
+  k_gather_args<<<n, 256, 0, st>>>(a, n_jobs, piece, done, flag, seq);
   return cudaGetLastError();
 }
 
