@@ -212,3 +212,42 @@ def test_static_ids_and_counts_over_sizes(many_keys, P, shift):
         assert got[shift + n] == 0xFFFF  # nothing past the last row
         assert np.array_equal(counts.cpu().numpy(), np.bincount(want, minlength=P)), (n, P)
     del hold
+
+
+def test_static_calls_in_a_row_and_in_a_captured_graph(many_keys):
+    """Calls whose kernels may come up while the previous call's still run: each call reads the keys that
+    the kernel before it wrote and the scratch rows of its own counting kernel; the same in a graph."""
+    schema, batch, pids = many_keys
+    n, P = 20000, 2000
+    v = torch.from_numpy(batch.buffers[1].view(np.int64)[:n].copy()).cuda()
+    keys = [torch.empty_like(v) for _ in range(4)]
+    outs = [(torch.empty(n, dtype=torch.int16, device="cuda"), torch.empty(P, dtype=torch.int64, device="cuda")) for _ in keys]
+    cols = [(GzKeyColumn * 1)() for _ in keys]
+    for c, k in zip(cols, keys):
+        c[0].type, c[0].values, c[0].validity = W.TYPE_CODES["int64"], k.data_ptr(), None
+
+    def calls(stream):
+        for i, (k, (o, cnt)) in enumerate(zip(keys, outs)):
+            k.copy_(v + i)
+            assert _entry()(0, P, cols[i], 1, n, o.data_ptr(), cnt.data_ptr(), stream) == 0, _last_error()
+
+    def check():
+        for i, (o, cnt) in enumerate(outs):
+            b = W.Batch(n, [np.zeros(0, np.uint8), (v.cpu().numpy() + i).view(np.uint8)])
+            want = _oracle_pids([W.Field("k", "int64")], [0], P, b)
+            assert np.array_equal(o.cpu().numpy().view(np.uint16), want)
+            assert np.array_equal(cnt.cpu().numpy(), np.bincount(want, minlength=P))
+
+    calls(torch.cuda.current_stream().cuda_stream)
+    torch.cuda.synchronize()
+    check()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        calls(torch.cuda.current_stream().cuda_stream)
+    for _ in range(3):
+        for o, cnt in outs:
+            o.zero_()
+            cnt.zero_()
+        g.replay()
+        torch.cuda.synchronize()
+        check()
