@@ -29,6 +29,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "copy.cuh"
 #include "lz4_kernels.h"
 
 namespace gz {
@@ -334,11 +335,14 @@ __device__ bool decode_block(const uint8_t* src, uint32_t n, uint8_t* dst, uint6
 // three wide record batches (100 frames, 1.4 MB decoded), most SMs idle; one warp per block, staged
 // in shared memory: 261 us, still the chain (about 1000 sequences of 500 cycles).  The frames the
 // splitter writes hold independent blocks of at most kLz4MaxBlock bytes, so here
-//   k_lz4_blocks  gives every block a CTA that follows no chain: where the next token would be is
-//                 computed for every byte position at once, the positions reached from the first
-//                 are marked by pointer doubling (about ten rounds), the sequences' sizes are
-//                 scanned, and every output byte's source is followed to a literal by pointer
-//                 jumping.  Bound by instruction issue and shared memory (43 KiB: five CTAs per SM).
+//   k_lz4_blocks  gives every block a CTA that follows no long chain: where the next token would be is
+//                 computed for every byte position at once; every thread resolves where a chain leaves
+//                 its 32 positions, from the last one back, so one thread crosses the block in at most 256
+//                 steps; the threads whose positions it enters list their tokens, the sequences' sizes
+//                 are scanned, and every output byte's source is followed to a literal by pointer
+//                 jumping.  Bound by instruction issue and shared memory (43 KiB: five CTAs per SM):
+//                 67 us when the tokens were found by pointer doubling (ten rounds over all positions) and
+//                 every byte was looked at in every round of jumping; 22 us less per map output now.
 //                 Where a block's bytes go depends on the sizes of the blocks before it, so they
 //                 go to a slot of their own
 //   k_lz4_place   adds up the sizes and moves slots (and stored blocks) to their place
@@ -346,15 +350,15 @@ __device__ bool decode_block(const uint8_t* src, uint32_t n, uint8_t* dst, uint6
 // blocks than slots, malformed) is decoded as a whole by one warp of k_lz4_place.
 constexpr uint32_t kNoSlot = 0xffffffffu;      // the block cannot be decoded on its own
 constexpr int kDT = 256;                       // threads per block
-constexpr int kPer = kLz4MaxBlock / kDT;       // byte positions per thread
 constexpr uint32_t kInStage = kLz4MaxBlock + 64;   // + the phase of its first byte
 constexpr uint32_t kMaxSeq = kLz4MaxBlock / 4 + 1; // every match yields four bytes or more
 constexpr uint32_t kSeqRoom = (kMaxSeq + 1 + 7) & ~7u;
 constexpr uint32_t kPtrRoom = kLz4MaxBlock + 2 * (kLz4MaxBlock / 32);
-constexpr size_t kDecodeSmem = kInStage + 2 * kPtrRoom + 4 * 2 * kSeqRoom;
-static_assert(kLz4MaxBlock == kDT * 32, "a mark word per thread");
-static_assert(kDecodeSmem <= 46 * 1024, "five CTAs per SM, no opt-in");
-// index of output byte o in the pointer array: a thread's 32 bytes start in a bank of their own
+constexpr size_t kDecodeSmem = kInStage + 2 * 2 * kPtrRoom;
+static_assert(kLz4MaxBlock == kDT * 32, "32 positions per thread");
+static_assert(4 * kSeqRoom <= kPtrRoom, "the sequences' arrays fit over the exits");
+static_assert(kDecodeSmem <= 44 * 1024, "five CTAs per SM, no opt-in");
+// index of position / output byte o in an array: a thread's 32 entries start in a bank of their own
 __device__ __forceinline__ uint32_t swz(uint32_t o) { return o + 2 * (o >> 5); }
 
 // Reads and checks a frame's header; false when malformed.  *pos: its first block.
@@ -429,51 +433,43 @@ __device__ __forceinline__ uint32_t cta_exscan(uint32_t x, uint32_t* warp_sum, u
 // 16-byte aligned, room for cap bytes rounded up to 16); returns its size, or kNoSlot when it is
 // malformed, longer than `cap` or reaches back before its first byte.
 __device__ uint32_t decode_staged(const uint8_t* in, uint32_t n, uint32_t cap, uint16_t* ptr, uint16_t* seq,
-                                  uint32_t* marks, uint32_t* warp_sum, uint8_t* out) {
+                                  uint16_t* entry, uint32_t* warp_sum, uint8_t* out) {
   const uint32_t t = threadIdx.x;
   uint16_t* start = seq;                 // first output byte of each sequence
   uint16_t* mst = seq + kSeqRoom;        // its first match byte
   uint16_t* lpos = seq + 2 * kSeqRoom;   // its literals in the input
   uint16_t* offs = seq + 3 * kSeqRoom;   // its match offset
   uint32_t lit, lp, ml;
-  // where a sequence at each position would end: n the block's end, 0xffff nowhere
-  uint16_t* J = ptr;
-  for (uint32_t q = t; q < n; q += kDT) J[q] = (uint16_t)parse_seq(in, n, cap, q, &lit, &lp, &ml);
-  marks[t] = t == 0 ? 1u : 0u;
+  // next: where a sequence at each position would end: n the block's end, 0xffff nowhere
+  uint16_t* next = ptr;
+  for (uint32_t q = t; q < n; q += kDT) next[swz(q)] = (uint16_t)parse_seq(in, n, cap, q, &lit, &lp, &ml);
+  entry[t] = 0xffff;
   __syncthreads();
-  // J jumps 2^r sequences and the first 2^r are marked: until the first one's jump ends the block
-  while (J[0] < n) {
-    uint32_t nj[kPer / 2];
-#pragma unroll
-    for (int j = 0; j < kPer; j++) {
-      const uint32_t q = j * kDT + t;
-      if (j * kDT >= (int)n) break;
-      uint32_t v = 0;
-      if (q < n) {
-        v = J[q];
-        if (v < n) {
-          if ((marks[q >> 5] >> (q & 31)) & 1u) atomicOr(&marks[v >> 5], 1u << (v & 31));
-          v = J[v];
-        }
-      }
-      if (j & 1) nj[j >> 1] |= v << 16;
-      else nj[j >> 1] = v;
-    }
-    __syncthreads();
-#pragma unroll
-    for (int j = 0; j < kPer; j++) {
-      const uint32_t q = j * kDT + t;
-      if (j * kDT >= (int)n) break;
-      if (q < n) J[q] = (uint16_t)(nj[j >> 1] >> (16 * (j & 1)));
-    }
-    __syncthreads();
+  // leave: where the chain from each position first leaves its thread's 32 positions
+  uint16_t* leave = seq;
+  const uint32_t q0 = 32 * t, q1 = min(n, q0 + 32);
+  for (uint32_t q = q1; q-- > q0;) {  // (not entered when q1 < q0)
+    uint32_t x = next[swz(q)];
+    if (x < q1) x = leave[swz(x)];
+    leave[swz(q)] = (uint16_t)x;
   }
-  if (J[0] != n) return kNoSlot;
-  // the marked positions in order
-  uint32_t nseq, total;
-  uint32_t k = cta_exscan(__popc(marks[t]), warp_sum, &nseq);
+  __syncthreads();
+  if (t == 0) {
+    uint32_t q = 0;
+    do {
+      entry[q >> 5] = (uint16_t)q;
+      q = leave[swz(q)];
+    } while (q < n);
+    warp_sum[kDT / 32] = q;
+  }
+  __syncthreads();
+  if (warp_sum[kDT / 32] != n) return kNoSlot;
+  // the chain's positions in order
+  uint32_t nseq, total, mine = 0;
+  for (uint32_t q = entry[t]; q < q1; q = next[swz(q)]) mine++;
+  uint32_t k = cta_exscan(mine, warp_sum, &nseq);  // (its barriers: `leave` is read no more)
   if (nseq > kMaxSeq) return kNoSlot;
-  for (uint32_t m = marks[t]; m; m &= m - 1) lpos[k++] = (uint16_t)(32 * t + __ffs(m) - 1);
+  for (uint32_t q = entry[t]; q < q1; q = next[swz(q)]) lpos[k++] = (uint16_t)q;
   __syncthreads();
   // sizes, output starts, offsets: a thread takes sequences [k0, k1)
   const uint32_t per = (nseq + kDT - 1) / kDT;
@@ -534,18 +530,20 @@ __device__ uint32_t decode_staged(const uint8_t* in, uint32_t n, uint32_t cap, u
   }
   __syncthreads();
   // every source followed to its literal (a pointer read while its owner moves it on is an
-  // earlier one of the same chain: still right)
+  // earlier one of the same chain: still right); thread t keeps bytes t + 256 j, bit j not there yet
+  uint32_t todo = 0;
+  for (uint32_t j = 0; j < (total + kDT - 1 - t) / kDT; j++) todo |= 1u << j;
   for (;;) {
-    bool more = false;
-    for (uint32_t q = t; q < total; q += kDT) {
+    for (uint32_t m = todo; m; m &= m - 1) {
+      const uint32_t j = __ffs(m) - 1, q = j * kDT + t;
       uint32_t v = ptr[swz(q)];
       if (!(v & 0x8000u)) {
         v = ptr[swz(v)];
         ptr[swz(q)] = (uint16_t)v;
-        more |= !(v & 0x8000u);
       }
+      if (v & 0x8000u) todo &= ~(1u << j);
     }
-    if (!__syncthreads_or(more)) break;
+    if (!__syncthreads_or(todo)) break;
   }
   for (uint32_t w = t; w < (total + 3) >> 2; w += kDT) {
     // (bytes past the end come from whatever the array holds there, an index inside the stage)
@@ -562,8 +560,8 @@ __device__ uint32_t decode_staged(const uint8_t* in, uint32_t n, uint32_t cap, u
 __global__ void __launch_bounds__(kDT, 5) k_lz4_blocks(const Lz4Frame* __restrict__ frames, const uint32_t* __restrict__ frame_of,
                                                        Lz4Slot* __restrict__ slots, uint8_t* __restrict__ slot_mem) {
   extern __shared__ __align__(16) uint8_t dsm[];
-  __shared__ uint32_t marks[kDT];
-  __shared__ uint32_t warp_sum[kDT / 32];
+  __shared__ uint16_t entry[kDT];
+  __shared__ uint32_t warp_sum[kDT / 32 + 1];
   const uint32_t g = blockIdx.x;
   const Lz4Frame fr = frames[frame_of[g]];
   const uint32_t i = g - fr.slot0;
@@ -616,38 +614,12 @@ __global__ void __launch_bounds__(kDT, 5) k_lz4_blocks(const Lz4Frame* __restric
       __syncthreads();
       const uint32_t slot = lz4_slot_bytes(fr.dst_len);
       uint16_t* ptr = reinterpret_cast<uint16_t*>(dsm + kInStage);
-      sl.size = decode_staged(dsm + phase, sz, slot, ptr, ptr + kPtrRoom, marks, warp_sum,
+      sl.size = decode_staged(dsm + phase, sz, slot, ptr, ptr + kPtrRoom, entry, warp_sum,
                               slot_mem + fr.mem0 + (size_t)i * slot);
       if (sl.size != kNoSlot) sl.state = 3;
     }
   }
   if (threadIdx.x == 0) slots[g] = sl;
-}
-
-// n bytes from src to dst by one warp, in aligned 16- or 4-byte words of dst.
-__device__ void warp_copy(uint8_t* dst, const uint8_t* src, uint32_t n) {
-  const uint32_t lane = lane_id();
-  const uint32_t W = ((reinterpret_cast<uintptr_t>(src) ^ reinterpret_cast<uintptr_t>(dst)) & 15) == 0 ? 16u : 4u;
-  const uint32_t head = min(n, (uint32_t)(-reinterpret_cast<intptr_t>(dst) & (W - 1)));
-  if (lane < head) dst[lane] = src[lane];
-  dst += head;
-  src += head;
-  n -= head;
-  const uint32_t nv = n / W;
-  if (W == 16) {
-    const uint4* a = reinterpret_cast<const uint4*>(src);
-#pragma unroll 8
-    for (uint32_t q = lane; q < nv; q += 32) reinterpret_cast<uint4*>(dst)[q] = __ldg(a + q);
-  } else {
-    // a funnel shift of two aligned source words, each holding bytes of [src, src + n)
-    const uint32_t sh = (uint32_t)(reinterpret_cast<uintptr_t>(src) & 3) * 8;
-    const uint32_t* a = reinterpret_cast<const uint32_t*>(src - (sh >> 3));
-    const uint32_t up = sh ? 1u : 0u;
-#pragma unroll 8
-    for (uint32_t q = lane; q < nv; q += 32)
-      reinterpret_cast<uint32_t*>(dst)[q] = __funnelshift_r(__ldg(a + q), __ldg(a + q + up), sh);
-  }
-  for (uint32_t q = nv * W + lane; q < n; q += 32) dst[q] = src[q];
 }
 
 // The whole frame by one warp, its blocks in order (matches may reach back into earlier ones).
@@ -712,8 +684,8 @@ __global__ void __launch_bounds__(kWarps * 32) k_lz4_place(const Lz4Frame* __res
     return;
   }
   const Lz4Slot sl = slots[g];
-  if (sl.state == 2) warp_copy(fr.dst + before, fr.src + sl.pos, sl.size);
-  else if (sl.state == 3) warp_copy(fr.dst + before, slot_mem + fr.mem0 + (size_t)i * lz4_slot_bytes(fr.dst_len), sl.size);
+  if (sl.state == 2) copy_bytes<32>(fr.dst + before, fr.src + sl.pos, sl.size, lane);
+  else if (sl.state == 3) copy_bytes<32>(fr.dst + before, slot_mem + fr.mem0 + (size_t)i * lz4_slot_bytes(fr.dst_len), sl.size, lane);
 }
 
 int sm_count() {
