@@ -207,6 +207,7 @@ struct ForJob {
   std::function<void(size_t)> own;  // Background's function
   const std::function<void(size_t)>* fn;
   size_t n;
+  size_t step = 1;  // items claimed at a time
   std::atomic<size_t> next{0};
   std::atomic<size_t> done{0};
   std::mutex mu;
@@ -214,10 +215,11 @@ struct ForJob {
 
   void Work() {
     for (;;) {
-      const size_t i = next.fetch_add(1);
+      const size_t i = next.fetch_add(step);
       if (i >= n) return;
-      (*fn)(i);
-      if (done.fetch_add(1) + 1 == n) {
+      const size_t m = std::min(step, n - i);
+      for (size_t j = 0; j < m; j++) (*fn)(i + j);
+      if (done.fetch_add(m) + m == n) {
         std::lock_guard<std::mutex> lk(mu);
         cv.notify_all();
       }
@@ -276,6 +278,7 @@ void ParallelFor(size_t n, const std::function<void(size_t)>& fn, int max_helper
   auto job = std::make_shared<ForJob>();
   job->fn = &fn;
   job->n = n;
+  job->step = std::max<size_t>(1, std::min<size_t>(16, n / 256));
   ForPool& pool = ForPool::Get();
   const int helpers = (int)std::min<size_t>({(size_t)max_helpers, (size_t)pool.workers(), n - 1});
   pool.Post(job, helpers);

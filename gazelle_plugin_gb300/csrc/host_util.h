@@ -37,7 +37,8 @@ void ParallelCopy(const std::vector<CopyJob>& jobs, size_t total_bytes);
 
 // Runs fn(i) for every i in [0, n) on the calling thread and up to `max_helpers` threads of a
 // process-wide pool (shared by all splitters: concurrent calls share its workers); returns when
-// every fn(i) has returned.  Items are claimed one at a time, so long and short items balance.
+// every fn(i) has returned.  Items are claimed one at a time (a few at a time when there are hundreds),
+// so long and short items balance.
 void ParallelFor(size_t n, const std::function<void(size_t)>& fn, int max_helpers = 15);
 
 // Starts fn on up to `threads` threads of that pool and returns at once; fn runs at most that often

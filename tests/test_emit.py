@@ -1,4 +1,4 @@
-"""Stop's data file put together by the device (k_emit, from a megabyte of input on): the bytes of the
+"""Stop's data file put together by the device (k_emit, from four megabytes of input on): the bytes of the
 oracle, and with a codec those of the path that gathers them on the host (taken when local-dir spill
 files may hold passes), over host and device-resident inputs, one and many passes, data in a file
 and in memory, record batches that span passes, files of one and of many windows."""
@@ -66,9 +66,9 @@ def _run(schema, keys, P, batches, path, device=False, **kw):
     return data, r
 
 
-# (input, batches, partitions): a little over a megabyte, one window; several windows; many windows of
+# (input, batches, partitions): a little over that, two windows; several windows; many windows of
 # tiny partitions; lists, nested columns and null-type columns; one partition with pieces of megabytes
-CASES = [("c1", 14, 8), ("c2", 40, 200), ("c2", 40, 3000), ("nested", 12, 64), ("c2", 60, 1)]
+CASES = [("c1", 44, 8), ("c2", 40, 200), ("c2", 40, 3000), ("nested", 30, 64), ("c2", 60, 1)]
 
 
 @pytest.mark.parametrize("which,n,P", CASES)
@@ -76,7 +76,7 @@ CASES = [("c1", 14, 8), ("c2", 40, 200), ("c2", 40, 3000), ("nested", 12, 64), (
 @pytest.mark.parametrize("flush", [0, 1 << 20])
 def test_emit_equals_oracle(tmp_path, which, n, P, device, flush):
     schema, keys, batches = _batches(which, n)
-    assert sum(b.nbytes for b in batches) >= 1 << 20
+    assert sum(b.nbytes for b in batches) >= 4 << 20
     want = O.run_oracle(schema, batches, P, keys)
     opts = dict(flush_bytes=flush) if flush else {}
     for path in (str(tmp_path / "x.data"), ""):
@@ -95,11 +95,19 @@ def test_emit_lz4_equals_host_gather(tmp_path, which, n, P):
         assert got == want
 
 
+@pytest.mark.parametrize("which,n,P", [("c1", 1, 8), ("c1", 10, 2500), ("c2", 5, 64), ("nested", 6, 900)])
+def test_small_files_written_once_equal_oracle(tmp_path, which, n, P):
+    """Below that the CPU gathers the partitions and writes them with one call."""
+    schema, keys, batches = _batches(which, n)
+    data, _ = _run(schema, keys, P, batches, str(tmp_path / "x.data"))
+    assert data == O.run_oracle(schema, batches, P, keys).data
+
+
 def test_emit_rewrites_a_longer_file_and_reports_a_bad_path(tmp_path):
-    schema, keys, batches = _batches("c1", 14)
+    schema, keys, batches = _batches("c1", 44)
     path = str(tmp_path / "x.data")
     with open(path, "wb") as f:
-        f.write(b"\xee" * (8 << 20))
+        f.write(b"\xee" * (16 << 20))
     data, _ = _run(schema, keys, 8, batches, path)
     assert data == O.run_oracle(schema, batches, 8, keys).data
     with pytest.raises(S.SplitterError) as e:
