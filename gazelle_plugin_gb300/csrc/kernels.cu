@@ -387,9 +387,18 @@ __device__ __forceinline__ unsigned long long shfl64(unsigned long long v, int s
   return __shfl_sync(kFull, v, src);
 }
 
+// The four come up early (programmatic launches) and wait here for the one before them: a small pass is
+// a chain of launches.
+__device__ __forceinline__ void plan_begin() {
+  cudaTriggerProgrammaticLaunchCompletion();
+  cudaGridDependencySynchronize();
+}
+
 __global__ void __launch_bounds__(kPlanThreads) k_plan_prep(const SchemaDesc sd, const FlushDesc fd) {
   __shared__ unsigned long long s_warp[kPlanThreads / 32];
+  plan_begin();
   const int NB = fd.n_batches;
+  if (threadIdx.x == 0) *fd.emit_count = 0;
   const int A = sd.n_array;
   const int per = (NB + kPlanThreads - 1) / kPlanThreads;
   const int lo = threadIdx.x * per, hi = min(lo + per, NB);
@@ -399,6 +408,7 @@ __global__ void __launch_bounds__(kPlanThreads) k_plan_prep(const SchemaDesc sd,
     for (int a = 0; a < A; a++)
       if (fd.nullcnt[(size_t)b * A + a]) m |= 1ull << a;
     fd.hn[b] = m;
+    fd.call_flags[b] = 0;
     run |= m & sd.quirk_mask;
   }
   // exclusive OR-scan of the per-thread ORs across the block
@@ -426,6 +436,7 @@ __global__ void __launch_bounds__(kPlanThreads) k_plan_prep(const SchemaDesc sd,
 }
 
 __global__ void __launch_bounds__(kPlanRowsThreads) k_plan_rows(const SchemaDesc sd, const FlushDesc fd) {
+  plan_begin();
   const int P = sd.P;
   const int p = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   if (p >= P) return;  // whole warps exit together
@@ -572,6 +583,7 @@ __global__ void __launch_bounds__(kPlanRowsThreads) k_plan_rows(const SchemaDesc
 }
 
 __global__ void __launch_bounds__(kPlanRowsThreads) k_plan_bytes(const SchemaDesc sd, const FlushDesc fd) {
+  plan_begin();
   const int P = sd.P;
   const int nstr = sd.n_str;
   const int wid = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -640,12 +652,15 @@ __global__ void __launch_bounds__(kPlanRowsThreads) k_plan_bytes(const SchemaDes
   }
 }
 
+// One block per scan (one after another they took 7 us of a small pass, together 3).
 __global__ void __launch_bounds__(kPlanThreads) k_plan_scan(const SchemaDesc sd, const FlushDesc fd) {
   __shared__ uint32_t scan_scratch[33];
+  plan_begin();
   const int P = sd.P;
-  block_exscan<kPlanThreads>(fd.pstart, P, scan_scratch);
-  block_exscan<kPlanThreads>(fd.vstart, P, scan_scratch);
-  for (int k = 0; k < sd.n_str; k++) block_exscan<kPlanThreads>(fd.cstart + (size_t)k * P, P, scan_scratch);
+  uint32_t* data = blockIdx.x == 0 ? fd.pstart : blockIdx.x == 1 ? fd.vstart : fd.cstart + (size_t)(blockIdx.x - 2) * P;
+  block_exscan<kPlanThreads>(data, P, scan_scratch);
+  // the last batch's call flag, for the empirical-size bookkeeping
+  if (blockIdx.x == 0 && threadIdx.x == 0) *fd.call_last = fd.call_flags[fd.n_batches - 1];
 }
 
 // =======================================================================================
@@ -1736,21 +1751,25 @@ cudaError_t launch_hash_count(const SchemaDesc& sd, const FlushDesc& fd, cudaStr
 }
 
 cudaError_t launch_plan(const SchemaDesc& sd, const FlushDesc& fd, cudaStream_t st) {
-  k_plan_prep<<<1, kPlanThreads, 0, st>>>(sd, fd);
-  cudaError_t e = cudaGetLastError();
-  if (e != cudaSuccess) return e;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.stream = st;
+  cfg.attrs = at;
+  auto launch = [&](void (*k)(SchemaDesc, FlushDesc), int blocks, int threads) {
+    cfg.gridDim = (unsigned)blocks;
+    cfg.blockDim = (unsigned)threads;
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, k, sd, fd);
+    cfg.numAttrs = 1;  // the first waits for k_hash_count by an event
+    return e;
+  };
   const int wpb = kPlanRowsThreads / 32;
-  k_plan_rows<<<(sd.P + wpb - 1) / wpb, kPlanRowsThreads, 0, st>>>(sd, fd);
-  e = cudaGetLastError();
-  if (e != cudaSuccess) return e;
-  if (sd.n_str > 0) {
-    const int n = sd.n_str * sd.P;
-    k_plan_bytes<<<(n + wpb - 1) / wpb, kPlanRowsThreads, 0, st>>>(sd, fd);
-    e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
-  }
-  k_plan_scan<<<1, kPlanThreads, 0, st>>>(sd, fd);
-  return cudaGetLastError();
+  cudaError_t e = launch(k_plan_prep, 1, kPlanThreads);
+  if (e == cudaSuccess) e = launch(k_plan_rows, (sd.P + wpb - 1) / wpb, kPlanRowsThreads);
+  if (e == cudaSuccess && sd.n_str > 0) e = launch(k_plan_bytes, (sd.n_str * sd.P + wpb - 1) / wpb, kPlanRowsThreads);
+  if (e == cudaSuccess) e = launch(k_plan_scan, 2 + sd.n_str, kPlanThreads);
+  return e;
 }
 
 cudaError_t launch_nest_prep(const NestJob* jobs, uint32_t n_jobs, int32_t* err, cudaStream_t st) {

@@ -939,13 +939,19 @@ Status Splitter::Flush() {
   uint64_t emit_bound_a = 0;
   uint32_t smin = UINT32_MAX, capmax = (uint32_t)opts_.buffer_size;
   uint32_t NT = 0;  // tiles
+  // Passes with fewer segments than SMs get shorter ones (a segment's tiles are hashed one after
+  // another: four 3109-row batches of the wide table over 996 partitions 36.5 us with a segment each,
+  // 18.2 with one per tile), but not so many per batch that the plan's warps, which add them up one by
+  // one, wait longer than that.
+  const uint32_t few = opts_.seg_tiles > 0 ? seg_tiles_ : (uint32_t)std::min<size_t>(seg_tiles_, (pending_tiles_ + 151) / 152);
   segs.reserve(pending_tiles_);
   tiles.reserve(pending_tiles_);
   for (uint32_t b = 0; b < NB; b++) {
     const PendingBatch& pb = pending_[b];
     // as few segments as seg_tiles allows, of equal length (no short last segment)
     const uint32_t bt = (pb.nrows + kTileRows - 1) / kTileRows;
-    const uint32_t ns = (bt + seg_tiles_ - 1) / seg_tiles_;
+    const uint32_t st_b = std::max(few, std::min(seg_tiles_, (bt + 7) / 8));
+    const uint32_t ns = (bt + st_b - 1) / st_b;
     const uint32_t seg_rows = ns ? (bt + ns - 1) / ns * (uint32_t)kTileRows : (uint32_t)kTileRows;
     batches[b] = BatchDesc{pb.nrows, (uint32_t)segs.size(), ns, pb.split_size};
     for (uint32_t g = 0; g < ns; g++) {
@@ -1122,6 +1128,7 @@ Status Splitter::Flush() {
   fd.tilepre = tile_prefix ? reinterpret_cast<uint32_t*>(S + s_tpre) : nullptr;
   fd.tilebpre = tile_prefix ? reinterpret_cast<uint32_t*>(S + s_tbpre) : nullptr;
   fd.call_flags = reinterpret_cast<uint32_t*>(S + s_call);
+  fd.call_last = d_call_;
   fd.rec_idx = reinterpret_cast<uint32_t*>(S + s_rec);
   fd.hn = reinterpret_cast<unsigned long long*>(S + s_hn);
   fd.ihn = reinterpret_cast<unsigned long long*>(S + s_ihn);
@@ -1230,10 +1237,6 @@ Status Splitter::Flush() {
 
   st = Cuda(cudaMemsetAsync(S + s_null, 0, (size_t)NB * A * 4, hstream_), "memset");
   if (!st.ok()) return st;
-  st = Cuda(cudaMemsetAsync(S + s_call, 0, (size_t)NB * 4, hstream_), "memset");
-  if (!st.ok()) return st;
-  st = Cuda(cudaMemsetAsync(fd.emit_count, 0, 4, hstream_), "memset");
-  if (!st.ok()) return st;
   if (!fd.hist_in_smem) {
     st = Cuda(cudaMemsetAsync(S + s_cnt, 0, TP * 4, hstream_), "memset");
     if (!st.ok()) return st;
@@ -1263,9 +1266,6 @@ Status Splitter::Flush() {
   st = Cuda(launch_plan(sd_, fd, pstream_), "k_plan");
   if (!st.ok()) return st;
   cudaEventRecord(fr.ev[2], pstream_);
-  // the last batch's call flag, for the empirical-size bookkeeping
-  st = Cuda(cudaMemcpyAsync(d_call_, fd.call_flags + (NB - 1), 4, cudaMemcpyDeviceToDevice, pstream_), "D2D");
-  if (!st.ok()) return st;
   // flush metadata to pinned host memory
   fr.meta_words = meta_words;
   st = PinnedMeta(meta_words * 4, &fr.h_meta);
