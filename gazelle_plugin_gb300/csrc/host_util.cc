@@ -269,8 +269,21 @@ class ForPool {
 
 }  // namespace
 
+namespace {
+std::atomic<int> g_users{0};
+}  // namespace
+
+ParallelUser::ParallelUser() { g_users.fetch_add(1); }
+ParallelUser::~ParallelUser() { g_users.fetch_sub(1); }
+
+int ParallelHelpers(int most) {
+  const int workers = ForPool::Get().workers();
+  return std::min(most, std::max(0, (workers + 1) / std::max(1, g_users.load()) - 1));
+}
+
 void ParallelFor(size_t n, const std::function<void(size_t)>& fn, int max_helpers) {
   if (n == 0) return;
+  if (n > 1) max_helpers = ParallelHelpers(max_helpers);
   if (n == 1 || max_helpers <= 0) {
     for (size_t i = 0; i < n; i++) fn(i);
     return;
@@ -279,23 +292,20 @@ void ParallelFor(size_t n, const std::function<void(size_t)>& fn, int max_helper
   job->fn = &fn;
   job->n = n;
   job->step = std::max<size_t>(1, std::min<size_t>(16, n / 256));
-  ForPool& pool = ForPool::Get();
-  const int helpers = (int)std::min<size_t>({(size_t)max_helpers, (size_t)pool.workers(), n - 1});
-  pool.Post(job, helpers);
+  ForPool::Get().Post(job, (int)std::min<size_t>((size_t)max_helpers, n - 1));
   job->Work();
   std::unique_lock<std::mutex> lk(job->mu);
   job->cv.wait(lk, [&] { return job->done.load() == n; });
 }
 
 void Background(int threads, const std::function<void()>& fn) {
-  ForPool& pool = ForPool::Get();
-  const int n = std::min(threads, pool.workers());
+  const int n = ParallelHelpers(threads);
   if (n <= 0) return;
   auto job = std::make_shared<ForJob>();
   job->own = [fn](size_t) { fn(); };
   job->fn = &job->own;
   job->n = (size_t)n;
-  pool.Post(job, n);
+  ForPool::Get().Post(job, n);
 }
 
 void ParallelCopy(const std::vector<CopyJob>& jobs, size_t total_bytes) {

@@ -41,6 +41,18 @@ void ParallelCopy(const std::vector<CopyJob>& jobs, size_t total_bytes);
 // so long and short items balance.
 void ParallelFor(size_t n, const std::function<void(size_t)>& fn, int max_helpers = 15);
 
+// A caller about to use the pool's threads a number of times (a task's Stop): while several do, each
+// gets its share of them (16 tasks that stop at once, 283 MB, wake and contend for 15 workers otherwise:
+// 9.7 to 11.2 ms, 8.9 to 9.1 with shares).
+struct ParallelUser {
+  ParallelUser();
+  ~ParallelUser();
+  ParallelUser(const ParallelUser&) = delete;
+  ParallelUser& operator=(const ParallelUser&) = delete;
+};
+// The share, at most `most`.
+int ParallelHelpers(int most);
+
 // Starts fn on up to `threads` threads of that pool and returns at once; fn runs at most that often
 // (not at all while the pool is busy), possibly after the caller is done: it owns what it uses.
 void Background(int threads, const std::function<void()>& fn);

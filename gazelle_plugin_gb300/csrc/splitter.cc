@@ -1851,6 +1851,7 @@ Status Splitter::Stop() {
   if (stopped_) return Status::Error(GZ_INVALID, "splitter already stopped");
   Status st = Cuda(cudaSetDevice(device_), "cudaSetDevice");
   if (!st.ok()) return st;
+  const ParallelUser user;
   emit_at_stop_ = EmitAtStop();
   st = Drain();
   if (!st.ok()) return st;
@@ -2083,7 +2084,6 @@ struct PageToucher {
 
 // Bytes of the files this process is writing through mappings without having allocated them.
 std::atomic<int64_t> g_unallocated{0};
-std::atomic<int> g_emitting{0};  // files this process is writing through mappings
 
 // Whether `total` more bytes go into the file system of `fd` with room to spare: then its pages are
 // allocated by their first touch.  Allocating them beforehand serialises on the file's lock (a 720 MB
@@ -2131,11 +2131,8 @@ Status Splitter::EmitData(const std::vector<std::vector<SegMsg>>& msgs, const st
   if (map) {
     pages = std::make_shared<PageToucher>(map, fd, total, W, !spare);
     if (fd >= 0 && spare) g_unallocated.fetch_add(total);
-    // eight threads in all: more only contend (720 MB of tmpfs pages: 8.7 ms with 4, 6.3 with 8, 7.3 with
-    // 16), also those of other tasks' files (16 tasks, 283 MB: 11.2 ms with seven helpers each, 9.6 with none)
-    const int cores = (int)std::max(1u, std::thread::hardware_concurrency());
-    const int helpers = std::min(7, cores / (g_emitting.fetch_add(1) + 1) - 1);
-    Background((int)std::min<int64_t>(helpers, total / pages->unit), [pages] {
+    // eight threads in all: more only contend (720 MB of tmpfs pages: 8.7 ms with 4, 6.3 with 8, 7.3 with 16)
+    Background((int)std::min<int64_t>(7, total / pages->unit), [pages] {
       while (pages->Work()) {
       }
     });
@@ -2145,7 +2142,6 @@ Status Splitter::EmitData(const std::vector<std::vector<SegMsg>>& msgs, const st
   if (pages) {
     for (size_t w = 0; w < nw; w++) pages->Wait(w);  // nobody touches the mapping any more
     if (fd >= 0 && spare) g_unallocated.fetch_sub(total);
-    g_emitting.fetch_sub(1);
   }
   if (fd >= 0) {
     bool ok = true;
