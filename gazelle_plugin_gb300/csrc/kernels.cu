@@ -1613,16 +1613,17 @@ __device__ __forceinline__ void gather_words(const uint8_t* src, uint8_t* dst, u
   const V* sv = reinterpret_cast<const V*>(src + head);
   V* dv = reinterpret_cast<V*>(dst + head);
   constexpr int U = 4;  // loads in flight per thread, also in the last round
-  for (uint64_t i = threadIdx.x; i < nv; i += U * 256) {
+  const uint32_t T = blockDim.x;
+  for (uint64_t i = threadIdx.x; i < nv; i += U * T) {
     V v[U];
 #pragma unroll
     for (int u = 0; u < U; u++)
-      if (i + u * 256 < nv) v[u] = sv[i + u * 256];
+      if (i + u * T < nv) v[u] = sv[i + u * T];
 #pragma unroll
     for (int u = 0; u < U; u++)
-      if (i + u * 256 < nv) dv[i + u * 256] = v[u];
+      if (i + u * T < nv) dv[i + u * T] = v[u];
   }
-  for (uint64_t j = head + nv * W + threadIdx.x; j < n; j += 256) dst[j] = src[j];
+  for (uint64_t j = head + nv * W + threadIdx.x; j < n; j += T) dst[j] = src[j];
 }
 
 __global__ void __launch_bounds__(256) k_gather(const HostCopy* __restrict__ jobs, uint32_t n_jobs) {
@@ -1646,15 +1647,15 @@ __global__ void __launch_bounds__(256) k_gather(const HostCopy* __restrict__ job
 // descriptor), and the last block tells the host itself, through a word the caller polls (an event
 // behind the kernel costs its record, the semaphore and the wait).  One task's split of a 4096-row,
 // 737 KB batch: 21.8 us with k_gather and an event, 14.5 us now; of 64 rows: 13.5 and 10.5.
-__global__ void __launch_bounds__(256) k_gather_args(const __grid_constant__ GatherArgs a, uint32_t n_jobs, uint32_t piece,
-                                                     uint32_t* done, volatile uint32_t* flag, uint32_t seq) {
+__global__ void __launch_bounds__(1024) k_gather_args(const __grid_constant__ GatherArgs a, uint32_t n_jobs, uint32_t piece,
+                                                      uint32_t align, uint32_t* done, volatile uint32_t* flag, uint32_t seq) {
   // the buffer of this block's piece: the last one whose first piece is not after it
   uint32_t j = 0;
   for (uint32_t step = kGatherArgs / 2; step; step >>= 1)
     if (j + step < n_jobs && a.first[j + step] <= blockIdx.x) j += step;
   const HostCopy job = a.job[j];
-  // pieces start at multiples of 16 bytes of the source
-  const uint32_t ph = (uint32_t)(reinterpret_cast<uintptr_t>(job.src) & 15);
+  // pieces start at multiples of `align` of the source
+  const uint32_t ph = (uint32_t)(reinterpret_cast<uintptr_t>(job.src) & (align - 1));
   const uint64_t end = job.bytes + ph, lo = (uint64_t)(blockIdx.x - a.first[j]) * piece;
   const uint64_t from = lo > ph ? lo - ph : 0, to = (lo + piece < end ? lo + piece : end) - ph;
   const uint8_t* src = job.src + from;
@@ -1665,7 +1666,7 @@ __global__ void __launch_bounds__(256) k_gather_args(const __grid_constant__ Gat
   } else if ((phase & 3) == 0) {
     gather_words<uint32_t>(src, dst, to - from);
   } else {
-    for (uint64_t i = threadIdx.x; i < to - from; i += 256) dst[i] = src[i];
+    for (uint64_t i = threadIdx.x; i < to - from; i += blockDim.x) dst[i] = src[i];
   }
   if (flag == nullptr) return;
   // Every load of the block has returned: the store of its value has been issued.  That is all the
@@ -1797,27 +1798,46 @@ cudaError_t launch_gather(const HostCopy* jobs, uint32_t n_jobs, cudaStream_t st
   return cudaGetLastError();
 }
 
+namespace {
+cudaError_t gather_args(const HostCopy* jobs, uint32_t n_jobs, uint32_t threads, uint32_t piece, uint32_t align, uint32_t* done,
+                        uint32_t* flag, uint32_t seq, cudaStream_t st) {
+  GatherArgs a;
+  uint32_t n = 0;
+  for (uint32_t i = 0; i < n_jobs; i++) {
+    a.job[i] = jobs[i];
+    a.first[i] = n;
+    n += (uint32_t)((jobs[i].bytes + (reinterpret_cast<uintptr_t>(jobs[i].src) & (align - 1)) + piece - 1) / piece);
+  }
+  k_gather_args<<<n, threads, 0, st>>>(a, n_jobs, piece, align, done, flag, seq);
+  return cudaGetLastError();
+}
+}  // namespace
+
 cudaError_t launch_gather_args(const HostCopy* jobs, uint32_t n_jobs, uint32_t* done, uint32_t* flag, uint32_t seq,
                                cudaStream_t st) {
   if (n_jobs == 0 || n_jobs > kGatherArgs) return n_jobs ? cudaErrorInvalidValue : cudaSuccess;
-  GatherArgs a;
-  uint64_t total = 0;
-  for (uint32_t i = 0; i < n_jobs; i++) {
-    a.job[i] = jobs[i];
-    total += jobs[i].bytes;
-  }
   // one round of four 16-byte loads per thread (a 737 KB batch: 14.5 us a call from 4 to 16 KB pieces,
   // 15.2 at 32 KB with two loads a thread), longer pieces where there are blocks enough anyway (5.9 MB:
   // 41 us with 48 blocks or more, 50 with 16)
+  uint64_t total = 0;
+  for (uint32_t i = 0; i < n_jobs; i++) total += jobs[i].bytes;
   uint32_t piece = 16u << 10;
   while (piece < (1u << 20) && total / piece > 128) piece <<= 1;
-  uint32_t n = 0;
-  for (uint32_t i = 0; i < n_jobs; i++) {
-    a.first[i] = n;
-    n += (uint32_t)((jobs[i].bytes + (reinterpret_cast<uintptr_t>(jobs[i].src) & 15) + piece - 1) / piece);
-  }
-  k_gather_args<<<n, 256, 0, st>>>(a, n_jobs, piece, done, flag, seq);
-  return cudaGetLastError();
+  return gather_args(jobs, n_jobs, 256, piece, 16, done, flag, seq, st);
+}
+
+cudaError_t launch_gather_stream(const HostCopy& job, cudaStream_t st) {
+  if (job.bytes == 0) return cudaSuccess;
+  // A reduce task's streams are pages of data files the device has not seen before: every SM that reads a
+  // page asks the host for its translation, so from 256 KB on few blocks read whole pages (64 KB, a
+  // round of a block's loads) one after another; four or five keep the link busy.  2.3 MB streams, 1 / 4 /
+  // 16 readers at once: 44 / 83 / 112 GB/s in 512 KB pieces, 44 / 68 / 86 in 128 KB ones, 42 / 47 / 61 in
+  // 64 KB ones (256 threads, 256 KB from the stream's start on: 29 / 72 / 111).  Eight loads a thread:
+  // 45 / 89 / 113, but 2.12 ms instead of 1.94 for 141 MB of pages already translated.
+  constexpr uint64_t page = 64u << 10;
+  if (job.bytes < 4 * page) return gather_args(&job, 1, 256, 16u << 10, 16, nullptr, nullptr, 0, st);
+  const uint64_t piece = (job.bytes / 4 + page - 1) / page * page;
+  return gather_args(&job, 1, 1024, (uint32_t)(piece < 8 * page ? piece : 8 * page), (uint32_t)page, nullptr, nullptr, 0, st);
 }
 
 size_t scatter_smem_bytes() {

@@ -336,7 +336,7 @@ Status PartitionReader::AddStream(const uint8_t* data, int64_t len) {
     // device itself where it walks the host page tables, else by a copy
     if (direct_) {
       const HostCopy job{data, d, (uint64_t)len};
-      st = Cuda(launch_gather_args(&job, 1, nullptr, nullptr, 0, stream_), "k_gather");
+      st = Cuda(launch_gather_stream(job, stream_), "k_gather");
     } else {
       st = Cuda(cudaMemcpyAsync(d, data, (size_t)len, cudaMemcpyHostToDevice, stream_), "H2D stream");
     }

@@ -199,3 +199,23 @@ def test_gpu_reader_errors():
     with pytest.raises(S.SplitterError):
         r.addStream(s)  # finished
     r.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("offset", [0, 1, 8, 20, 65528])
+@pytest.mark.parametrize("rows", [32000, 32760, 33000, 65600, 300000])
+def test_gpu_reader_stream_sizes_and_starts(rows, offset):
+    """Streams around 256 KB, from which on the device reads them in whole 64 KB pages by few large
+    blocks, and of several pieces, at any start within a page."""
+    schema = [W.Field("k", "int64", False)]
+    rng = np.random.default_rng(rows)
+    batches = [W.Batch(n, W._column(rng, schema[0], n, rng.integers(0, 1 << 40, size=n), 0.0))
+               for n in (rows // 2, rows - rows // 2)]
+    s = np.frombuffer(O.run_oracle(schema, batches, 1, [0]).partition_bytes(0), np.uint8)
+    buf = np.zeros(s.size + (1 << 18), np.uint8)
+    at = (-buf.ctypes.data) % 65536 + offset
+    buf[at:at + s.size] = s
+    _, cols = R.read_partition(schema, [s.tobytes()] * 2)
+    grows, _, gcols = _gpu_read(schema, [buf[at:at + s.size], s])
+    assert grows == 2 * rows
+    assert gcols[0][2].tobytes() == cols[0][2]
