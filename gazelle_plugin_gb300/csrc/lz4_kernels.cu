@@ -257,7 +257,7 @@ k_lz4_compress(const Lz4Chunk* __restrict__ chunks, uint32_t n_chunks, uint32_t*
 
 // xxHash32 of a few bytes (the frame descriptor), seed 0: the published algorithm's path for
 // inputs shorter than 16 bytes.
-__device__ uint32_t xxh32_short(const uint8_t* p, uint32_t n) {
+__host__ __device__ uint32_t xxh32_short(const uint8_t* p, uint32_t n) {
   constexpr uint32_t P1 = 2654435761u, P2 = 2246822519u, P3 = 3266489917u, P4 = 668265263u, P5 = 374761393u;
   uint32_t h = P5 + n;
   uint32_t i = 0;
@@ -278,7 +278,7 @@ __device__ uint32_t xxh32_short(const uint8_t* p, uint32_t n) {
   return h;
 }
 
-__device__ __forceinline__ uint32_t le32(const uint8_t* p) {
+__host__ __device__ __forceinline__ uint32_t le32(const uint8_t* p) {
   return (uint32_t)p[0] | (uint32_t)p[1] << 8 | (uint32_t)p[2] << 16 | (uint32_t)p[3] << 24;
 }
 
@@ -335,34 +335,50 @@ __device__ bool decode_block(const uint8_t* src, uint32_t n, uint8_t* dst, uint6
 // three wide record batches (100 frames, 1.4 MB decoded), most SMs idle; one warp per block, staged
 // in shared memory: 261 us, still the chain (about 1000 sequences of 500 cycles).  The frames the
 // splitter writes hold independent blocks of at most kLz4MaxBlock bytes, so here
+//   lz4_index     finds the blocks from the frames' headers, on the host while the device reads the stream
 //   k_lz4_blocks  gives every block a CTA that follows no long chain: where the next token would be is
-//                 computed for every byte position at once; every thread resolves where a chain leaves
-//                 its 32 positions, from the last one back, so one thread crosses the block in at most 256
-//                 steps; the threads whose positions it enters list their tokens, the sequences' sizes
-//                 are scanned, and every output byte's source is followed to a literal by pointer
-//                 jumping.  Bound by instruction issue and shared memory (43 KiB: five CTAs per SM):
-//                 67 us when the tokens were found by pointer doubling (ten rounds over all positions) and
-//                 every byte was looked at in every round of jumping; 22 us less per map output now.
+//                 computed for every byte position at once; a warp's shuffles find where the chain from each
+//                 of 32 positions leaves them, one pass more where it leaves a warp's 512; so one thread
+//                 crosses the block in at most 16 steps and one a warp its part in 16 more; the threads
+//                 whose positions are entered list their tokens, the sequences' sizes are scanned, and
+//                 every output byte's source is followed to a literal by pointer jumping, 16 bytes in a
+//                 thread's registers.  Bound by instruction issue (parsing every position and the sources
+//                 take a fifth each; 16 warps, two CTAs per SM: three spilled or, with 40 registers,
+//                 took longer for the last ones to finish).  Both kernels for a map output of 242
+//                 compressed blocks: 80 us with the tokens found by ten rounds of pointer doubling, 55
+//                 with a thread per 32 positions and 256 steps, 35 now.
 //                 Where a block's bytes go depends on the sizes of the blocks before it, so they
 //                 go to a slot of their own
-//   k_lz4_place   adds up the sizes and moves slots (and stored blocks) to their place
+//   k_lz4_place   adds up the sizes and moves slots (and stored blocks) to their place, 128 threads each (a
+//                 warp each took 12 us)
 // A frame that is anything else (blocks that reach back into earlier ones, larger blocks, more
 // blocks than slots, malformed) is decoded as a whole by one warp of k_lz4_place.
-constexpr uint32_t kNoSlot = 0xffffffffu;      // the block cannot be decoded on its own
-constexpr int kDT = 256;                       // threads per block
+constexpr uint32_t kNoSlot = kLz4NoSlot;
+constexpr int kDT = 512;                       // threads per block
+constexpr int kSegs = kLz4MaxBlock / 32;       // segments of 32 positions, a warp's lanes each
+constexpr int kGroups = kDT / 32;              // groups of segments, a warp each
+constexpr int kOut = kLz4MaxBlock / kDT;       // output bytes of a thread
 constexpr uint32_t kInStage = kLz4MaxBlock + 64;   // + the phase of its first byte
 constexpr uint32_t kMaxSeq = kLz4MaxBlock / 4 + 1; // every match yields four bytes or more
-constexpr uint32_t kSeqRoom = (kMaxSeq + 1 + 7) & ~7u;
-constexpr uint32_t kPtrRoom = kLz4MaxBlock + 2 * (kLz4MaxBlock / 32);
-constexpr size_t kDecodeSmem = kInStage + 2 * 2 * kPtrRoom;
-static_assert(kLz4MaxBlock == kDT * 32, "32 positions per thread");
-static_assert(4 * kSeqRoom <= kPtrRoom, "the sequences' arrays fit over the exits");
-static_assert(kDecodeSmem <= 44 * 1024, "five CTAs per SM, no opt-in");
-// index of position / output byte o in an array: a thread's 32 entries start in a bank of their own
+constexpr uint32_t kPosRoom = kLz4MaxBlock + 2 * kSegs;
+constexpr uint32_t kPtrRoom = kLz4MaxBlock + 2 * kDT;
+constexpr uint32_t kChainEnd = kPosRoom - 2;   // entries that no position has: the block's end reached,
+constexpr uint32_t kChainBad = kPosRoom - 1;   // or a sequence that cannot be
+struct __align__(8) Seq {
+  uint16_t start, mst;  // its first output byte, its first match byte
+  uint16_t lpos, offs;  // its literals in the input, its match offset
+};
+constexpr size_t kDecodeSmem = kInStage + 2 * (kPtrRoom + 2 * kPosRoom);
+static_assert(kOut == 16 && kSegs % kGroups == 0, "a thread's bytes go out in one store");
+static_assert(kPtrRoom >= kPosRoom && sizeof(Seq) * (kMaxSeq + 1) <= 2 * kPosRoom, "what lies over what");
+static_assert(kDecodeSmem <= 61 * 1024, "three CTAs per SM");
+// index of position o (swz: a segment's 32 entries start in a bank of their own) and of output byte o
+// (a thread's 16)
 __device__ __forceinline__ uint32_t swz(uint32_t o) { return o + 2 * (o >> 5); }
+__device__ __forceinline__ uint32_t swz_out(uint32_t o) { return o + 2 * (o >> 4); }
 
 // Reads and checks a frame's header; false when malformed.  *pos: its first block.
-__device__ bool frame_header(const uint8_t* s, uint64_t n, uint64_t* pos, bool* block_sum, bool* content_sum) {
+__host__ __device__ bool frame_header(const uint8_t* s, uint64_t n, uint64_t* pos, bool* block_sum, bool* content_sum) {
   if (n < 7 || le32(s) != 0x184D2204u) return false;
   const uint8_t flg = s[4], bd = s[5];
   *block_sum = flg & 0x10;
@@ -409,6 +425,35 @@ __device__ __forceinline__ uint32_t parse_seq(const uint8_t* in, uint32_t n, uin
   return p;
 }
 
+// Where the sequence at position `at` of the staged block ends, or kNoSlot when it is cut off; its lengths
+// are checked where they are needed.  (A length byte is read before it is known to be inside the block:
+// one byte past it at most, inside the stage.)
+__device__ __forceinline__ uint32_t next_seq(const uint8_t* in, uint32_t n, uint32_t at) {
+  const uint32_t token = in[at];
+  uint32_t p = at + 1, b;
+  if (token >= 0xf0) {
+    b = in[p++];
+    uint32_t l = b;
+    while (b == 255 && p < n) {
+      b = in[p++];
+      l += b;
+    }
+    p += l;
+  }
+  p += token >> 4;
+  if (p == n) return n;
+  p += 2;
+  if (p > n) return kNoSlot;
+  if ((token & 15) == 15) {
+    do {
+      b = in[p++];
+    } while (b == 255 && p < n);
+    // (cut off when the last byte says that more follow)
+    if (p > n || b == 255) return kNoSlot;
+  }
+  return p;
+}
+
 // Exclusive scan of x over the CTA; *total gets the sum.
 __device__ __forceinline__ uint32_t cta_exscan(uint32_t x, uint32_t* warp_sum, uint32_t* total) {
   uint32_t inc = x;
@@ -431,195 +476,171 @@ __device__ __forceinline__ uint32_t cta_exscan(uint32_t x, uint32_t* warp_sum, u
 
 // Decodes the block staged at `in` (n >= 1 bytes) on its own, by the whole CTA, into `out` (global,
 // 16-byte aligned, room for cap bytes rounded up to 16); returns its size, or kNoSlot when it is
-// malformed, longer than `cap` or reaches back before its first byte.
-__device__ uint32_t decode_staged(const uint8_t* in, uint32_t n, uint32_t cap, uint16_t* ptr, uint16_t* seq,
-                                  uint16_t* entry, uint32_t* warp_sum, uint8_t* out) {
-  const uint32_t t = threadIdx.x;
-  uint16_t* start = seq;                 // first output byte of each sequence
-  uint16_t* mst = seq + kSeqRoom;        // its first match byte
-  uint16_t* lpos = seq + 2 * kSeqRoom;   // its literals in the input
-  uint16_t* offs = seq + 3 * kSeqRoom;   // its match offset
+// malformed, longer than `cap` or reaches back before its first byte.  mem: kPtrRoom + 2 kPosRoom entries.
+__device__ uint32_t decode_staged(const uint8_t* in, uint32_t n, uint32_t cap, uint16_t* mem, uint8_t* out) {
+  __shared__ uint16_t entry[kSegs], group[kGroups];
+  __shared__ uint32_t warp_sum[kDT / 32 + 1];
+  const uint32_t t = threadIdx.x, lane = lane_id(), warp = t >> 5;
+  uint16_t* const next = mem;              // where a sequence at each position would end
+  uint16_t* const leave = mem + kPtrRoom;  // the index where the chain from each position first leaves its segment
+  uint16_t* const far = leave + kPosRoom;  // ... its warp's segments
+  uint16_t* const ptr = mem;               // over next, later: every output byte's source
+  Seq* const seq = reinterpret_cast<Seq*>(leave);  // over leave, later
   uint32_t lit, lp, ml;
-  // next: where a sequence at each position would end: n the block's end, 0xffff nowhere
-  uint16_t* next = ptr;
-  for (uint32_t q = t; q < n; q += kDT) next[swz(q)] = (uint16_t)parse_seq(in, n, cap, q, &lit, &lp, &ml);
-  entry[t] = 0xffff;
+  for (uint32_t q = t; q - lane < n; q += kDT) {
+    uint32_t x = q < n ? next_seq(in, n, q) : kNoSlot;
+    if (q < n) next[swz(q)] = (uint16_t)x;
+    const uint32_t end = min(n, (q | 31) + 1);
+#pragma unroll
+    for (int r = 0; r < 4; r++) {  // a sequence with a match takes three bytes or more: at most 11 in 32
+      const uint32_t y = __shfl_sync(kFull, x, x & 31);
+      if (x < end) x = y;
+    }
+    if (q < n) leave[swz(q)] = (uint16_t)(x < n ? swz(x) : x == n ? kChainEnd : kChainBad);
+  }
+  if (t < kSegs) entry[t] = 0xffff;
+  if (t < kGroups) group[t] = 0xffff;
   __syncthreads();
-  // leave: where the chain from each position first leaves its thread's 32 positions
-  uint16_t* leave = seq;
-  const uint32_t q0 = 32 * t, q1 = min(n, q0 + 32);
-  for (uint32_t q = q1; q-- > q0;) {  // (not entered when q1 < q0)
-    uint32_t x = next[swz(q)];
-    if (x < q1) x = leave[swz(x)];
-    leave[swz(q)] = (uint16_t)x;
+  constexpr uint32_t kIn = kSegs / kGroups;  // segments of a warp
+  for (uint32_t s = kIn; s-- > 0;) {
+    const uint32_t q = (warp * kIn + s) * 32 + lane;
+    if (q < n) {
+      const uint32_t x = leave[swz(q)];
+      far[swz(q)] = (uint16_t)(x < min((warp + 1) * kIn * 34, kChainEnd) ? far[x] : x);
+    }
+    __syncwarp();
   }
   __syncthreads();
+  // one thread crosses the block group by group, then one a group its segments
   if (t == 0) {
     uint32_t q = 0;
-    do {
-      entry[q >> 5] = (uint16_t)q;
-      q = leave[swz(q)];
-    } while (q < n);
+    for (; q < kChainEnd; q = far[q]) group[q / (kIn * 34)] = (uint16_t)q;
     warp_sum[kDT / 32] = q;
   }
   __syncthreads();
-  if (warp_sum[kDT / 32] != n) return kNoSlot;
+  if (warp_sum[kDT / 32] != kChainEnd) return kNoSlot;
+  if (lane == 0)
+    for (uint32_t q = group[warp]; q < min((warp + 1) * kIn * 34, kChainEnd); q = leave[q]) entry[q / 34] = (uint16_t)q;
+  __syncthreads();
   // the chain's positions in order
   uint32_t nseq, total, mine = 0;
-  for (uint32_t q = entry[t]; q < q1; q = next[swz(q)]) mine++;
+  const uint32_t q1 = min(n, 32 * t + 32);
+  const uint32_t qe = t < kSegs && entry[t] != 0xffff ? entry[t] - 2 * t : 0xffff;
+  for (uint32_t q = qe; q < q1; q = next[swz(q)]) mine++;
   uint32_t k = cta_exscan(mine, warp_sum, &nseq);  // (its barriers: `leave` is read no more)
   if (nseq > kMaxSeq) return kNoSlot;
-  for (uint32_t q = entry[t]; q < q1; q = next[swz(q)]) lpos[k++] = (uint16_t)q;
+  for (uint32_t q = qe; q < q1; q = next[swz(q)]) seq[k++].lpos = (uint16_t)q;
   __syncthreads();
   // sizes, output starts, offsets: a thread takes sequences [k0, k1)
   const uint32_t per = (nseq + kDT - 1) / kDT;
   const uint32_t k0 = min(nseq, t * per), k1 = min(nseq, k0 + per);
   uint32_t sum = 0;
-  for (k = k0; k < k1; k++) {
-    parse_seq(in, n, cap, lpos[k], &lit, &lp, &ml);
-    lpos[k] = (uint16_t)lp;
-    start[k] = (uint16_t)(lit + ml);  // at most 2 * cap
-    mst[k] = (uint16_t)lit;
-    offs[k] = ml ? (uint16_t)((uint32_t)in[lp + lit] | (uint32_t)in[lp + lit + 1] << 8) : (uint16_t)0;
-    sum += lit + ml;
-  }
-  uint32_t o = cta_exscan(sum, warp_sum, &total);
-  if (total > cap) return kNoSlot;
   bool bad = false;
   for (k = k0; k < k1; k++) {
-    const uint32_t len = start[k], l = mst[k];
-    start[k] = (uint16_t)o;
-    mst[k] = (uint16_t)(o + l);
-    if (len > l) bad |= offs[k] == 0 || offs[k] > o + l;
+    if (parse_seq(in, n, cap, seq[k].lpos, &lit, &lp, &ml) == kNoSlot) {
+      bad = true;
+      break;
+    }
+    const uint32_t f = ml ? (uint32_t)in[lp + lit] | (uint32_t)in[lp + lit + 1] << 8 : 0u;
+    seq[k] = Seq{(uint16_t)(lit + ml), (uint16_t)lit, (uint16_t)lp, (uint16_t)f};  // lit + ml: at most 2 * cap
+    sum += lit + ml;
+  }
+  if (__syncthreads_or(bad)) return kNoSlot;
+  uint32_t o = cta_exscan(sum, warp_sum, &total);
+  if (total > cap) return kNoSlot;
+  for (k = k0; k < k1; k++) {
+    const uint32_t len = seq[k].start, l = seq[k].mst, f = seq[k].offs;
+    seq[k].start = (uint16_t)o;
+    seq[k].mst = (uint16_t)(o + l);
+    if (len > l) bad |= f == 0 || f > o + l;
     o += len;
   }
-  if (t == 0) start[nseq] = (uint16_t)total;
+  if (t == 0) seq[nseq].start = (uint16_t)total;
   if (__syncthreads_or(bad)) return kNoSlot;
-  // every output byte's source: a literal (bit 15 and its input position) or an earlier output byte
-  {
-    const uint32_t o0 = 32 * t, o1 = min(total, o0 + 32);
-    if (o0 < o1) {
-      uint32_t lo = 0, hi = nseq;  // start[lo] <= o0 < start[hi]
-      while (hi - lo > 1) {
-        const uint32_t mid = (lo + hi) >> 1;
-        if (start[mid] <= o0) lo = mid;
-        else hi = mid;
-      }
-      uint32_t s0 = start[lo], s1 = start[lo + 1], m0 = mst[lo], l0 = lpos[lo], f0 = offs[lo];
-      for (o = o0; o < o1; o++) {
-        while (o >= s1) {
-          lo++;
-          s0 = s1;
-          s1 = start[lo + 1];
-          m0 = mst[lo];
-          l0 = lpos[lo];
-          f0 = offs[lo];
+  // the sources of the thread's bytes: a literal (bit 15 and its input position) or an earlier output byte
+  const uint32_t o0 = kOut * t;
+  uint32_t v[kOut];
+#pragma unroll
+  for (int u = 0; u < kOut; u++) v[u] = 0x8000u;
+  if (o0 < total) {
+    uint32_t lo = 0, hi = nseq;  // seq[lo].start <= o0 < seq[hi].start
+    while (hi - lo > 1) {
+      const uint32_t mid = (lo + hi) >> 1;
+      if (seq[mid].start <= o0) lo = mid;
+      else hi = mid;
+    }
+    Seq c = seq[lo], after = seq[lo + 1];
+    // byte d of a match repeats byte d mod offset of its source run
+    uint32_t d = o0 > c.mst ? o0 - c.mst : 0;
+    if (d >= c.offs && d) d %= c.offs;
+#pragma unroll
+    for (int u = 0; u < kOut; u++) {
+      o = o0 + u;
+      if (o < total) {
+        if (o >= after.start) {  // (only the last sequence can be empty)
+          c = after;
+          after = seq[++lo + 1];
+          d = 0;
         }
-        uint32_t v;
-        if (o < m0) {
-          v = 0x8000u | (l0 + o - s0);
+        if (o < c.mst) {
+          v[u] = 0x8000u | (c.lpos + o - c.start);
         } else {
-          // byte d of a match repeats byte d mod offset of its source run
-          uint32_t d = o - m0;
-          if (d >= f0) d %= f0;
-          v = m0 - f0 + d;
+          v[u] = c.mst - c.offs + d;
+          if (++d == c.offs) d = 0;
         }
-        ptr[swz(o)] = (uint16_t)v;
       }
     }
   }
+  uint32_t* const own = reinterpret_cast<uint32_t*>(ptr + swz_out(o0));
+#pragma unroll
+  for (int u = 0; u < kOut; u += 2) own[u / 2] = v[u] | v[u + 1] << 16;
   __syncthreads();
   // every source followed to its literal (a pointer read while its owner moves it on is an
-  // earlier one of the same chain: still right); thread t keeps bytes t + 256 j, bit j not there yet
-  uint32_t todo = 0;
-  for (uint32_t j = 0; j < (total + kDT - 1 - t) / kDT; j++) todo |= 1u << j;
-  for (;;) {
-    for (uint32_t m = todo; m; m &= m - 1) {
-      const uint32_t j = __ffs(m) - 1, q = j * kDT + t;
-      uint32_t v = ptr[swz(q)];
-      if (!(v & 0x8000u)) {
-        v = ptr[swz(v)];
-        ptr[swz(q)] = (uint16_t)v;
-      }
-      if (v & 0x8000u) todo &= ~(1u << j);
+  // earlier one of the same chain: still right)
+  for (bool open = true;;) {
+    if (open) {
+      open = false;
+#pragma unroll
+      for (int u = 0; u < kOut; u++)
+        if (!(v[u] & 0x8000u)) {
+          v[u] = ptr[swz_out(v[u])];
+          open |= !(v[u] & 0x8000u);
+        }
+#pragma unroll
+      for (int u = 0; u < kOut; u += 2) own[u / 2] = v[u] | v[u + 1] << 16;
     }
-    if (!__syncthreads_or(todo)) break;
+    if (!__syncthreads_or(open)) break;
   }
-  for (uint32_t w = t; w < (total + 3) >> 2; w += kDT) {
-    // (bytes past the end come from whatever the array holds there, an index inside the stage)
-    const uint32_t i = swz(4 * w);
-    const uint32_t a = *reinterpret_cast<const uint32_t*>(ptr + i), b = *reinterpret_cast<const uint32_t*>(ptr + i + 2);
-    const uint32_t x = in[a & 0x1fff] | (uint32_t)in[(a >> 16) & 0x1fff] << 8 | (uint32_t)in[b & 0x1fff] << 16 |
-                       (uint32_t)in[(b >> 16) & 0x1fff] << 24;
-    reinterpret_cast<uint32_t*>(out)[w] = x;
+  if (o0 < total) {
+    uint32_t x[4];
+#pragma unroll
+    for (int u = 0; u < 4; u++)
+      x[u] = in[v[4 * u] & 0x1fff] | (uint32_t)in[v[4 * u + 1] & 0x1fff] << 8 | (uint32_t)in[v[4 * u + 2] & 0x1fff] << 16 |
+             (uint32_t)in[v[4 * u + 3] & 0x1fff] << 24;
+    reinterpret_cast<uint4*>(out)[t] = make_uint4(x[0], x[1], x[2], x[3]);
   }
   return total;
 }
 
-// One CTA per (frame, block ordinal): block `i` of frame `fi` into slot frames[fi].slot0 + i.
-__global__ void __launch_bounds__(kDT, 5) k_lz4_blocks(const Lz4Frame* __restrict__ frames, const uint32_t* __restrict__ frame_of,
-                                                       Lz4Slot* __restrict__ slots, uint8_t* __restrict__ slot_mem) {
+// One CTA per block.
+__global__ void __launch_bounds__(kDT, 2) k_lz4_blocks(const Lz4Frame* __restrict__ frames, Lz4Slot* __restrict__ slots,
+                                                       uint8_t* __restrict__ slot_mem, bool early) {
   extern __shared__ __align__(16) uint8_t dsm[];
-  __shared__ uint16_t entry[kDT];
-  __shared__ uint32_t warp_sum[kDT / 32 + 1];
-  const uint32_t g = blockIdx.x;
-  const Lz4Frame fr = frames[frame_of[g]];
-  const uint32_t i = g - fr.slot0;
-  const uint8_t* s = fr.src;
-  const uint64_t n = fr.src_len;
-  Lz4Slot sl{0, 0, kNoSlot, 0};  // a bad frame, or a block that cannot be decoded on its own
-  uint64_t pos = 0;
-  bool block_sum = false, content_sum = false;
-  bool ok = n < (1ull << 31) && frame_header(s, n, &pos, &block_sum, &content_sum);
-  uint32_t sz = 0;
-  bool stored = false;
-  for (uint32_t b = 0; ok; b++) {  // (every thread walks the headers: uniform loads)
-    if (n - pos < 4) {
-      ok = false;
-      break;
-    }
-    const uint32_t bs = le32(s + pos);
-    pos += 4;
-    if (bs == 0) {  // end mark: fewer than i + 1 blocks
-      sl.size = 0;
-      sl.state = 1;
-      ok = false;
-      break;
-    }
-    sz = bs & 0x7FFFFFFFu;
-    stored = bs & 0x80000000u;
-    if (sz > n - pos || (block_sum && n - pos - sz < 4)) {
-      ok = false;
-      break;
-    }
-    if (b == i) break;
-    pos += sz + (block_sum ? 4 : 0);
-  }
-  if (ok && i + 1 == fr.n_slots) {  // the last slot: the end mark must follow
-    const uint64_t after = pos + sz + (block_sum ? 4 : 0);
-    if (n - after < 4 || le32(s + after) != 0) ok = false;
-  }
-  if (ok) {
-    sl.pos = (uint32_t)pos;
-    if (stored) {
-      sl.size = sz;
-      sl.state = 2;
-    } else if (sz > 0 && sz <= kLz4MaxBlock) {
-      // the aligned 16-byte words that hold the block (they stay inside the stream's allocation)
-      const uint8_t* src = s + pos;
-      const uint32_t phase = (uint32_t)(reinterpret_cast<uintptr_t>(src) & 15);
-      const uint4* a = reinterpret_cast<const uint4*>(src - phase);
-      const uint32_t nw = (phase + sz + 15) >> 4;
-      for (uint32_t q = threadIdx.x; q < nw; q += kDT) reinterpret_cast<uint4*>(dsm)[q] = __ldg(a + q);
-      __syncthreads();
-      const uint32_t slot = lz4_slot_bytes(fr.dst_len);
-      uint16_t* ptr = reinterpret_cast<uint16_t*>(dsm + kInStage);
-      sl.size = decode_staged(dsm + phase, sz, slot, ptr, ptr + kPtrRoom, entry, warp_sum,
-                              slot_mem + fr.mem0 + (size_t)i * slot);
-      if (sl.size != kNoSlot) sl.state = 3;
-    }
-  }
-  if (threadIdx.x == 0) slots[g] = sl;
+  if (early) cudaTriggerProgrammaticLaunchCompletion();
+  const Lz4Slot sl = slots[blockIdx.x];
+  if (sl.state != 3) return;
+  const Lz4Frame fr = frames[sl.frame];
+  // the aligned 16-byte words that hold the block (they stay inside the stream's allocation)
+  const uint8_t* src = fr.src + sl.pos;
+  const uint32_t phase = (uint32_t)(reinterpret_cast<uintptr_t>(src) & 15);
+  const uint4* a = reinterpret_cast<const uint4*>(src - phase);
+  const uint32_t nw = (phase + sl.size + 15) >> 4;
+  for (uint32_t q = threadIdx.x; q < nw; q += kDT) reinterpret_cast<uint4*>(dsm)[q] = __ldg(a + q);
+  __syncthreads();
+  const uint32_t slot = lz4_slot_bytes(fr.dst_len);
+  const uint32_t size = decode_staged(dsm + phase, sl.size, slot, reinterpret_cast<uint16_t*>(dsm + kInStage),
+                                      slot_mem + fr.mem0 + (size_t)(blockIdx.x - fr.slot0) * slot);
+  if (threadIdx.x == 0) slots[blockIdx.x].size = size;
 }
 
 // The whole frame by one warp, its blocks in order (matches may reach back into earlier ones).
@@ -651,14 +672,13 @@ __device__ bool decode_frame(const Lz4Frame& fr) {
   return ok && o == fr.dst_len;
 }
 
-__global__ void __launch_bounds__(kWarps * 32) k_lz4_place(const Lz4Frame* __restrict__ frames,
-                                                           const uint32_t* __restrict__ frame_of, uint32_t n_slots,
-                                                           const Lz4Slot* __restrict__ slots,
+__global__ void __launch_bounds__(kWarps * 32) k_lz4_place(const Lz4Frame* __restrict__ frames, const Lz4Slot* __restrict__ slots,
                                                            const uint8_t* __restrict__ slot_mem, int32_t* err) {
-  const uint32_t g = blockIdx.x * kWarps + (threadIdx.x >> 5);
-  if (g >= n_slots) return;
-  const uint32_t lane = lane_id();
-  const Lz4Frame fr = frames[frame_of[g]];
+  cudaTriggerProgrammaticLaunchCompletion();
+  cudaGridDependencySynchronize();
+  const uint32_t g = blockIdx.x, lane = lane_id();
+  const Lz4Slot sl = slots[g];
+  const Lz4Frame fr = frames[sl.frame];
   const uint32_t i = g - fr.slot0;
   // the frame's blocks: any that could not be decoded on its own, their sizes before this one
   uint64_t before = 0, total = 0;
@@ -678,14 +698,13 @@ __global__ void __launch_bounds__(kWarps * 32) k_lz4_place(const Lz4Frame* __res
   bad = bad || total != fr.dst_len;
   // a frame with a content checksum is checked for it by decode_frame
   if (bad || (fr.src_len > 4 && (fr.src[4] & 0x04))) {
-    if (i != 0) return;
+    if (i != 0 || threadIdx.x >= 32) return;
     const bool ok = decode_frame(fr);
     if (!ok && lane == 0) atomicOr(err, 1);
     return;
   }
-  const Lz4Slot sl = slots[g];
-  if (sl.state == 2) copy_bytes<32>(fr.dst + before, fr.src + sl.pos, sl.size, lane);
-  else if (sl.state == 3) copy_bytes<32>(fr.dst + before, slot_mem + fr.mem0 + (size_t)i * lz4_slot_bytes(fr.dst_len), sl.size, lane);
+  const uint8_t* from = sl.state == 2 ? fr.src + sl.pos : slot_mem + fr.mem0 + (size_t)i * lz4_slot_bytes(fr.dst_len);
+  copy_bytes<kWarps * 32>(fr.dst + before, from, sl.size, threadIdx.x);
 }
 
 int sm_count() {
@@ -717,14 +736,96 @@ cudaError_t launch_lz4_compress(const Lz4Chunk* chunks, uint32_t n_chunks, uint3
   return cudaGetLastError();
 }
 
-cudaError_t launch_lz4_decode(const Lz4Frame* frames, const uint32_t* frame_of, uint32_t n_slots, Lz4Slot* slots,
-                              uint8_t* slot_mem, int32_t* err, cudaStream_t st) {
+// The headers are a chain through the frame, 14 for a wide batch's worded column.  Followed by every
+// block's CTA they took it a fifth of its time (5 of 27 thousand cycles, 14 at the end of such a frame), and
+// its slots had to be guessed; the host follows them while the device reads the stream, all frames a step
+// at a time, the next headers on their way.
+void lz4_index(const uint8_t* const* src, Lz4Frame* frames, uint32_t n, std::vector<Lz4Slot>* slots, size_t* mem) {
+  struct Walk {
+    uint64_t pos = 0;
+    size_t first = 0;  // its slots in `found`
+    uint32_t room = 0, count = 0;
+    bool block_sum = false, bad = false;
+  };
+  std::vector<Walk> w(n);
+  std::vector<uint32_t> active(n);
+  size_t room = 0;
+  for (uint32_t k = 0; k < n; k++) {
+    __builtin_prefetch(src[k]);
+    active[k] = k;
+    w[k].first = room;
+    w[k].room = (uint32_t)std::min<uint64_t>(lz4_frame_slots(frames[k].dst_len), frames[k].src_len / 4 + 1);
+    room += w[k].room;
+  }
+  std::vector<Lz4Slot> found(room);
+  for (bool first = true; !active.empty(); first = false) {
+    size_t left = 0;
+    for (const uint32_t k : active) {
+      Walk& x = w[k];
+      const uint8_t* s = src[k];
+      const uint64_t len = frames[k].src_len;
+      if (first) {
+        bool content_sum;
+        x.bad = len >= (1ull << 31) || !frame_header(s, len, &x.pos, &x.block_sum, &content_sum);
+      }
+      if (x.bad || len - x.pos < 4) {
+        x.bad = true;
+        continue;
+      }
+      const uint32_t bs = le32(s + x.pos), sz = bs & 0x7FFFFFFFu;
+      x.pos += 4;
+      if (bs == 0) continue;  // end mark
+      const bool stored = bs & 0x80000000u;
+      if (x.count == x.room || sz > len - x.pos || (x.block_sum && len - x.pos - sz < 4) || (!stored && sz > kLz4MaxBlock)) {
+        x.bad = true;
+        continue;
+      }
+      found[x.first + x.count++] = Lz4Slot{(uint32_t)x.pos, k, sz, stored ? 2u : 3u};
+      x.pos += sz + (x.block_sum ? 4 : 0);
+      __builtin_prefetch(s + x.pos);
+      active[left++] = k;
+    }
+    active.resize(left);
+  }
+  slots->clear();
+  slots->reserve(room + n);
+  *mem = 0;
+  for (uint32_t k = 0; k < n; k++) {
+    frames[k].slot0 = (uint32_t)slots->size();
+    frames[k].mem0 = *mem;
+    if (w[k].bad) slots->push_back(Lz4Slot{0, k, kNoSlot, 0});
+    else if (w[k].count == 0) slots->push_back(Lz4Slot{0, k, 0, 1});
+    else slots->insert(slots->end(), found.begin() + (ptrdiff_t)w[k].first, found.begin() + (ptrdiff_t)(w[k].first + w[k].count));
+    frames[k].n_slots = (uint32_t)slots->size() - frames[k].slot0;
+    *mem += (size_t)frames[k].n_slots * lz4_slot_bytes(frames[k].dst_len);
+  }
+}
+
+cudaError_t launch_lz4_decode(const Lz4Frame* frames, Lz4Slot* slots, uint32_t n_slots, uint8_t* slot_mem, int32_t* err,
+                              cudaStream_t st) {
   if (n_slots == 0) return cudaSuccess;
-  k_lz4_blocks<<<n_slots, kDT, kDecodeSmem, st>>>(frames, frame_of, slots, slot_mem);
-  const cudaError_t e = cudaGetLastError();
+  static bool attr = false;
+  if (!attr) {
+    const cudaError_t e = cudaFuncSetAttribute(k_lz4_blocks, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDecodeSmem);
+    if (e != cudaSuccess) return e;
+    attr = true;
+  }
+  // the second comes up while the first runs, unless there are more blocks than can run at once: it would
+  // hold what they wait for
+  const bool early = n_slots <= 2u * (uint32_t)sm_count();
+  k_lz4_blocks<<<n_slots, kDT, kDecodeSmem, st>>>(frames, slots, slot_mem, early);
+  cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
-  k_lz4_place<<<(n_slots + kWarps - 1) / kWarps, kWarps * 32, 0, st>>>(frames, frame_of, n_slots, slots, slot_mem, err);
-  return cudaGetLastError();
+  cudaLaunchAttribute at;
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = n_slots;
+  cfg.blockDim = kWarps * 32;
+  cfg.stream = st;
+  cfg.attrs = &at;
+  cfg.numAttrs = early ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, k_lz4_place, frames, (const Lz4Slot*)slots, (const uint8_t*)slot_mem, err);
 }
 
 }  // namespace gz

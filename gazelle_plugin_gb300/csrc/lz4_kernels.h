@@ -3,6 +3,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <vector>
+
 namespace gz {
 
 constexpr uint32_t kLz4MaxBlock = 8192;  // bytes of input per block (at most the frame's 64 KiB block size)
@@ -27,18 +29,19 @@ struct Lz4Frame {  // one frame to decode: src_len bytes into exactly dst_len by
   uint8_t* dst;
   uint64_t dst_len;
   uint32_t slot0;    // its first block slot
-  uint32_t n_slots;  // its slots (lz4_frame_slots)
+  uint32_t n_slots;  // its slots: one a block, at least one
   uint64_t mem0;     // where the slots' memory starts (lz4_slot_bytes each)
 };
 
 struct Lz4Slot {  // one block of a frame
   uint32_t pos;    // its payload inside the frame
-  uint32_t pad;
-  uint32_t size;   // decoded bytes, or 0xffffffff: not decodable on its own
-  uint32_t state;  // 0: see size, 1: no such block, 2: stored, 3: decoded into its slot
+  uint32_t frame;
+  uint32_t size;   // bytes of the payload, once decoded those it gives; kLz4NoSlot: not decodable on its own
+  uint32_t state;  // 0: see size, 1: a frame without blocks, 2: stored, 3: compressed
 };
+constexpr uint32_t kLz4NoSlot = 0xffffffffu;
 
-// Block slots for a frame of dst_len bytes: blocks of kLz4MaxBlock bytes, and three shorter ones
+// Most block slots of a frame of dst_len bytes: blocks of kLz4MaxBlock bytes, and three shorter ones
 // inside it (an offsets buffer starts with its own first offset, a batch may continue from an
 // earlier device pass); a frame with more blocks is decoded by one warp.
 inline uint32_t lz4_frame_slots(uint64_t dst_len) {
@@ -64,11 +67,15 @@ inline uint32_t lz4_slot_bytes(uint64_t dst_len) {
   return dst_len < kLz4MaxBlock ? ((uint32_t)dst_len + 15u) & ~15u : kLz4MaxBlock;
 }
 
-// Decodes every frame; *err gets bit 0 for a malformed frame or a size that differs.  frame_of[g]:
-// the frame of slot g (n_slots of them, every frame's in a row); `slots` and `slot_mem`
-// are scratch.  The sources' allocations start and end on 16-byte
+// Host: the blocks of n frames from their headers, every frame's slots in a row (slot0, n_slots and mem0
+// of each frame are set; *mem gets the bytes of all slots).  src[k]: frame k's bytes in host memory.  A frame that is
+// malformed or has more blocks than slots gets one slot that cannot be decoded on its own.
+void lz4_index(const uint8_t* const* src, Lz4Frame* frames, uint32_t n, std::vector<Lz4Slot>* slots, size_t* mem);
+
+// Decodes every frame; *err gets bit 0 for a malformed frame or a size that differs.  `slots` (n_slots of
+// them, lz4_index's) are written, `slot_mem` is scratch.  The sources' allocations start and end on 16-byte
 // boundaries.
-cudaError_t launch_lz4_decode(const Lz4Frame* frames, const uint32_t* frame_of, uint32_t n_slots, Lz4Slot* slots,
-                              uint8_t* slot_mem, int32_t* err, cudaStream_t st);
+cudaError_t launch_lz4_decode(const Lz4Frame* frames, Lz4Slot* slots, uint32_t n_slots, uint8_t* slot_mem, int32_t* err,
+                              cudaStream_t st);
 
 }  // namespace gz

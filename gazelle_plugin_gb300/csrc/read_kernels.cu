@@ -12,6 +12,8 @@
 #include "copy.cuh"
 #include "read_kernels.h"
 
+#include <algorithm>
+
 namespace gz {
 
 namespace {
@@ -71,6 +73,7 @@ __global__ void __launch_bounds__(kThreads) k_read(const ReadJobs jobs) {
 }
 
 __global__ void __launch_bounds__(kThreads) k_read_words(const int32_t* const* __restrict__ src, int32_t* out, size_t n) {
+  cudaGridDependencySynchronize();
   for (size_t i = (size_t)blockIdx.x * kThreads + threadIdx.x; i < n; i += (size_t)gridDim.x * kThreads) out[i] = *src[i];
 }
 
@@ -87,22 +90,19 @@ unsigned grid_for(uint32_t n_jobs) {
 
 }  // namespace
 
-cudaError_t gather_words(const int32_t* const* src, int32_t* out, size_t n, cudaStream_t st) {
+cudaError_t launch_read_words(const int32_t* const* src, int32_t* out, size_t n, cudaStream_t st) {
   if (n == 0) return cudaSuccess;
-  uint8_t* d = nullptr;
-  const size_t pb = (n * sizeof(void*) + 255) / 256 * 256;
-  cudaError_t e = cudaMallocAsync(reinterpret_cast<void**>(&d), pb + n * sizeof(int32_t), st);
-  if (e != cudaSuccess) return e;
-  e = cudaMemcpyAsync(d, src, n * sizeof(void*), cudaMemcpyHostToDevice, st);
-  if (e == cudaSuccess) {
-    const size_t blocks = (n + kThreads - 1) / kThreads;
-    k_read_words<<<blocks < 1024 ? (unsigned)blocks : 1024u, kThreads, 0, st>>>(
-        reinterpret_cast<const int32_t* const*>(d), reinterpret_cast<int32_t*>(d + pb), n);
-    e = cudaGetLastError();
-  }
-  if (e == cudaSuccess) e = cudaMemcpyAsync(out, d + pb, n * sizeof(int32_t), cudaMemcpyDeviceToHost, st);
-  cudaFreeAsync(d, st);
-  return e;
+  const size_t blocks = (n + kThreads - 1) / kThreads;
+  cudaLaunchAttribute at;  // it comes up while the kernel before it runs
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = (unsigned)std::min<size_t>(blocks, 1024);
+  cfg.blockDim = kThreads;
+  cfg.stream = st;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, k_read_words, src, out, n);
 }
 
 cudaError_t launch_read_jobs(const ReadJobs& jobs, cudaStream_t st) {

@@ -27,9 +27,8 @@ struct BitJob {  // bits [src_bit, src_bit + nbits) of src (all ones when src is
   uint64_t nbits;
 };
 
-// out[i] = *src[i] for n device addresses (host arrays; waits for nothing but the copies it
-// enqueues: the caller synchronises `st` before reading out).
-cudaError_t gather_words(const int32_t* const* src, int32_t* out, size_t n, cudaStream_t st);
+// out[i] = *src[i] for n device addresses; src is in device memory, out wherever the device can write.
+cudaError_t launch_read_words(const int32_t* const* src, int32_t* out, size_t n, cudaStream_t st);
 
 struct ReadJobs {  // the job lists, in device memory
   const ByteJob* bytes;

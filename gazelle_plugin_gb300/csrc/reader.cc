@@ -353,48 +353,44 @@ Status PartitionReader::AddStream(const uint8_t* data, int64_t len) {
   arenas_.push_back(nullptr);
   if (!frames.empty() && d != nullptr) {  // (batches without rows leave no image)
     // compressed buffers: every LZ4 frame decoded by the device into the stream's arena; the
-    // jobs, the frame of every block slot, the error word and the slots lie in front of it
+    // jobs, the blocks, the addresses of the words the host wants back, the error word (the first
+    // of these) and the words themselves lie in front of it, what goes up in one copy
     std::vector<Lz4Frame> jobs;
-    std::vector<uint32_t> frame_of;
-    size_t slot_bytes = 0;
+    std::vector<const uint8_t*> bytes;
     for (const FrameRef& f : frames) {
-      const uint32_t ns = lz4_frame_slots((uint64_t)f.dst_len);
-      jobs.push_back(Lz4Frame{nullptr, (uint64_t)f.src_len, nullptr, (uint64_t)f.dst_len, (uint32_t)frame_of.size(), ns,
-                              slot_bytes});
-      slot_bytes += (size_t)ns * lz4_slot_bytes((uint64_t)f.dst_len);
-      frame_of.resize(frame_of.size() + ns, (uint32_t)jobs.size() - 1);
+      jobs.push_back(Lz4Frame{nullptr, (uint64_t)f.src_len, nullptr, (uint64_t)f.dst_len, 0, 0, 0});
+      bytes.push_back(data + f.src);
     }
-    const size_t jb = AlignUp(sizeof(Lz4Frame) * jobs.size(), 256), fb = AlignUp(4 * frame_of.size(), 256),
-                 sb = AlignUp(sizeof(Lz4Slot) * frame_of.size(), 256);
-    const size_t head = jb + fb + 256 + sb;
+    std::vector<Lz4Slot> slots;
+    size_t slot_bytes = 0;
+    lz4_index(bytes.data(), jobs.data(), (uint32_t)jobs.size(), &slots, &slot_bytes);
+    size_t max_words = 1;
+    for (const Batch& b : bs)
+      for (const ColRef& c : b.cols) max_words += 4 * std::max<size_t>(1, c.nodes.size());
+    const size_t jb = AlignUp(sizeof(Lz4Frame) * jobs.size(), 256), sb = AlignUp(sizeof(Lz4Slot) * slots.size(), 256),
+                 wb = AlignUp(sizeof(void*) * max_words, 256);
+    const size_t head = jb + sb + wb + 256 + AlignUp(4 * max_words, 256);
     st = Cuda(cudaMallocAsync(reinterpret_cast<void**>(&arena), head + AlignUp((size_t)arena_bytes, 256), stream_),
               "cudaMallocAsync(decode)");
-    if (!st.ok()) return st;
     uint8_t* slot_mem = nullptr;
-    st = Cuda(cudaMallocAsync(reinterpret_cast<void**>(&slot_mem), std::max<size_t>(slot_bytes, 256), stream_),
-              "cudaMallocAsync(decode)");
-    if (!st.ok()) return st;
+    if (st.ok()) {
+      arena_mem_.push_back(arena);
+      st = Cuda(cudaMallocAsync(reinterpret_cast<void**>(&slot_mem), std::max<size_t>(slot_bytes, 256), stream_),
+                "cudaMallocAsync(decode)");
+    }
+    if (!st.ok()) {
+      cudaStreamSynchronize(stream_);  // the caller's bytes are being read
+      return st;
+    }
     arenas_.back() = arena + head;
     for (size_t i = 0; i < jobs.size(); i++) {
       jobs[i].src = d + frames[i].src;
       jobs[i].dst = arenas_.back() + frames[i].dst;
     }
-    std::vector<uint8_t> up(jb + fb + 4, 0);  // with the error word, zero
-    memcpy(up.data(), jobs.data(), sizeof(Lz4Frame) * jobs.size());
-    memcpy(up.data() + jb, frame_of.data(), 4 * frame_of.size());
-    int32_t* d_err = reinterpret_cast<int32_t*>(arena + jb + fb);
-    int32_t err = 0;
-    st = Cuda(cudaMemcpyAsync(arena, up.data(), up.size(), cudaMemcpyHostToDevice, stream_), "H2D");
-    if (st.ok())
-      st = Cuda(launch_lz4_decode(reinterpret_cast<const Lz4Frame*>(arena), reinterpret_cast<const uint32_t*>(arena + jb),
-                                  (uint32_t)frame_of.size(), reinterpret_cast<Lz4Slot*>(arena + jb + fb + 256), slot_mem,
-                                  d_err, stream_),
-                "k_lz4_blocks");
-    cudaFreeAsync(slot_mem, stream_);
-    if (st.ok()) st = Cuda(cudaMemcpyAsync(&err, d_err, 4, cudaMemcpyDeviceToHost, stream_), "D2H");
+    int32_t* d_err = reinterpret_cast<int32_t*>(arena + jb + sb + wb);
     // the decoded offsets bound each batch's characters (and a nested node's child entries): for
     // each, the 4-byte words of its first and last offset (low word, then high word of a 64-bit one)
-    std::vector<const int32_t*> where;
+    std::vector<const int32_t*> where{d_err};
     std::vector<std::pair<size_t, size_t>> which;  // (batch, field)
     std::vector<std::pair<NodeRef*, int>> nested;  // a nested node and its offset width
     auto queue_ends = [&](const int32_t* o, int64_t n, int ow) {
@@ -422,11 +418,29 @@ Status PartitionReader::AddStream(const uint8_t* data, int64_t len) {
           queue_ends(reinterpret_cast<const int32_t*>(arenas_.back() + nr.offsets.offset), nr.length, ow);
           nested.push_back({&nr, ow});
         }
-    std::vector<int32_t> ends(where.size());
-    if (st.ok() && !where.empty()) st = Cuda(gather_words(where.data(), ends.data(), where.size(), stream_), "offsets");
-    if (st.ok()) st = Cuda(cudaStreamSynchronize(stream_), "k_lz4_place");
+    std::vector<uint8_t> up(jb + sb + wb + 4, 0);  // with the error word, zero
+    memcpy(up.data(), jobs.data(), sizeof(Lz4Frame) * jobs.size());
+    memcpy(up.data() + jb, slots.data(), sizeof(Lz4Slot) * slots.size());
+    memcpy(up.data() + jb + sb, where.data(), sizeof(void*) * where.size());
+    st = Cuda(cudaMemcpyAsync(arena, up.data(), up.size(), cudaMemcpyHostToDevice, stream_), "H2D");
+    if (st.ok())
+      st = Cuda(launch_lz4_decode(reinterpret_cast<const Lz4Frame*>(arena), reinterpret_cast<Lz4Slot*>(arena + jb),
+                                  (uint32_t)slots.size(), slot_mem, d_err, stream_),
+                "k_lz4_blocks");
+    // written to host memory as they are read where the device can do that: a copy behind the kernel
+    // is staged and waited for on its own (34 us from the decoded bytes to the caller with it, 16 without)
+    std::vector<int32_t> words(where.size());
+    int32_t* const out = direct_ ? words.data() : d_err + 64;
+    if (st.ok())
+      st = Cuda(launch_read_words(reinterpret_cast<const int32_t* const*>(arena + jb + sb), out, where.size(), stream_), "offsets");
+    if (st.ok() && !direct_)
+      st = Cuda(cudaMemcpyAsync(words.data(), out, 4 * words.size(), cudaMemcpyDeviceToHost, stream_), "D2H");
+    const Status read = Cuda(cudaStreamSynchronize(stream_), "k_lz4_place");
+    cudaFreeAsync(slot_mem, stream_);
+    if (st.ok()) st = read;
     if (!st.ok()) return st;
-    if (err) return Status::Error(GZ_INVALID, "a compressed buffer is not a valid LZ4 frame of its stated length");
+    if (words[0]) return Status::Error(GZ_INVALID, "a compressed buffer is not a valid LZ4 frame of its stated length");
+    const int32_t* const ends = words.data() + 1;
     size_t e = 0;
     auto word = [&](int ow) -> int64_t {
       const int64_t v = ow == 8 ? (int64_t)((uint64_t)(uint32_t)ends[e] | (uint64_t)(uint32_t)ends[e + 1] << 32)
@@ -447,7 +461,6 @@ Status PartitionReader::AddStream(const uint8_t* data, int64_t len) {
       x.first->o0 = word(x.second);
       x.first->o1 = word(x.second);
     }
-    arena_mem_.push_back(arena);
   } else {
     st = Cuda(cudaStreamSynchronize(stream_), "H2D stream");
     if (!st.ok()) return st;

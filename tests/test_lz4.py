@@ -295,3 +295,33 @@ def test_gpu_decoder_malformed_frames(how):
     with pytest.raises(S.SplitterError) as e:
         _read_values_frame(frame, n)
     assert e.value.status == S.GZ_INVALID
+
+
+DENSE_SHAPES = {
+    # blocks, their size, FLG byte, and what their sequences look like
+    "as many sequences as fit": (3, 8192, 0x60, [0], [4], range(1, 9)),
+    "three-byte tokens, far sources": (2, 8192, 0x60, [0, 1], [4], range(1, 8190)),
+    "one run": (2, 8192, 0x60, [1], [8180], [1]),
+    "hardly a match": (2, 8192, 0x60, [3900], [80], [9]),
+    "block checksums": (3, 4096, 0x70, range(0, 6), range(4, 12), range(1, 4000)),
+    "content checksum": (3, 4096, 0x64, range(0, 6), range(4, 12), range(1, 4000)),
+    "more blocks than run at once": (500, 8192, 0x60, range(0, 40), range(4, 30), range(1, 8000)),
+}
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("shape", list(DENSE_SHAPES))
+def test_gpu_decoder_blocks_at_their_limits(shape):
+    """The most sequences a block can hold, one sequence over all segments, long chains of matches, frames
+    with checksums, and more blocks than the device runs at once."""
+    count, size, flg, lits, mls, offs = DENSE_SHAPES[shape]
+    rng = np.random.default_rng(1)
+    some = [_lz4_block(rng, size, list(lits), list(mls), list(offs)) for _ in range(min(count, 5))]
+    desc = bytes([flg, 0x40])
+    frame, want = b"\x04\x22\x4d\x18" + desc + bytes([(O.xxh32(desc) >> 8) & 255]), b""
+    for i in range(count):
+        b, d = some[i % len(some)]
+        frame += len(b).to_bytes(4, "little") + b + (b"sums" if flg & 0x10 else b"")
+        want += d
+    frame += bytes(4) + (b"sum." if flg & 0x04 else b"")
+    assert _read_values_frame(frame, len(want)) == want
