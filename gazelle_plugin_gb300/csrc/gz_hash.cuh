@@ -64,12 +64,11 @@ __device__ __forceinline__ uint32_t fastmod_u32(uint32_t a, uint32_t d, unsigned
   const unsigned long long low = M * (unsigned long long)a;
   return (uint32_t)__umul64hi(low, (unsigned long long)d);
 }
-// Spark pmod(h, P).
+// Spark pmod(h, P): h - P floor(h / P), and floor(h / P) of a negative h is ~floor(~h / P).
 __device__ __forceinline__ uint32_t pmod_div(int32_t h, const PmodDiv& d) {
-  if (d.P == 1) return 0;
-  const uint32_t a = h < 0 ? 0u - (uint32_t)h : (uint32_t)h;
-  const uint32_t r = a - (__umulhi(a, d.m) >> d.shift) * d.P;
-  return h < 0 && r != 0 ? d.P - r : r;
+  const uint32_t sign = (uint32_t)(h >> 31);
+  const uint32_t q = (__umulhi((uint32_t)h ^ sign, d.m) >> d.shift) ^ sign;
+  return d.P == 1 ? 0u : (uint32_t)h - q * d.P;
 }
 
 __device__ __forceinline__ bool get_bit(const uint8_t* bits, uint32_t i) {

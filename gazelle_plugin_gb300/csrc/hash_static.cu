@@ -26,6 +26,7 @@ using namespace hash;
 constexpr uint32_t kTile = 1024;             // rows behind each row of counters in the limit on a call
 constexpr uint32_t kGroup = 4;               // consecutive rows of a thread
 constexpr uint32_t kSmemHistMaxP = 57344;    // a block's histogram stays in shared memory (224 KB)
+constexpr int kAny = -1, kMixed = -2;         // see k_hash_count_static
 constexpr uint32_t kWideHistP = 2048;        // larger histograms: blocks of 1024 threads share one
 
 // Row counts of each block, [block][partition], of the most recent call on this device.  Every call
@@ -141,57 +142,104 @@ __device__ __forceinline__ void hash_key(int kind, const Group& g, int32_t* h) {
 }
 
 // Every block takes a contiguous range of rows: partition id of every row, and the block's row count
-// per partition into row blockIdx.x of `count_rows`.  Bound by the hash's integer instructions and
-// their latency.  A thread takes four consecutive rows, loaded 16 bytes at a time one key ahead of
+// per partition into row blockIdx.x of `count_rows`.  Bound by the hash's integer instructions.  A
+// thread takes four consecutive rows, loaded 16 bytes at a time one key ahead of
 // the hashing, and a block keeps one histogram for all its rows, so only a row of counters per
 // resident block is left to be added up.  16M rows of two nullable int64 keys and 200 partitions (290
 // MB): 156 us with scalar loads and a row of counters per 1024 rows, 84 us with wide loads and few
-// counters (59% of the issue slots, 55% of the 64-bit multiply pipe), 71 us with the next key's loads
-// ahead and the 32-bit pmod (4.1 TB/s).
-template <int kThreads, int kMinBlocks>
+// counters (59% of the issue slots, 55% of the 64-bit multiply pipe), 70 us with the next key's loads
+// ahead and the 32-bit pmod (117 instructions a row, 75% of the issue slots), 55 us (5.2 TB/s) with counters known to be in shared
+// memory (a pointer to either memory costs an address test and a branch per row), the last, partial
+// groups apart and the alignment and the kind of the keys settled by the host; one int32 key: 47 and 32 us.
+// (A ring of four keys' values on their way into shared memory by cp.async: 46 us for one int32 key
+// against 47, 90 for the two int64 against 70: not the loads but the instructions bound it.)
+// kSmem: the counters are in shared memory.  kKind: all keys are of that kind, their values on the
+// boundaries of a group's wide loads and the ids on 8-byte ones; kMixed: any kinds, so aligned; kAny.
+template <int kThreads, int kMinBlocks, bool kSmem, int kKind>
 __global__ void __launch_bounds__(kThreads, kMinBlocks)
-k_hash_count_static(const KeySet keys, uint32_t nrows, uint32_t rows_per_block, PmodDiv pmod, int hist_in_smem,
+k_hash_count_static(const KeySet keys, uint32_t nrows, uint32_t rows_per_block, PmodDiv pmod,
                     uint16_t* __restrict__ pids, uint32_t* __restrict__ count_rows) {
   extern __shared__ uint32_t smem[];
   cudaTriggerProgrammaticLaunchCompletion();  // k_sum_tile_counts may come up, and wait
   cudaGridDependencySynchronize();            // (this kernel came up early as well)
   const uint32_t P = pmod.P;
-  uint32_t* row = count_rows + (size_t)blockIdx.x * P;
-  uint32_t* H = hist_in_smem ? smem : row;
+  uint32_t* const row = count_rows + (size_t)blockIdx.x * P;
+  uint32_t* const H = kSmem ? smem : row;
   const uint32_t lo = blockIdx.x * rows_per_block;  // a multiple of 4
   const uint32_t hi = min(nrows, lo + rows_per_block);
   uint32_t r0 = lo + kGroup * threadIdx.x;
-  Group cur, nxt;
-  cur.lo = cur.hi = nxt.lo = nxt.hi = make_uint4(0, 0, 0, 0);
-  cur.valid = 0;
-  if (r0 < hi && keys.n > 0) load_key(keys, 0, r0, min(kGroup, hi - r0), &cur);
-  for (uint32_t i = threadIdx.x; i < P; i += kThreads) H[i] = 0;
-  __syncthreads();
-  for (; r0 < hi; r0 += kGroup * kThreads) {
-    const uint32_t m = min(kGroup, hi - r0), r1 = r0 + kGroup * kThreads;
-    int32_t h[kGroup] = {42, 42, 42, 42};
-    for (int k = 0; k < keys.n; k++) {
-      // the next key, or the next group's first, is on its way while this one is hashed
-      if (k + 1 < keys.n) load_key(keys, k + 1, r0, m, &nxt);
-      else if (r1 < hi) load_key(keys, 0, r1, min(kGroup, hi - r1), &nxt);
-      hash_key(keys.kind[k], cur, h);
-      cur = nxt;
+  auto load = [&](int k, uint32_t r, uint32_t m, Group* g) {
+    if (kKind == kMixed && m == kGroup) {
+      const uint8_t* v = keys.values[k];
+      switch (keys.kind[k]) {
+        case KEY_I64:
+          g->lo = __ldg(reinterpret_cast<const uint4*>(v) + (r >> 1));
+          g->hi = __ldg(reinterpret_cast<const uint4*>(v) + (r >> 1) + 1);
+          break;
+        case KEY_I32: g->lo = __ldg(reinterpret_cast<const uint4*>(v) + (r >> 2)); break;
+        case KEY_I16: {
+          const uint2 x = __ldg(reinterpret_cast<const uint2*>(v) + (r >> 2));
+          g->lo.x = x.x;
+          g->lo.y = x.y;
+          break;
+        }
+        case KEY_I8: g->lo.x = __ldg(reinterpret_cast<const uint32_t*>(v) + (r >> 2)); break;
+        default: g->lo.x = load_nibble(v, r); break;
+      }
+      g->valid = keys.validity[k] != nullptr ? load_nibble(keys.validity[k], r) : 15u;
+    } else if (kKind >= 0 && m == kGroup) {
+      const uint4* v = reinterpret_cast<const uint4*>(keys.values[k]) + (r >> 2) * (kKind == KEY_I64 ? 2 : 1);
+      g->lo = __ldg(v);
+      if (kKind == KEY_I64) g->hi = __ldg(v + 1);
+      g->valid = keys.validity[k] != nullptr ? load_nibble(keys.validity[k], r) : 15u;
+    } else {
+      load_key(keys, k, r, m, g);
     }
+  };
+  auto hash = [&](int k, const Group& g, int32_t* h) { hash_key(kKind >= 0 ? kKind : keys.kind[k], g, h); };
+  // the ids of m rows from r on
+  auto put = [&](const int32_t* h, uint32_t r, uint32_t m) {
     uint32_t p[kGroup];
 #pragma unroll
     for (uint32_t u = 0; u < kGroup; u++) p[u] = pmod_div(h[u], pmod);
-    if (m == kGroup && (reinterpret_cast<uintptr_t>(pids) & 7) == 0) {
-      *reinterpret_cast<uint2*>(pids + r0) = make_uint2(p[0] | p[1] << 16, p[2] | p[3] << 16);
+    if (m == kGroup && (kKind != kAny || (reinterpret_cast<uintptr_t>(pids) & 7) == 0)) {
+      *reinterpret_cast<uint2*>(pids + r) = make_uint2(p[0] | p[1] << 16, p[2] | p[3] << 16);
     } else {
 #pragma unroll
       for (uint32_t u = 0; u < kGroup; u++)
-        if (u < m) pids[r0 + u] = (uint16_t)p[u];
+        if (u < m) pids[r + u] = (uint16_t)p[u];
     }
 #pragma unroll
     for (uint32_t u = 0; u < kGroup; u++)
       if (u < m) atomicAdd(&H[p[u]], 1u);
+  };
+  Group cur, nxt;
+  cur.lo = cur.hi = nxt.lo = nxt.hi = make_uint4(0, 0, 0, 0);
+  cur.valid = 0;
+  if (r0 + kGroup <= hi && keys.n > 0) load(0, r0, kGroup, &cur);
+  for (uint32_t i = threadIdx.x; i < P; i += kThreads) H[i] = 0;
+  __syncthreads();
+  for (; r0 + kGroup <= hi; r0 += kGroup * kThreads) {
+    const uint32_t r1 = r0 + kGroup * kThreads;
+    int32_t h[kGroup] = {42, 42, 42, 42};
+    for (int k = 0; k < keys.n; k++) {
+      // the next key, or the next group's first, is on its way while this one is hashed
+      if (k + 1 < keys.n) load(k + 1, r0, kGroup, &nxt);
+      else if (r1 + kGroup <= hi) load(0, r1, kGroup, &nxt);
+      hash(k, cur, h);
+      cur = nxt;
+    }
+    put(h, r0, kGroup);
   }
-  if (hist_in_smem) {
+  if (r0 < hi) {  // the call's last rows, fewer than a group
+    int32_t h[kGroup] = {42, 42, 42, 42};
+    for (int k = 0; k < keys.n; k++) {
+      load(k, r0, hi - r0, &cur);
+      hash(k, cur, h);
+    }
+    put(h, r0, hi - r0);
+  }
+  if (kSmem) {
     __syncthreads();
     for (uint32_t i = threadIdx.x; i < P; i += kThreads) row[i] = H[i];
   }
@@ -220,6 +268,18 @@ k_sum_tile_counts(const uint32_t* __restrict__ count_rows, uint32_t n_rows, uint
   }
 }
 
+using CountFn = void (*)(const KeySet, uint32_t, uint32_t, PmodDiv, uint16_t*, uint32_t*);
+// wide: blocks of 1024 threads share a histogram (always in shared memory)
+CountFn CountKernel(bool wide, bool smem, int kind) {
+  if (!smem) return k_hash_count_static<512, 3, false, kAny>;
+  switch (kind) {
+    case KEY_I32: return wide ? k_hash_count_static<1024, 1, true, KEY_I32> : k_hash_count_static<512, 3, true, KEY_I32>;
+    case KEY_I64: return wide ? k_hash_count_static<1024, 1, true, KEY_I64> : k_hash_count_static<512, 3, true, KEY_I64>;
+    case kMixed: return wide ? k_hash_count_static<1024, 1, true, kMixed> : k_hash_count_static<512, 3, true, kMixed>;
+    default: return wide ? k_hash_count_static<1024, 1, true, kAny> : k_hash_count_static<512, 3, true, kAny>;
+  }
+}
+
 std::mutex g_mu;
 // device address of g_tile_counts, per device ordinal, in that device's primary context (the
 // one the runtime API uses; other contexts are not supported)
@@ -235,11 +295,15 @@ cudaError_t ScratchAddress(int device, uint32_t** out, uint32_t* sms) {
     void* p = nullptr;
     cudaError_t e = cudaGetSymbolAddress(&p, g_tile_counts);
     cudaFuncAttributes fa;
-    if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, k_hash_count_static<512, 3>);
+    for (const bool wide : {false, true})
+      for (const bool smem : {false, true})
+        for (const int kind : {kAny, kMixed, (int)KEY_I32, (int)KEY_I64}) {
+          if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, CountKernel(wide, smem, kind));
+          if (e == cudaSuccess && wide && smem)
+            e = cudaFuncSetAttribute(CountKernel(wide, smem, kind), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)(kSmemHistMaxP * sizeof(uint32_t)));
+        }
     if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, k_sum_tile_counts);
-    if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(k_hash_count_static<1024, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)(kSmemHistMaxP * sizeof(uint32_t)));
     if (e == cudaSuccess && (int)g_sms.size() <= device) g_sms.resize(device + 1, 0);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&g_sms[device], cudaDevAttrMultiProcessorCount, device);
     if (e != cudaSuccess) return e;
@@ -356,8 +420,15 @@ GzStatus HashPartitionStatic(int32_t device, int32_t P, const GzKeyColumn* keys,
       cfg.gridDim = (unsigned)blocks;
       cfg.blockDim = threads;
       cfg.dynamicSmemBytes = smem_hist ? sizeof(uint32_t) * parts : 0;
-      e = cudaLaunchKernelEx(&cfg, wide ? k_hash_count_static<1024, 1> : k_hash_count_static<512, 3>, ks, n, per, pmod,
-                             smem_hist ? 1 : 0, pids, scratch);
+      // columns on their boundaries (not slices): no look at that per group, nor at the kind when there is one
+      int kind = ks.n > 0 && (ks.kind[0] == KEY_I32 || ks.kind[0] == KEY_I64) ? ks.kind[0] : kMixed;
+      if ((reinterpret_cast<uintptr_t>(pids) & 7) != 0) kind = kAny;
+      for (int k = 0; k < ks.n && kind != kAny; k++) {
+        const uint32_t wide_load = ks.kind[k] == KEY_I8 ? 4 : ks.kind[k] == KEY_I16 ? 8 : ks.kind[k] == KEY_BOOL ? 1 : 16;
+        if ((reinterpret_cast<uintptr_t>(ks.values[k]) & (wide_load - 1)) != 0) kind = kAny;
+        else if (ks.kind[k] != kind) kind = kMixed;
+      }
+      e = cudaLaunchKernelEx(&cfg, CountKernel(wide, smem_hist, kind), ks, n, per, pmod, pids, scratch);
     }
     if (e == cudaSuccess) {
       cfg.gridDim = (parts + 31) / 32;

@@ -1799,8 +1799,10 @@ cudaError_t launch_gather(const HostCopy* jobs, uint32_t n_jobs, cudaStream_t st
 }
 
 namespace {
+// piece: a multiple of align, a power of two (with a smaller one the first would start before the buffer)
 cudaError_t gather_args(const HostCopy* jobs, uint32_t n_jobs, uint32_t threads, uint32_t piece, uint32_t align, uint32_t* done,
                         uint32_t* flag, uint32_t seq, cudaStream_t st) {
+  if (piece % align != 0) return cudaErrorInvalidValue;
   GatherArgs a;
   uint32_t n = 0;
   for (uint32_t i = 0; i < n_jobs; i++) {

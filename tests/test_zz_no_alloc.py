@@ -251,3 +251,35 @@ def test_static_calls_in_a_row_and_in_a_captured_graph(many_keys):
         g.replay()
         torch.cuda.synchronize()
         check()
+
+
+# keys of one kind (their kernel, and the general one when a column or the ids lie off their boundaries)
+@pytest.mark.parametrize("off", ["", "last key", "ids"])
+@pytest.mark.parametrize("P", [1, 200, 3000, 57345])
+@pytest.mark.parametrize("keys", [[1], [0], [0, 5]])
+def test_static_ids_of_keys_of_one_kind(many_keys, keys, P, off):
+    schema, batch, _ = many_keys
+    want_all = _oracle_pids(schema, keys, P, batch)
+    cols = (GzKeyColumn * len(keys))()
+    hold = []
+    for j, k in enumerate(keys):
+        f = schema[k]
+        w = W.BYTE_WIDTH[f.type] if off == "last key" and k == keys[-1] else 0
+        t = torch.from_numpy(np.concatenate([np.zeros(w, np.uint8), batch.buffers[2 * k + 1].view(np.uint8)])).cuda()
+        m = torch.from_numpy(batch.buffers[2 * k].view(np.uint8).copy()).cuda()
+        hold += [t, m]
+        cols[j].type, cols[j].values, cols[j].validity = f.code, t.data_ptr() + w, m.data_ptr()
+    for n in (1, 4, 2047, 2048, 2051, 65533):
+        if -(-n // TILE_ROWS) * P > MAX_COUNTERS:
+            continue
+        shift = int(off == "ids")
+        out = torch.full((n + 2,), -1, dtype=torch.int16, device="cuda")
+        counts = torch.full((P,), -1, dtype=torch.int64, device="cuda")
+        st = _entry()(0, P, cols, len(keys), n, out.data_ptr() + 2 * shift, counts.data_ptr(),
+                      torch.cuda.current_stream().cuda_stream)
+        assert st == 0, _last_error()
+        got = out.cpu().numpy().view(np.uint16)
+        assert np.array_equal(got[shift:shift + n], want_all[:n])
+        assert got[shift + n] == 0xFFFF
+        assert np.array_equal(counts.cpu().numpy(), np.bincount(want_all[:n], minlength=P))
+    del hold
