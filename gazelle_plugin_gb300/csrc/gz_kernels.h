@@ -18,7 +18,7 @@ cudaError_t launch_gather_args(const HostCopy* jobs, uint32_t n_jobs, uint32_t* 
 // The derived arrays of a pass's nested columns (`jobs` in device memory); errors into *err.
 cudaError_t launch_nest_prep(const NestJob* jobs, uint32_t n_jobs, int32_t* err, cudaStream_t st);
 // One range of host bytes the device has not read before.
-cudaError_t launch_gather_stream(const HostCopy& job, cudaStream_t st);
+cudaError_t launch_gather_stream(const HostCopy& job, uint32_t* done, uint32_t* flag, uint32_t seq, cudaStream_t st);
 size_t scatter_smem_bytes();
 int max_str_columns();
 

@@ -1828,7 +1828,7 @@ cudaError_t launch_gather_args(const HostCopy* jobs, uint32_t n_jobs, uint32_t* 
   return gather_args(jobs, n_jobs, 256, piece, 16, done, flag, seq, st);
 }
 
-cudaError_t launch_gather_stream(const HostCopy& job, cudaStream_t st) {
+cudaError_t launch_gather_stream(const HostCopy& job, uint32_t* done, uint32_t* flag, uint32_t seq, cudaStream_t st) {
   if (job.bytes == 0) return cudaSuccess;
   // A reduce task's streams are pages of data files the device has not seen before: every SM that reads a
   // page asks the host for its translation, so from 256 KB on few blocks read whole pages (64 KB, a
@@ -1837,9 +1837,9 @@ cudaError_t launch_gather_stream(const HostCopy& job, cudaStream_t st) {
   // 64 KB ones (256 threads, 256 KB from the stream's start on: 29 / 72 / 111).  Eight loads a thread:
   // 45 / 89 / 113, but 2.12 ms instead of 1.94 for 141 MB of pages already translated.
   constexpr uint64_t page = 64u << 10;
-  if (job.bytes < 4 * page) return gather_args(&job, 1, 256, 16u << 10, 16, nullptr, nullptr, 0, st);
+  if (job.bytes < 4 * page) return gather_args(&job, 1, 256, 16u << 10, 16, done, flag, seq, st);
   const uint64_t piece = (job.bytes / 4 + page - 1) / page * page;
-  return gather_args(&job, 1, 1024, (uint32_t)(piece < 8 * page ? piece : 8 * page), (uint32_t)page, nullptr, nullptr, 0, st);
+  return gather_args(&job, 1, 1024, (uint32_t)(piece < 8 * page ? piece : 8 * page), (uint32_t)page, done, flag, seq, st);
 }
 
 size_t scatter_smem_bytes() {

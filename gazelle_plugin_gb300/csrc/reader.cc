@@ -11,6 +11,7 @@
 #include "host_util.h"
 #include "lz4_kernels.h"
 #include "read_kernels.h"
+#include "stream_pool.h"
 
 namespace gz {
 
@@ -114,6 +115,11 @@ Status PartitionReader::Make(std::vector<Field> fields, int device, std::unique_
   cudaDeviceGetAttribute(&pageable, cudaDevAttrPageableMemoryAccess, device);
   cudaDeviceGetAttribute(&host_tables, cudaDevAttrPageableMemoryAccessUsesHostPageTables, device);
   r->direct_ = pageable != 0 && host_tables != 0;
+  if (r->direct_) {
+    st = r->Cuda(cudaMallocAsync(reinterpret_cast<void**>(&r->d_done_), 256, r->stream_), "cudaMallocAsync(reader)");
+    if (st.ok()) st = r->Cuda(cudaMemsetAsync(r->d_done_, 0, 4, r->stream_), "memset(reader)");
+    if (!st.ok()) return st;
+  }
   r->out_.assign(r->fields_.size(), OutCol());
   *out = std::move(r);
   return Status::OK();
@@ -126,6 +132,7 @@ PartitionReader::~PartitionReader() {
   for (uint8_t* p : arena_mem_)
     if (p) cudaFreeAsync(p, stream_);
   if (out_mem_) cudaFreeAsync(out_mem_, stream_);
+  if (d_done_) cudaFreeAsync(d_done_, stream_);
   if (stream_) {
     cudaStreamSynchronize(stream_);
     cudaStreamDestroy(stream_);
@@ -336,7 +343,7 @@ Status PartitionReader::AddStream(const uint8_t* data, int64_t len) {
     // device itself where it walks the host page tables, else by a copy
     if (direct_) {
       const HostCopy job{data, d, (uint64_t)len};
-      st = Cuda(launch_gather_stream(job, stream_), "k_gather");
+      st = Cuda(launch_gather_stream(job, d_done_, &landed_, ++reads_, stream_), "k_gather");
     } else {
       st = Cuda(cudaMemcpyAsync(d, data, (size_t)len, cudaMemcpyHostToDevice, stream_), "H2D stream");
     }
@@ -461,8 +468,11 @@ Status PartitionReader::AddStream(const uint8_t* data, int64_t len) {
       x.first->o0 = word(x.second);
       x.first->o1 = word(x.second);
     }
-  } else {
-    st = Cuda(cudaStreamSynchronize(stream_), "H2D stream");
+  } else if (d != nullptr) {
+    // a word that the read's last block writes is seen sooner than the end of the stream's work (32 streams
+    // of 4.4 MB 1.87 -> 1.76 ms a reader, 36 of a few KB 1.04 -> 0.96)
+    st = direct_ ? Cuda(WaitForWord(&landed_, reads_, stream_), "H2D stream")
+                 : Cuda(cudaStreamSynchronize(stream_), "H2D stream");
     if (!st.ok()) return st;
   }
   // nested fields: list / map children hold exactly the parent's entries from 0 (as Arrow's

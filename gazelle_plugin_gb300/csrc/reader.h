@@ -112,6 +112,9 @@ class PartitionReader {
   std::vector<uint8_t*> arenas_;  // decoded compressed buffers of every stream
   std::vector<uint8_t*> arena_mem_;  // their allocations
   bool direct_ = false;        // the device reads pageable host memory (coherent link)
+  uint32_t* d_done_ = nullptr;     // blocks that have read their part of a stream
+  alignas(64) uint32_t landed_ = 0;  // number of the last stream read, written by the device
+  uint32_t reads_ = 0;             // streams read so far
   std::vector<Batch> batches_;
   std::vector<OutCol> out_;
   uint8_t* out_mem_ = nullptr;

@@ -519,15 +519,8 @@ Status Splitter::WaitHostReads() {
   Status st;
   if (reads_word_) {
     reads_word_ = false;
-    for (uint32_t polls = 1; __atomic_load_n(h_reads_, __ATOMIC_ACQUIRE) != reads_seq_; polls++) {
-      if (polls % 4096) continue;
-      // taking long: a failed launch never writes the word
-      const cudaError_t e = cudaStreamQuery(cstream_);
-      if (e == cudaSuccess) break;
-      if (e != cudaErrorNotReady) return Cuda(e, "host reads");
-      cudaGetLastError();
-      std::this_thread::yield();
-    }
+    st = Cuda(WaitForWord(h_reads_, reads_seq_, cstream_), "host reads");
+    if (!st.ok()) return st;
   } else {
     st = Cuda(cudaEventSynchronize(gather_ev_), "host reads");
     if (!st.ok()) return st;

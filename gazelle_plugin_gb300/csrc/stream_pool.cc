@@ -3,6 +3,7 @@
 #include <algorithm>
 #include <map>
 #include <mutex>
+#include <thread>
 #include <vector>
 
 namespace gz {
@@ -80,6 +81,18 @@ void ReleaseStreams(StreamSet* set) {
     }
   }
   DestroyStreams(set);
+}
+
+cudaError_t WaitForWord(const uint32_t* word, uint32_t seq, cudaStream_t st) {
+  for (uint32_t polls = 1; __atomic_load_n(word, __ATOMIC_ACQUIRE) != seq; polls++) {
+    if (polls % 4096) continue;
+    // taking long: a failed launch never writes the word
+    const cudaError_t e = cudaStreamQuery(st);
+    if (e != cudaErrorNotReady) return e;
+    cudaGetLastError();
+    std::this_thread::yield();
+  }
+  return cudaSuccess;
 }
 
 cudaError_t AcquireEvent(int device, cudaEvent_t* out) {

@@ -5,6 +5,7 @@
 // of three batches took 1.75 ms instead of 0.8, a reader of 36 short streams 2.2 instead of 1.05).
 #pragma once
 #include <cuda_runtime.h>
+#include <stdint.h>
 
 namespace gz {
 
@@ -21,6 +22,9 @@ cudaError_t AcquireStreams(int device, StreamSet* out);
 // Takes an idle set back (at most kPooledSets are kept, the others destroyed); clears *set.
 void ReleaseStreams(StreamSet* set);
 void DestroyStreams(StreamSet* set);
+
+// Waits until a launch on `st` has written seq to *word (k_gather_args), or `st` is done without.
+cudaError_t WaitForWord(const uint32_t* word, uint32_t seq, cudaStream_t st);
 
 // Timing events of the current device `device`, likewise.
 cudaError_t AcquireEvent(int device, cudaEvent_t* out);
