@@ -337,15 +337,15 @@ typedef struct GzKeyColumn {
  * cudaMalloc would escape), and code that must not stall the device, as cudaMalloc and
  * cudaFree may synchronise it.  Inputs and outputs are the caller's device memory.
  *
- * Its scratch, the per-tile row counts, is one 16 MiB array in the library's own device
+ * Its scratch, its blocks' row counts per partition, is one 16 MiB array in the library's own device
  * memory, held until the process exits on every device where the library has run.  With CUDA's
  * lazy module loading (the default) the array is reserved on a device by the first call there,
  * so make that first call (a zero-row call will do) before a pool reserves the device's free
  * memory; if it cannot be reserved the call returns GZ_OOM.  A call needs
  * ceil(num_rows / 1024) * num_partitions 32-bit counters, at most 4,194,304 (e.g. 65,536 rows
  * at 65,536 partitions, or 21 million rows at 200); a larger call returns GZ_INVALID.  All calls
- * on a device share the array and it keeps the last call's contents (each call clears what it
- * uses), so calls that may overlap on the GPU (other streams, other threads) race and give
+ * on a device share the array and it keeps the last call's contents (each call writes what it
+ * reads), so calls that may overlap on the GPU (other streams, other threads) race and give
  * wrong counts: put them on one stream.  The first call on a device looks up the array's device
  * address with that device current; make that first call before any stream capture.  Only the
  * device's primary context (the CUDA runtime's) is supported.  A CUDA error already pending on
