@@ -7,7 +7,6 @@
 #include <string.h>
 #include <sys/mman.h>
 #include <sys/stat.h>
-#include <sys/statvfs.h>
 #include <sys/uio.h>
 #include <unistd.h>
 
@@ -16,9 +15,9 @@
 #include <chrono>
 #include <functional>
 #include <numeric>
-#include <thread>
 
 #include "emit_kernels.h"
+#include "file_pages.h"
 #include "gz_kernels.h"
 #include "lz4_kernels.h"
 #include "stream_pool.h"
@@ -2024,78 +2023,12 @@ Status Splitter::WriteData(const std::vector<std::vector<SegMsg>>& msgs, const s
   return Status::OK();
 }
 
-namespace {
-
-// Makes the pages of a fresh mapping present, in order, on helper threads and on the calling one
-// whenever it has to wait.  With `allocate` a window's pages are allocated in the file system first, where
-// a full one is an error (at the first touch of a mapping it is a signal).
-struct PageToucher {
-  uint8_t* map;
-  int fd;
-  int64_t total, window, unit, page;
-  std::atomic<int64_t> next{0};
-  std::vector<std::atomic<int>> left;   // units of each window not touched yet
-  std::vector<std::atomic<int>> state;  // of each window: 1 may be touched, 0 not yet, -1 cannot be
-
-  PageToucher(uint8_t* m, int f, int64_t n, int64_t w, bool allocate)
-      : map(m), fd(f), total(n), window(w), unit(w / 8), page(sysconf(_SC_PAGESIZE)), left((size_t)((n + w - 1) / w)),
-        state(left.size()) {
-    for (size_t i = 0; i < left.size(); i++) {
-      const int64_t len = std::min(window, total - (int64_t)i * window);
-      left[i].store((int)((len + unit - 1) / unit));
-      state[i].store(allocate ? 0 : 1);
-    }
-  }
-  // One unit; false when there are none left.
-  bool Work() {
-    const int64_t lo = next.fetch_add(unit);
-    if (lo >= total) return false;
-    const size_t w = (size_t)(lo / window);
-    const int64_t w0 = (int64_t)w * window, hi = std::min(total, lo + unit);
-    if (state[w].load() == 0) {
-      if (lo == w0) {  // units are claimed in order: a window's first one is always on its way
-        int r;
-        while ((r = fallocate(fd, 0, w0, std::min(window, total - w0))) != 0 && errno == EINTR) {
-        }
-        state[w].store(r == 0 ? 1 : -1);
-      } else {
-        while (state[w].load() == 0) std::this_thread::yield();
-      }
-    }
-    if (state[w].load() > 0)
-      for (int64_t x = lo; x < hi; x += page) *reinterpret_cast<volatile uint8_t*>(map + x) = 0;
-    left[w].fetch_sub(1);
-    return true;
-  }
-  // Until window w's pages are there; false when they cannot be.
-  bool Wait(size_t w) {
-    while (left[w].load() > 0)
-      if (!Work()) std::this_thread::yield();
-    return state[w].load() > 0;
-  }
-};
-
-// Bytes of the files this process is writing through mappings without having allocated them.
-std::atomic<int64_t> g_unallocated{0};
-
-// Whether `total` more bytes go into the file system of `fd` with room to spare: then its pages are
-// allocated by their first touch.  Allocating them beforehand serialises on the file's lock (a 720 MB
-// file: 11.2 ms against 6.0), so that is left to file systems that are nearly full.
-bool RoomToSpare(int fd, int64_t total) {
-  struct statvfs v;
-  if (fstatvfs(fd, &v) != 0) return false;
-  const int64_t room = (int64_t)v.f_bavail * (int64_t)v.f_frsize, size = (int64_t)v.f_blocks * (int64_t)v.f_frsize;
-  return room > 2 * (g_unallocated.load() + total) + std::max<int64_t>(1ll << 30, size / 20);
-}
-
-}  // namespace
-
 Status Splitter::EmitData(const std::vector<std::vector<SegMsg>>& msgs, const std::vector<uint8_t>& schema_msg,
                           const std::vector<int64_t>& start, int64_t total) {
   // the file, or memory, mapped whole; no mapping: through a pinned block
   int fd = -1;
   uint8_t* map = nullptr;
-  bool spare = true;
+  int zero = -1;
   if (data_file_.empty()) {
     data_bytes_.reset(new uint8_t[(size_t)std::max<int64_t>(total, 1)]);
     data_size_ = total;
@@ -2108,11 +2041,12 @@ Status Splitter::EmitData(const std::vector<std::vector<SegMsg>>& msgs, const st
       close(fd);
       return Status::Error(GZ_IO, "cannot size data file " + data_file_ + ": " + why);
     }
-    // a mapping only where it cannot run out of space under the copy
-    spare = RoomToSpare(fd, total);
-    if (total > 0 && (spare || fallocate(fd, 0, 0, 1) == 0 || errno == ENOSPC || errno == EINTR)) {
+    // a mapping only with what makes its pages present without a signal where they cannot be
+    if (total > 0) zero = open("/dev/zero", O_RDONLY | O_CLOEXEC);
+    if (zero >= 0) {
       void* m = mmap(nullptr, (size_t)total, PROT_READ | PROT_WRITE, MAP_SHARED, fd, 0);
       if (m != MAP_FAILED) map = static_cast<uint8_t*>(m);
+      else close(zero);
     }
   }
   if (total == 0) return fd >= 0 && close(fd) != 0 ? Status::Error(GZ_IO, "writing the data file failed: " + data_file_)
@@ -2122,20 +2056,19 @@ Status Splitter::EmitData(const std::vector<std::vector<SegMsg>>& msgs, const st
   const size_t nw = (size_t)((total + W - 1) / W);
   std::shared_ptr<PageToucher> pages;
   if (map) {
-    pages = std::make_shared<PageToucher>(map, fd, total, W, !spare);
-    if (fd >= 0 && spare) g_unallocated.fetch_add(total);
-    // eight threads in all: more only contend (720 MB of tmpfs pages: 8.7 ms with 4, 6.3 with 8, 7.3 with 16)
-    Background((int)std::min<int64_t>(7, total / pages->unit), [pages] {
+    // eight threads in all: more only contend (720 MB of tmpfs pages: 8.9 ms with 4, 6.7 with 8, 7.5 with 12);
+    // none to help: many Stops at once
+    const int helpers = ParallelHelpers(7);
+    pages = std::make_shared<PageToucher>(map, total, W, zero, helpers == 0 ? fd : -1);
+    Background((int)std::min<int64_t>(helpers, total / pages->unit()), [pages] {
       while (pages->Work()) {
       }
     });
   }
   Status st = EmitWindows(msgs, schema_msg, start, total, W, fd, map, pages ? [&](size_t w) { return pages->Wait(w); }
                                                                             : std::function<bool(size_t)>());
-  if (pages) {
+  if (pages)
     for (size_t w = 0; w < nw; w++) pages->Wait(w);  // nobody touches the mapping any more
-    if (fd >= 0 && spare) g_unallocated.fetch_sub(total);
-  }
   if (fd >= 0) {
     bool ok = true;
     if (map && munmap(map, (size_t)total) != 0) ok = false;
