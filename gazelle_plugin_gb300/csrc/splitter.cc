@@ -1960,12 +1960,42 @@ Status Splitter::Stop() {
   return Status::OK();
 }
 
+namespace {
+
+// Maps the n > 0 bytes of `fd`; nullptr where that is not possible, or not with what makes the pages present
+// without a signal where they cannot be.  *zero: as MakePresent takes it, to be closed.
+uint8_t* MapForWriting(int fd, int64_t n, int* zero) {
+  *zero = open("/dev/zero", O_RDONLY | O_CLOEXEC);
+  if (*zero < 0) return nullptr;
+  void* m = mmap(nullptr, (size_t)n, PROT_READ | PROT_WRITE, MAP_SHARED, fd, 0);
+  if (m != MAP_FAILED) return static_cast<uint8_t*>(m);
+  close(*zero);
+  *zero = -1;
+  return nullptr;
+}
+
+// Starts to make the n bytes at `map` present (fd, zero: -1 for heap memory).
+std::shared_ptr<PageToucher> StartPages(uint8_t* map, int64_t n, int64_t window, int zero, int fd) {
+  // eight threads in all: more only contend (720 MB of tmpfs pages: 8.9 ms with 4, 6.7 with 8, 7.5 with 12);
+  // none to help: many Stops at once
+  const int helpers = ParallelHelpers(7);
+  auto pages = std::make_shared<PageToucher>(map, n, window, zero, helpers == 0 ? fd : -1);
+  Background((int)std::min<int64_t>(helpers, n / pages->unit()), [pages] {
+    while (pages->Work()) {
+    }
+  });
+  return pages;
+}
+
+}  // namespace
+
 // The data file's bytes written by the CPU from the host copies of the pass outputs.
 Status Splitter::WriteData(const std::vector<std::vector<SegMsg>>& msgs, const std::vector<uint8_t>& schema_msg,
                            const std::vector<int64_t>& start, int64_t total) {
   int fd = -1;
   uint8_t* mem = nullptr;
   void* mapped = nullptr;
+  int zero = -1;
   if (data_file_.empty()) {
     data_bytes_.reset(new uint8_t[(size_t)std::max<int64_t>(total, 1)]);
     data_size_ = total;
@@ -1982,11 +2012,7 @@ Status Splitter::WriteData(const std::vector<std::vector<SegMsg>>& msgs, const s
     }
     // Writes to one file serialise on the file's lock; a large file is mapped instead, so that
     // the partitions are copied into it in parallel.
-    if (regular && total >= kMapWriteBytes) {
-      mapped = mmap(nullptr, (size_t)total, PROT_READ | PROT_WRITE, MAP_SHARED, fd, 0);
-      if (mapped == MAP_FAILED) mapped = nullptr;
-      else mem = static_cast<uint8_t*>(mapped);
-    }
+    if (regular && total >= kMapWriteBytes) mapped = mem = MapForWriting(fd, total, &zero);
   }
   static const uint32_t kEos[2] = {0xFFFFFFFFu, 0u};  // WriteEOS (splitter.cc:166-172)
   std::vector<char> wrote(P_, 1);
@@ -2012,12 +2038,16 @@ Status Splitter::WriteData(const std::vector<std::vector<SegMsg>>& msgs, const s
   } else {
     ParallelFor((size_t)P_, [&](size_t pi) {
       RangeWriter w(fd, mem, start[pi]);
-      wrote[pi] = put(w, (int)pi) && w.Flush();
+      // (in a mapping the pages first: a store to one that there is no space for is a signal.  290 MB: a Stop
+      // of 8.3 ms instead of 7.3)
+      const bool there = !mapped || MakePresent(mem, start[pi], start[pi + 1], zero, -1);
+      wrote[pi] = there && put(w, (int)pi) && w.Flush();
     });
   }
   bool ok = true;
   for (int p = 0; p < P_; p++) ok = ok && wrote[p];
   if (mapped && munmap(mapped, (size_t)total) != 0) ok = false;
+  if (zero >= 0) close(zero);
   if (fd >= 0 && close(fd) != 0) ok = false;
   if (!ok) return Status::Error(GZ_IO, "writing the data file failed: " + data_file_);
   return Status::OK();
@@ -2041,13 +2071,7 @@ Status Splitter::EmitData(const std::vector<std::vector<SegMsg>>& msgs, const st
       close(fd);
       return Status::Error(GZ_IO, "cannot size data file " + data_file_ + ": " + why);
     }
-    // a mapping only with what makes its pages present without a signal where they cannot be
-    if (total > 0) zero = open("/dev/zero", O_RDONLY | O_CLOEXEC);
-    if (zero >= 0) {
-      void* m = mmap(nullptr, (size_t)total, PROT_READ | PROT_WRITE, MAP_SHARED, fd, 0);
-      if (m != MAP_FAILED) map = static_cast<uint8_t*>(m);
-      else close(zero);
-    }
+    if (total > 0) map = MapForWriting(fd, total, &zero);
   }
   if (total == 0) return fd >= 0 && close(fd) != 0 ? Status::Error(GZ_IO, "writing the data file failed: " + data_file_)
                                                    : Status::OK();
@@ -2055,16 +2079,7 @@ Status Splitter::EmitData(const std::vector<std::vector<SegMsg>>& msgs, const st
   const int64_t W = std::min(kEmitWindow, std::max<int64_t>(2 << 20, (int64_t)AlignUp((size_t)total / 8, 1 << 20)));
   const size_t nw = (size_t)((total + W - 1) / W);
   std::shared_ptr<PageToucher> pages;
-  if (map) {
-    // eight threads in all: more only contend (720 MB of tmpfs pages: 8.9 ms with 4, 6.7 with 8, 7.5 with 12);
-    // none to help: many Stops at once
-    const int helpers = ParallelHelpers(7);
-    pages = std::make_shared<PageToucher>(map, total, W, zero, helpers == 0 ? fd : -1);
-    Background((int)std::min<int64_t>(helpers, total / pages->unit()), [pages] {
-      while (pages->Work()) {
-      }
-    });
-  }
+  if (map) pages = StartPages(map, total, W, zero, fd);
   Status st = EmitWindows(msgs, schema_msg, start, total, W, fd, map, pages ? [&](size_t w) { return pages->Wait(w); }
                                                                             : std::function<bool(size_t)>());
   if (pages)

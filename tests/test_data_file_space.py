@@ -35,7 +35,7 @@ int main(int, char** v) {
     mem.reset(new uint8_t[total]);
     map = mem.get();
   } else {
-    fd = open(v[1], O_RDWR | O_CREAT | O_TRUNC, 0600);
+    fd = open(v[1] + (v[1][0] == '+'), O_RDWR | O_CREAT | O_TRUNC, 0600);
     if (fd < 0 || ftruncate(fd, file) != 0) return 2;
     map = static_cast<uint8_t*>(mmap(nullptr, total, PROT_READ | PROT_WRITE, MAP_SHARED, fd, 0));
     if (map == MAP_FAILED) return 2;
@@ -53,6 +53,12 @@ int main(int, char** v) {
   int64_t present = 0;
   if (!heap && mincore(map, total, in.data()) == 0)
     for (unsigned char c : in) present += c & 1;
+  if (v[1][0] == '+') {  // ranges that end on a boundary and 50 bytes after it, where the file ends there
+    if (ftruncate(fd, page * 700) != 0) return 2;
+    const int zero = open("/dev/zero", O_RDONLY);
+    if (!gz::MakePresent(map, page * 3 + 100, page * 700, zero, -1)) return 3;
+    if (gz::MakePresent(map, page * 3 + 100, page * 700 + 50, zero, -1)) return 4;
+  }
   printf("%ld of %ld windows, %ld of %ld pages\n", (long)ok, (long)nw, (long)present, (long)n);
   return 0;
 }
@@ -78,6 +84,12 @@ def test_pages_come_up_window_by_window(driver, tmp_path, total, threads, alloca
     assert (r.returncode, r.stdout) == (0, f"{nw} of {nw} windows, {n} of {n} pages\n")
     r = subprocess.run([driver, "", "0", str(total), str(2 << 20), str(threads), allocate], capture_output=True, text=True)
     assert r.returncode == 0 and r.stdout.startswith(f"{nw} of {nw} windows")
+
+
+def test_every_page_of_a_range_off_the_page_boundaries(driver, tmp_path):
+    total = os.sysconf("SC_PAGESIZE") * 800
+    r = subprocess.run([driver, "+" + str(tmp_path / "f"), str(total), str(total), str(2 << 20), "0", "0"], capture_output=True, text=True)
+    assert r.returncode == 0, r
 
 
 @pytest.mark.parametrize("threads", [0, 7])
@@ -110,15 +122,15 @@ def _small_tmpfs(tmp_path):
     return mnt, mount
 
 
-def _stop(path, device, tasks):
-    """Map tasks of the wide table that write about 40 MB each (a child process: see below)."""
+def _stop(path, device, tasks, n=56, **kw):
+    """Map tasks of the wide table that write about 0.72 MB a batch (a child process: see below)."""
     rng = np.random.default_rng(5)
-    batches = [W.c2_batch(rng, 4096) for _ in range(56)]
+    batches = [W.c2_batch(rng, 4096) for _ in range(n)]
     w = S.ShuffleSplitterJniWrapper()
 
     def task(p):
         h = w.make(S.NativePartitioning("hash", 200, None, W.C2_KEYS, list(W.C2_SCHEMA)), dataFile=p,
-                   keep_output_on_device=device)
+                   keep_output_on_device=device, **kw)
         for b in batches:
             a, z = b.addrs_sizes()
             w.split(h, b.num_rows, a, z)
@@ -144,5 +156,15 @@ def _stop(path, device, tasks):
 def test_gpu_stop_into_a_full_file_system_is_an_io_error(tmp_path, device, tasks):
     mnt, mount = _small_tmpfs(tmp_path)
     call = f"from tests.test_data_file_space import _stop; _stop({str(mnt / 'x.data')!r}, {device}, {tasks})"
+    r = subprocess.run(mount + [sys.executable, "-c", call], cwd=ROOT, capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0 and "reported" in r.stdout, (r.returncode, r.stdout, r.stderr)
+
+
+@pytest.mark.gpu
+def test_gpu_large_file_gathered_by_the_cpu_into_a_full_file_system_is_an_io_error(tmp_path):
+    """From 256 MB on the CPU copies into a mapping as well (passes may lie in local-dir files)."""
+    mnt, mount = _small_tmpfs(tmp_path)
+    call = (f"from tests.test_data_file_space import _stop; "
+            f"_stop({str(mnt / 'x.data')!r}, 0, 1, n=400, host_budget=1 << 40, localDirs={str(tmp_path)!r})")
     r = subprocess.run(mount + [sys.executable, "-c", call], cwd=ROOT, capture_output=True, text=True, timeout=300)
     assert r.returncode == 0 and "reported" in r.stdout, (r.returncode, r.stdout, r.stderr)
