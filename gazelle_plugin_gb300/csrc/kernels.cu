@@ -9,6 +9,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "device_info.h"
 #include "gz_engine.cuh"
 #include "gz_hash.cuh"
 #include "gz_kernels.h"
@@ -1742,8 +1743,7 @@ cudaError_t launch_hash_count(const SchemaDesc& sd, const FlushDesc& fd, cudaStr
   const size_t sm = fd.hist_in_smem ? sizeof(uint32_t) * sd.P * (1 + sd.n_str) : 0;
   const bool lists = sd.list_mask != 0;
   if (sm > 48 * 1024) {
-    cudaError_t e = lists ? cudaFuncSetAttribute(k_hash_count<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm)
-                          : cudaFuncSetAttribute(k_hash_count<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    const cudaError_t e = AllowSharedMemory(lists ? (const void*)k_hash_count<true> : (const void*)k_hash_count<false>, sm);
     if (e != cudaSuccess) return e;
   }
   if (lists) k_hash_count<true><<<fd.n_segs, kHashThreads, sm, st>>>(sd, fd);
@@ -1787,13 +1787,7 @@ cudaError_t launch_gather(const HostCopy* jobs, uint32_t n_jobs, cudaStream_t st
   if (n_jobs == 0) return cudaSuccess;
   // two CTAs per SM stride over the buffers: enough loads in flight to fill the host link
   // while leaving the SMs to the device pass that runs concurrently
-  static int sms = 0;
-  if (sms == 0) {
-    int dev = 0;
-    cudaGetDevice(&dev);
-    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0) sms = 152;
-  }
-  const uint32_t grid = n_jobs < (uint32_t)(2 * sms) ? n_jobs : (uint32_t)(2 * sms);
+  const uint32_t cap = 2u * (uint32_t)SmCount(), grid = n_jobs < cap ? n_jobs : cap;
   k_gather<<<grid, 256, 0, st>>>(jobs, n_jobs);
   return cudaGetLastError();
 }
@@ -1851,13 +1845,8 @@ size_t scatter_smem_bytes() {
 
 cudaError_t launch_scatter(const SchemaDesc& sd, const FlushDesc& fd, cudaStream_t st) {
   const size_t sm = scatter_smem_bytes();
-  static bool attr_set = false;
-  if (!attr_set) {
-    cudaError_t e = cudaFuncSetAttribute(k_scatter<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_scatter<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    if (e != cudaSuccess) return e;
-    attr_set = true;
-  }
+  const cudaError_t e = AllowSharedMemory(sd.list_mask ? (const void*)k_scatter<true> : (const void*)k_scatter<false>, sm);
+  if (e != cudaSuccess) return e;
   if (sd.list_mask) k_scatter<true><<<fd.n_tiles, kScatterBlock, sm, st>>>(sd, fd);
   else k_scatter<false><<<fd.n_tiles, kScatterBlock, sm, st>>>(sd, fd);
   return cudaGetLastError();

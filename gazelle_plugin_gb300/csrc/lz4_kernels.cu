@@ -30,6 +30,7 @@
 #include <stdint.h>
 
 #include "copy.cuh"
+#include "device_info.h"
 #include "lz4_kernels.h"
 
 namespace gz {
@@ -707,31 +708,17 @@ __global__ void __launch_bounds__(kWarps * 32) k_lz4_place(const Lz4Frame* __res
   copy_bytes<kWarps * 32>(fr.dst + before, from, sl.size, threadIdx.x);
 }
 
-int sm_count() {
-  static int sms = 0;
-  if (sms == 0) {
-    int dev = 0;
-    cudaGetDevice(&dev);
-    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0) sms = 152;
-  }
-  return sms;
-}
-
 }  // namespace
 
-uint32_t lz4_compress_warps() { return (uint32_t)sm_count() * kCBlocks * kCWarps; }
+uint32_t lz4_compress_warps() { return (uint32_t)SmCount() * kCBlocks * kCWarps; }
 
 cudaError_t launch_lz4_compress(const Lz4Chunk* chunks, uint32_t n_chunks, uint32_t* next, uint8_t* scratch,
                                 uint8_t* out, unsigned long long* out_used, unsigned long long out_cap,
                                 Lz4Block* res, bool skip_stored, int32_t* err, cudaStream_t st) {
   if (n_chunks == 0) return cudaSuccess;
   const uint32_t grid = lz4_compress_warps() / kCWarps;
-  static bool attr = false;
-  if (!attr) {
-    cudaError_t e = cudaFuncSetAttribute(k_lz4_compress, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kCompressSmem);
-    if (e != cudaSuccess) return e;
-    attr = true;
-  }
+  const cudaError_t e = AllowSharedMemory((const void*)k_lz4_compress, kCompressSmem);
+  if (e != cudaSuccess) return e;
   k_lz4_compress<<<grid, kCWarps * 32, kCompressSmem, st>>>(chunks, n_chunks, next, scratch, out, out_used, out_cap, res, skip_stored, err);
   return cudaGetLastError();
 }
@@ -804,17 +791,13 @@ void lz4_index(const uint8_t* const* src, Lz4Frame* frames, uint32_t n, std::vec
 cudaError_t launch_lz4_decode(const Lz4Frame* frames, Lz4Slot* slots, uint32_t n_slots, uint8_t* slot_mem, int32_t* err,
                               cudaStream_t st) {
   if (n_slots == 0) return cudaSuccess;
-  static bool attr = false;
-  if (!attr) {
-    const cudaError_t e = cudaFuncSetAttribute(k_lz4_blocks, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDecodeSmem);
-    if (e != cudaSuccess) return e;
-    attr = true;
-  }
+  cudaError_t e = AllowSharedMemory((const void*)k_lz4_blocks, kDecodeSmem);
+  if (e != cudaSuccess) return e;
   // the second comes up while the first runs, unless there are more blocks than can run at once: it would
   // hold what they wait for
-  const bool early = n_slots <= 2u * (uint32_t)sm_count();
+  const bool early = n_slots <= 2u * (uint32_t)SmCount();
   k_lz4_blocks<<<n_slots, kDT, kDecodeSmem, st>>>(frames, slots, slot_mem, early);
-  cudaError_t e = cudaGetLastError();
+  e = cudaGetLastError();
   if (e != cudaSuccess) return e;
   cudaLaunchAttribute at;
   at.id = cudaLaunchAttributeProgrammaticStreamSerialization;

@@ -10,6 +10,7 @@
 #include <stdint.h>
 
 #include "copy.cuh"
+#include "device_info.h"
 #include "read_kernels.h"
 
 #include <algorithm>
@@ -78,13 +79,7 @@ __global__ void __launch_bounds__(kThreads) k_read_words(const int32_t* const* _
 }
 
 unsigned grid_for(uint32_t n_jobs) {
-  static int sms = 0;
-  if (sms == 0) {
-    int dev = 0;
-    cudaGetDevice(&dev);
-    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0) sms = 152;
-  }
-  const uint32_t cap = 8u * (uint32_t)sms;
+  const uint32_t cap = 8u * (uint32_t)SmCount();
   return n_jobs < cap ? n_jobs : cap;
 }
 

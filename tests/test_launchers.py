@@ -1,0 +1,126 @@
+"""The host side of the kernel launches against a stand-in for the CUDA runtime with two devices (no GPU is
+used): what a device has to be told before a launch is told to every device."""
+import os
+import subprocess
+
+import pytest
+
+from gazelle_plugin_gb300 import build as B
+
+# Knows of each (device, kernel) the dynamic shared memory allowed, and refuses a launch that asks for more, as
+# the runtime does; 48 KB need no leave.
+RUNTIME = r"""
+#include <cuda_runtime.h>
+#include <stdio.h>
+#include <map>
+#include <string>
+#include <utility>
+#include <vector>
+static int g_dev = 0, g_lowered = 0, g_launched[2] = {0, 0};
+static std::vector<std::string> g_calls;
+static cudaError_t g_last = cudaSuccess;
+static std::map<std::pair<int, const void*>, int> g_limit;
+static struct { dim3 g, b; size_t sm; cudaStream_t st; } g_cfg;
+static cudaError_t launch(const void* f, size_t sm) {
+  auto it = g_limit.find({g_dev, f});
+  if (sm > (size_t)(it == g_limit.end() ? 48 * 1024 : it->second)) return g_last = cudaErrorInvalidValue;
+  g_launched[g_dev]++;
+  g_calls.push_back("launch");
+  return cudaSuccess;
+}
+extern "C" {
+void** __cudaRegisterFatBinary(void*) { static void* h; return &h; }
+void __cudaRegisterFatBinaryEnd(void**) {}
+void __cudaUnregisterFatBinary(void**) {}
+void __cudaRegisterFunction(void**, const char*, char*, const char*, int, uint3*, uint3*, dim3*, dim3*, int*) {}
+void __cudaRegisterVar(void**, char*, char*, const char*, int, size_t, int, int) {}
+cudaError_t __cudaGetKernel(cudaKernel_t* k, const void* f) { *k = (cudaKernel_t)f; return cudaSuccess; }
+unsigned __cudaPushCallConfiguration(dim3 g, dim3 b, size_t sm, cudaStream_t st) { g_cfg = {g, b, sm, st}; return 0; }
+cudaError_t __cudaPopCallConfiguration(dim3* g, dim3* b, size_t* sm, void* st) {
+  *g = g_cfg.g; *b = g_cfg.b; *sm = g_cfg.sm; *(cudaStream_t*)st = g_cfg.st;
+  return cudaSuccess;
+}
+cudaError_t __cudaLaunchKernel(cudaKernel_t k, dim3, dim3, void**, size_t sm, cudaStream_t) { return launch((const void*)k, sm); }
+cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t* c, const void* f, void**) { return launch(f, c->dynamicSmemBytes); }
+cudaError_t cudaGetLastError() { cudaError_t e = g_last; g_last = cudaSuccess; return e; }
+cudaError_t cudaPeekAtLastError() { return g_last; }
+const char* cudaGetErrorString(cudaError_t) { return "an error"; }
+cudaError_t cudaGetDevice(int* d) { *d = g_dev; return cudaSuccess; }
+cudaError_t cudaSetDevice(int d) { g_dev = d; g_calls.push_back("device " + std::to_string(d)); return cudaSuccess; }
+cudaError_t cudaDeviceGetAttribute(int* v, cudaDeviceAttr, int d) { *v = d == 0 ? 152 : 100; return cudaSuccess; }
+cudaError_t cudaFuncGetAttributes(cudaFuncAttributes*, const void*) { return cudaSuccess; }
+cudaError_t cudaGetSymbolAddress(void** p, const void*) { static char mem[256]; *p = mem; g_calls.push_back("symbol"); return cudaSuccess; }
+cudaError_t cudaFuncSetAttribute(const void* f, cudaFuncAttribute a, int v) {
+  if (a == cudaFuncAttributeMaxDynamicSharedMemorySize) {
+    int& have = g_limit[{g_dev, f}];
+    if (v < have) g_lowered++;
+    have = v;
+  }
+  return cudaSuccess;
+}
+}
+"""
+
+
+def _object(src, where):
+    """The built object of a source file, or one made here when it is missing or older than a source."""
+    obj = os.path.join(B.BUILD_DIR, os.path.splitext(src)[0] + ".o")
+    newest = max(os.path.getmtime(os.path.join(B.CSRC, f)) for f in os.listdir(B.CSRC))
+    if os.path.exists(obj) and os.path.getmtime(obj) >= newest:
+        return obj
+    obj = os.path.join(where, os.path.basename(obj))
+    subprocess.run([B.nvcc(), *B.GENCODE, "-O3", "-std=c++17", "-Xcompiler", "-fPIC", "-I", os.path.join(B.ROOT, "include"),
+                    "-c", os.path.join(B.CSRC, src), "-o", obj], check=True)
+    return obj
+
+
+def _run(where, objects, main):
+    """Builds and runs `main` (C++ statements; check(x, what) notes what does not hold) over the objects."""
+    try:
+        cuda = os.path.join(os.path.dirname(os.path.dirname(B.nvcc())), "include")
+    except RuntimeError:
+        pytest.skip("no CUDA toolkit")
+    src, exe = os.path.join(where, "m.cc"), os.path.join(where, "m")
+    with open(src, "w") as f:
+        f.write(RUNTIME + """
+#include "gz_kernels.h"
+#include "hash_static.h"
+#include "lz4_kernels.h"
+#include "read_kernels.h"
+static int bad = 0;
+static void check(bool ok, const char* what) { if (!ok) { bad++; printf("%s\\n", what); } }
+int main() {
+""" + main + "\n  return bad != 0;\n}\n")
+    subprocess.run(["g++", "-std=c++17", "-O1", "-I", cuda, "-I", B.CSRC, "-I", os.path.join(B.ROOT, "include"), src,
+                    *[_object(o, where) for o in objects], "-o", exe, "-pthread"], check=True)
+    r = subprocess.run([exe], capture_output=True, text=True, timeout=120)
+    assert r.returncode == 0, r.stdout + r.stderr
+
+
+def test_every_device_allows_the_shared_memory_of_its_launches(tmp_path):
+    _run(str(tmp_path), ["kernels.cu", "lz4_kernels.cu", "read_kernels.cu", "device_info.cc"], r"""
+  using namespace gz;
+  static SchemaDesc sd;
+  static FlushDesc fd;
+  fd.n_segs = fd.n_tiles = 1;
+  fd.hist_in_smem = 1;
+  uint32_t warps[2];
+  for (int round = 0; round < 2; round++)
+    for (int dev = 0; dev < 2; dev++) {
+      cudaSetDevice(dev);
+      check(launch_lz4_decode(nullptr, nullptr, 3, nullptr, nullptr, 0) == cudaSuccess, "LZ4 decode");
+      check(launch_lz4_compress(nullptr, 3, nullptr, nullptr, nullptr, nullptr, 0, nullptr, false, nullptr, 0) == cudaSuccess, "LZ4 compress");
+      for (int lists = 0; lists < 2; lists++) {
+        sd.list_mask = lists;
+        check(launch_scatter(sd, fd, 0) == cudaSuccess, "k_scatter");
+        for (int P : {40000, 20000, 40000}) {
+          sd.P = P;
+          check(launch_hash_count(sd, fd, 0) == cudaSuccess, "k_hash_count");
+        }
+      }
+      warps[dev] = lz4_compress_warps();
+    }
+  check(g_launched[0] == g_launched[1], "a launch on one device only");
+  check(g_lowered == 0, "a limit lowered, which another thread's launch may rely on");
+  check(warps[0] * 100 == warps[1] * 152, "the grid of the other device");
+""")
