@@ -378,7 +378,9 @@ GzStatus HashPartitionStatic(int32_t device, int32_t P, const GzKeyColumn* keys,
   }
   int prev = -1;
   cudaError_t e = cudaGetDevice(&prev);
-  if (e == cudaSuccess && prev != device) e = cudaSetDevice(device);
+  // also when that is the device already: a context of the driver API's own may be current, in which the
+  // primary context's array and kernels are not at hand
+  if (e == cudaSuccess) e = cudaSetDevice(device);
   uint32_t* scratch = nullptr;
   uint32_t sms = 0;
   if (e == cudaSuccess) {

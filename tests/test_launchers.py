@@ -124,3 +124,25 @@ def test_every_device_allows_the_shared_memory_of_its_launches(tmp_path):
   check(g_lowered == 0, "a limit lowered, which another thread's launch may rely on");
   check(warps[0] * 100 == warps[1] * 152, "the grid of the other device");
 """)
+
+
+def test_partition_ids_make_the_device_s_primary_context_current(tmp_path):
+    """cudaSetDevice before anything that belongs to a context, on every call and also when the device is
+    current already: a context of the driver API's own may be."""
+    _run(str(tmp_path), ["hash_static.cu"], r"""
+  int64_t counts[8];
+  uint16_t ids[8];
+  int32_t values[8] = {};
+  GzKeyColumn key{};
+  key.type = GZ_TYPE_INT32;
+  key.values = reinterpret_cast<const uint8_t*>(values);
+  std::string msg;
+  for (int call = 0; call < 2; call++)
+    for (int dev = 0; dev < 2; dev++) {
+      g_dev = 0;
+      g_calls.clear();
+      check(gz::HashPartitionStatic(dev, 8, &key, 1, 8, ids, counts, 0, &msg) == GZ_OK, "the call");
+      check(!g_calls.empty() && g_calls[0] == "device " + std::to_string(dev), "its device is made current first");
+      check(g_dev == 0, "the caller's device is current again");
+    }
+""")
