@@ -1944,7 +1944,11 @@ Status Splitter::Stop() {
   const int64_t t0 = NowNs();
   if (emit_at_stop_) st = EmitData(msgs, schema_msg, start, total);
   else st = WriteData(msgs, schema_msg, start, total);
-  if (!st.ok()) return st;
+  if (!st.ok()) {
+    data_bytes_.reset();  // (in memory) not all written
+    return st;
+  }
+  if (data_file_.empty()) data_size_ = total;
   total_bytes_written_ += total;
   stat_emitted_ = 0;
   for (auto& v : segments_) stat_emitted_ += (int64_t)v.size();
@@ -1998,7 +2002,6 @@ Status Splitter::WriteData(const std::vector<std::vector<SegMsg>>& msgs, const s
   int zero = -1;
   if (data_file_.empty()) {
     data_bytes_.reset(new uint8_t[(size_t)std::max<int64_t>(total, 1)]);
-    data_size_ = total;
     mem = data_bytes_.get();
   } else {
     fd = open(data_file_.c_str(), O_RDWR | O_CREAT | O_TRUNC, 0644);
@@ -2061,7 +2064,6 @@ Status Splitter::EmitData(const std::vector<std::vector<SegMsg>>& msgs, const st
   int zero = -1;
   if (data_file_.empty()) {
     data_bytes_.reset(new uint8_t[(size_t)std::max<int64_t>(total, 1)]);
-    data_size_ = total;
     map = data_bytes_.get();
   } else {
     fd = open(data_file_.c_str(), O_RDWR | O_CREAT | O_TRUNC | O_CLOEXEC, 0644);

@@ -1,0 +1,110 @@
+"""Calls while device memory is short: the device's memory pool is replaced by one of a limited size, filled
+up as far as a test wants, so that the library's stream-ordered allocations fail as they would with the
+device's memory in other hands."""
+import contextlib
+import ctypes
+
+import numpy as np
+import pytest
+
+from gazelle_plugin_gb300 import shuffle as S
+from gazelle_plugin_gb300 import workloads as W
+from oracle import oracle as O
+
+pytestmark = pytest.mark.gpu
+
+torch = pytest.importorskip("torch")
+
+
+class _Props(ctypes.Structure):  # CUmemPoolProps
+    _fields_ = [("alloc_type", ctypes.c_int), ("handle_types", ctypes.c_int), ("location_type", ctypes.c_int),
+                ("location_id", ctypes.c_int), ("security", ctypes.c_void_p), ("max_size", ctypes.c_size_t),
+                ("usage", ctypes.c_ushort), ("reserved", ctypes.c_ubyte * 54)]
+
+
+class Pool:
+    """Device 0's current memory pool: at most `size` bytes."""
+
+    def __init__(self, size):
+        torch.zeros(1, device="cuda")  # the primary context is current
+        self.cu = ctypes.CDLL("libcuda.so.1")
+        self.dev = ctypes.c_int(0)
+        props = _Props(alloc_type=1, location_type=1, max_size=size)  # PINNED on a DEVICE
+        self.pool, self.before, self.held = ctypes.c_void_p(), ctypes.c_void_p(), []
+        self._ok(self.cu.cuDeviceGetMemPool(ctypes.byref(self.before), self.dev))
+        self._ok(self.cu.cuMemPoolCreate(ctypes.byref(self.pool), ctypes.byref(props)))
+        self._ok(self.cu.cuDeviceSetMemPool(self.dev, self.pool))
+
+    @staticmethod
+    def _ok(r):
+        assert r == 0, f"CUDA driver error {r}"
+
+    def fill(self, leave=0):
+        """Takes what is left of the pool, but for about `leave` bytes."""
+        torch.cuda.synchronize()
+        spare = ctypes.c_void_p()
+        if leave:
+            self._ok(self.cu.cuMemAllocFromPoolAsync(ctypes.byref(spare), ctypes.c_size_t(leave), self.pool, None))
+        size = 1 << 30
+        while size >= 4096:
+            p = ctypes.c_void_p()
+            r = self.cu.cuMemAllocFromPoolAsync(ctypes.byref(p), ctypes.c_size_t(size), self.pool, None)
+            if r == 0:
+                self.held.append(p)
+            else:
+                assert r == 2, r  # CUDA_ERROR_OUT_OF_MEMORY
+                size //= 2
+        if leave:
+            self._ok(self.cu.cuMemFreeAsync(spare, None))
+        torch.cuda.synchronize()
+
+    def close(self):
+        torch.cuda.synchronize()
+        for p in self.held:
+            self._ok(self.cu.cuMemFreeAsync(p, None))
+        torch.cuda.synchronize()
+        self._ok(self.cu.cuDeviceSetMemPool(self.dev, self.before))
+        self._ok(self.cu.cuMemPoolDestroy(self.pool))
+
+
+@contextlib.contextmanager
+def pool(size):
+    p = Pool(size)
+    try:
+        yield p
+    finally:
+        p.close()
+
+
+def _resident_task(n, path, **kw):
+    """A task whose outputs lie in device memory: the wide table in device buffers, split and waited for."""
+    rng = np.random.default_rng(n)
+    batches = [W.c2_batch(rng, 4096) for _ in range(n)]
+    w = S.ShuffleSplitterJniWrapper()
+    h = w.make(S.NativePartitioning("hash", 200, None, W.C2_KEYS, list(W.C2_SCHEMA)), dataFile=path,
+               input_kind=S.GZ_INPUT_DEVICE_RETAINED, keep_output_on_device=1, **kw)
+    keep = []
+    for b in batches:
+        t = [torch.from_numpy(x.view(np.uint8).copy()).cuda() if x.nbytes else None for x in b.buffers]
+        keep.append(t)
+        a = np.array([0 if x is None else x.data_ptr() for x in t], np.int64)
+        torch.cuda.synchronize()
+        w.split(h, b.num_rows, a, b.addrs_sizes()[1])
+    w.sync(h)
+    return w, h, batches, keep
+
+
+def test_a_failed_stop_leaves_no_data_in_memory():
+    """Without a data file Stop's bytes are read with gz_split_data: all of them after a Stop that worked, none
+    after one that did not."""
+    with pool(1 << 30) as p:
+        w, h, batches, keep = _resident_task(40, "")
+        p.fill()
+        try:
+            w.stop(h)
+        except S.SplitterError:
+            assert w.data(h) == b""
+        else:
+            assert w.data(h) == O.run_oracle(W.C2_SCHEMA, batches, 200, W.C2_KEYS).data
+        w.close(h)
+        del keep
