@@ -2167,18 +2167,24 @@ Status Splitter::EmitWindows(const std::vector<std::vector<SegMsg>>& msgs, const
   const int64_t img_bytes = std::min(W, total);
   const PinnedBlock up = PinnedAcquire(ub);
   if (!up.ptr) return Status::Error(GZ_OOM, "pinned host memory for the data file's pieces");
-  PinnedBlock bounce;
-  if (!map) {
-    bounce = PinnedAcquire((size_t)img_bytes);
-    if (!bounce.ptr) {
-      PinnedRelease(up);
-      return Status::Error(GZ_OOM, "pinned host memory for the data file");
-    }
-  }
   const size_t img_room = AlignUp((size_t)img_bytes, 256);
   uint8_t* d = nullptr;
   cudaEvent_t built[2] = {nullptr, nullptr}, copied[2] = {nullptr, nullptr};
-  Status st = Cuda(cudaMallocAsync(reinterpret_cast<void**>(&d), ub + 2 * img_room, stream_), "cudaMallocAsync(data file)");
+  cudaError_t got = cudaMallocAsync(reinterpret_cast<void**>(&d), ub + 2 * img_room, stream_);
+  // No device memory to be had: pieces and images stay in pinned host memory, which the device reads and
+  // writes over the link (a task's Stop needs no device memory that the task does not hold)
+  const bool on_host = got == cudaErrorMemoryAllocation;
+  PinnedBlock bounce;
+  if (on_host) {
+    cudaGetLastError();
+    got = cudaSuccess;
+    d = nullptr;
+    bounce = PinnedAcquire(2 * img_room);
+  } else if (!map) {
+    bounce = PinnedAcquire((size_t)img_bytes);
+  }
+  Status st = Cuda(got, "cudaMallocAsync(data file)");
+  if (st.ok() && !bounce.ptr && (on_host || !map)) st = Status::Error(GZ_OOM, "pinned host memory for the data file");
   for (int i = 0; i < 2 && st.ok(); i++) {
     st = Cuda(cudaEventCreateWithFlags(&built[i], cudaEventDisableTiming), "cudaEventCreate");
     if (st.ok()) st = Cuda(cudaEventCreateWithFlags(&copied[i], cudaEventDisableTiming), "cudaEventCreate");
@@ -2186,11 +2192,13 @@ Status Splitter::EmitWindows(const std::vector<std::vector<SegMsg>>& msgs, const
   if (st.ok()) {
     jobs = reinterpret_cast<EmitJob*>(up.ptr);
     blob = up.ptr + jb;
-    d_blob = d + jb;
+    d_blob = (on_host ? up.ptr : d) + jb;
     ParallelFor((size_t)P_, [&](size_t p) { fill((int)p, true); });
-    st = Cuda(cudaMemcpyAsync(d, up.ptr, ub, cudaMemcpyHostToDevice, stream_), "H2D pieces");
+    if (!on_host) st = Cuda(cudaMemcpyAsync(d, up.ptr, ub, cudaMemcpyHostToDevice, stream_), "H2D pieces");
   }
-  uint8_t* img[2] = {d + ub, d + ub + img_room};
+  const EmitJob* const d_jobs = reinterpret_cast<const EmitJob*>(on_host ? up.ptr : d);
+  uint8_t* const img0 = on_host ? bounce.ptr : d + ub;
+  uint8_t* const img[2] = {img0, img0 + img_room};
   const size_t nw = (size_t)((total + W - 1) / W);
   auto first_job = [&](int64_t at) {
     return (size_t)(std::lower_bound(jobs, jobs + nj, (uint64_t)at, [](const EmitJob& j, uint64_t x) { return j.dst < x; }) - jobs);
@@ -2200,7 +2208,7 @@ Status Splitter::EmitWindows(const std::vector<std::vector<SegMsg>>& msgs, const
     if (w >= 2) b = Cuda(cudaStreamWaitEvent(stream_, copied[w & 1], 0), "wait copy");
     if (!b.ok()) return b;
     const size_t j0 = first_job((int64_t)w * W), j1 = first_job((int64_t)(w + 1) * W);
-    b = Cuda(launch_emit(reinterpret_cast<const EmitJob*>(d) + j0, (uint32_t)(j1 - j0), img[w & 1], (uint64_t)w * W, stream_), "k_emit");
+    b = Cuda(launch_emit(d_jobs + j0, (uint32_t)(j1 - j0), img[w & 1], (uint64_t)w * W, stream_), "k_emit");
     return b.ok() ? Cuda(cudaEventRecord(built[w & 1], stream_), "event") : b;
   };
   if (st.ok()) st = build(0);
@@ -2209,15 +2217,21 @@ Status Splitter::EmitWindows(const std::vector<std::vector<SegMsg>>& msgs, const
     const int64_t at = (int64_t)w * W, len = std::min(W, total - at);
     if (st.ok() && ready && !ready(w))
       st = Status::Error(GZ_IO, "cannot write the data file " + data_file_ + ": no space for its bytes");
-    if (st.ok()) st = Cuda(cudaStreamWaitEvent(ostream_, built[w & 1], 0), "wait image");
-    if (st.ok())
-      st = Cuda(cudaMemcpyAsync(map ? map + at : bounce.ptr, img[w & 1], (size_t)len, cudaMemcpyDeviceToHost, ostream_),
-                "data file bytes to host");
-    if (st.ok()) st = Cuda(cudaEventRecord(copied[w & 1], ostream_), "event");
+    const uint8_t* bytes = on_host ? img[w & 1] : bounce.ptr;  // (without a mapping)
+    if (on_host) {
+      if (st.ok()) st = Cuda(cudaEventSynchronize(built[w & 1]), "k_emit");
+      if (st.ok() && map) ParallelCopy({CopyJob{map + at, bytes, (size_t)len}}, (size_t)len);
+    } else {
+      if (st.ok()) st = Cuda(cudaStreamWaitEvent(ostream_, built[w & 1], 0), "wait image");
+      if (st.ok())
+        st = Cuda(cudaMemcpyAsync(map ? map + at : bounce.ptr, img[w & 1], (size_t)len, cudaMemcpyDeviceToHost, ostream_),
+                  "data file bytes to host");
+      if (st.ok()) st = Cuda(cudaEventRecord(copied[w & 1], ostream_), "event");
+      if (st.ok() && !map) st = Cuda(cudaStreamSynchronize(ostream_), "data file bytes to host");
+    }
     if (st.ok() && !map) {
-      st = Cuda(cudaStreamSynchronize(ostream_), "data file bytes to host");
       for (int64_t x = 0; x < len && st.ok();) {
-        const ssize_t r = pwrite(fd, bounce.ptr + x, (size_t)(len - x), at + x);
+        const ssize_t r = pwrite(fd, bytes + x, (size_t)(len - x), at + x);
         if (r > 0) x += r;
         else if (r == 0 || errno != EINTR)
           st = Status::Error(GZ_IO, "writing the data file failed: " + data_file_ + ": " + strerror(r == 0 ? EIO : errno));

@@ -108,3 +108,41 @@ def test_a_failed_stop_leaves_no_data_in_memory():
             assert w.data(h) == O.run_oracle(W.C2_SCHEMA, batches, 200, W.C2_KEYS).data
         w.close(h)
         del keep
+
+
+@pytest.mark.parametrize("n", [40, 120])
+@pytest.mark.parametrize("to_file", [False, True])
+def test_stop_writes_without_device_memory_of_its_own(tmp_path, n, to_file):
+    """Stop writes a task's outputs with no byte of device memory left (files of two windows and of several)."""
+    path = str(tmp_path / "x.data") if to_file else ""
+    with pool(1 << 30) as p:
+        w, h, batches, keep = _resident_task(n, path)
+        p.fill()
+        w.stop(h)
+        data = open(path, "rb").read() if to_file else w.data(h)
+        w.close(h)
+        del keep
+    assert data == O.run_oracle(W.C2_SCHEMA, batches, 200, W.C2_KEYS).data
+
+
+def test_stop_compresses_with_device_memory_for_the_bodies_only(tmp_path):
+    """Under LZ4_FRAME Stop needs device memory for the compressed bodies: with less it says so, with that
+    much and no more (the steps go past it) it writes the bytes of a Stop that has all it wants."""
+    path = str(tmp_path / "x.data")
+    want, states = None, []
+    for leave in [256 << 20] + [x << 20 for x in range(16, 96, 4)]:
+        with pool(1 << 30) as p:
+            w, h, _, keep = _resident_task(60, path, codec="lz4")
+            p.fill(leave)
+            try:
+                w.stop(h)
+                data = open(path, "rb").read()
+                want = want or data
+                assert data == want
+                states.append(True)
+            except S.SplitterError as e:
+                assert e.status == S.GZ_OOM and "partition" not in str(e) and "data file" not in str(e), e
+                states.append(False)
+            w.close(h)
+            del keep
+    assert states[1:] == sorted(states[1:]) and states[0] and states[-1] and not states[1]
