@@ -788,6 +788,16 @@ void lz4_index(const uint8_t* const* src, Lz4Frame* frames, uint32_t n, std::vec
   }
 }
 
+void lz4_index_whole(Lz4Frame* frames, uint32_t n, std::vector<Lz4Slot>* slots) {
+  slots->clear();
+  for (uint32_t k = 0; k < n; k++) {
+    frames[k].slot0 = k;
+    frames[k].n_slots = 1;
+    frames[k].mem0 = 0;
+    slots->push_back(Lz4Slot{0, k, kNoSlot, 0});
+  }
+}
+
 cudaError_t launch_lz4_decode(const Lz4Frame* frames, Lz4Slot* slots, uint32_t n_slots, uint8_t* slot_mem, int32_t* err,
                               cudaStream_t st) {
   if (n_slots == 0) return cudaSuccess;

@@ -72,6 +72,10 @@ inline uint32_t lz4_slot_bytes(uint64_t dst_len) {
 // malformed or has more blocks than slots gets one slot that cannot be decoded on its own.
 void lz4_index(const uint8_t* const* src, Lz4Frame* frames, uint32_t n, std::vector<Lz4Slot>* slots, size_t* mem);
 
+// The same with one slot a frame that cannot be decoded on its own: the frames are decoded whole, without
+// memory for slots (never more slots than lz4_index's).
+void lz4_index_whole(Lz4Frame* frames, uint32_t n, std::vector<Lz4Slot>* slots);
+
 // Decodes every frame; *err gets bit 0 for a malformed frame or a size that differs.  `slots` (n_slots of
 // them, lz4_index's) are written, `slot_mem` is scratch.  The sources' allocations start and end on 16-byte
 // boundaries.

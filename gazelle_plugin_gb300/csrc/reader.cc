@@ -382,8 +382,14 @@ Status PartitionReader::AddStream(const uint8_t* data, int64_t len) {
     uint8_t* slot_mem = nullptr;
     if (st.ok()) {
       arena_mem_.push_back(arena);
-      st = Cuda(cudaMallocAsync(reinterpret_cast<void**>(&slot_mem), std::max<size_t>(slot_bytes, 256), stream_),
-                "cudaMallocAsync(decode)");
+      const cudaError_t got = cudaMallocAsync(reinterpret_cast<void**>(&slot_mem), std::max<size_t>(slot_bytes, 256), stream_);
+      if (got == cudaErrorMemoryAllocation) {  // no room beside image and arena: frames decoded whole, into their place
+        cudaGetLastError();
+        slot_mem = nullptr;
+        lz4_index_whole(jobs.data(), (uint32_t)jobs.size(), &slots);
+      } else {
+        st = Cuda(got, "cudaMallocAsync(decode)");
+      }
     }
     if (!st.ok()) {
       cudaStreamSynchronize(stream_);  // the caller's bytes are being read
@@ -443,7 +449,7 @@ Status PartitionReader::AddStream(const uint8_t* data, int64_t len) {
     if (st.ok() && !direct_)
       st = Cuda(cudaMemcpyAsync(words.data(), out, 4 * words.size(), cudaMemcpyDeviceToHost, stream_), "D2H");
     const Status read = Cuda(cudaStreamSynchronize(stream_), "k_lz4_place");
-    cudaFreeAsync(slot_mem, stream_);
+    if (slot_mem) cudaFreeAsync(slot_mem, stream_);
     if (st.ok()) st = read;
     if (!st.ok()) return st;
     if (words[0]) return Status::Error(GZ_INVALID, "a compressed buffer is not a valid LZ4 frame of its stated length");

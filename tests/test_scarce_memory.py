@@ -146,3 +146,31 @@ def test_stop_compresses_with_device_memory_for_the_bodies_only(tmp_path):
             w.close(h)
             del keep
     assert states[1:] == sorted(states[1:]) and states[0] and states[-1] and not states[1]
+
+
+def test_compressed_streams_are_read_with_memory_for_image_and_columns_only():
+    """A compressed stream needs its image and its decoded buffers; the decoder that takes a block a CTA wants
+    as much again, and without it the frames are decoded the slower way."""
+    rng = np.random.default_rng(3)
+    schema = [W.Field("k", "int64", False)]
+    batches = [W.Batch(n, W._column(rng, schema[0], n, rng.integers(0, 50, size=n), 0.0)) for n in (2_000_000, 2_000_003)]
+    res, data = S.split_batches(schema, batches, 1, [0], codec="lz4")
+    stream = np.frombuffer(data, np.uint8)
+    want = np.concatenate([b.buffers[1].view(np.int64) for b in batches])
+    assert stream.nbytes < want.nbytes // 2
+    read = []
+    # the image, the decoded buffers and their tables, but not as much again; then all that is wanted
+    for leave in (stream.nbytes + want.nbytes * 5 // 4 + (4 << 20), stream.nbytes + want.nbytes * 4):
+        with pool(1 << 30) as p:
+            r = S.PartitionReader(schema)
+            p.fill(leave)
+            r.addStream(stream)
+            for q in p.held:
+                p._ok(p.cu.cuMemFreeAsync(q, None))
+            p.held = []
+            torch.cuda.synchronize()
+            r.finish()
+            read.append(r.column_to_host(0))
+            r.close()
+    for c in read:
+        assert np.array_equal(np.asarray(c[2]).view(np.int64), want)
