@@ -116,9 +116,16 @@ Status PartitionReader::Make(std::vector<Field> fields, int device, std::unique_
   cudaDeviceGetAttribute(&host_tables, cudaDevAttrPageableMemoryAccessUsesHostPageTables, device);
   r->direct_ = pageable != 0 && host_tables != 0;
   if (r->direct_) {
-    st = r->Cuda(cudaMallocAsync(reinterpret_cast<void**>(&r->d_done_), 256, r->stream_), "cudaMallocAsync(reader)");
-    if (st.ok()) st = r->Cuda(cudaMemsetAsync(r->d_done_, 0, 4, r->stream_), "memset(reader)");
-    if (!st.ok()) return st;
+    const cudaError_t got = cudaMallocAsync(reinterpret_cast<void**>(&r->d_done_), 256, r->stream_);
+    if (got == cudaErrorMemoryAllocation) {  // not needed by copies, nor by a reader that gets no rows
+      cudaGetLastError();
+      r->d_done_ = nullptr;
+      r->direct_ = false;
+    } else {
+      st = r->Cuda(got, "cudaMallocAsync(reader)");
+      if (st.ok()) st = r->Cuda(cudaMemsetAsync(r->d_done_, 0, 4, r->stream_), "memset(reader)");
+      if (!st.ok()) return st;
+    }
   }
   r->out_.assign(r->fields_.size(), OutCol());
   *out = std::move(r);
@@ -337,8 +344,16 @@ Status PartitionReader::AddStream(const uint8_t* data, int64_t len) {
   uint8_t* d = nullptr;
   uint8_t* arena = nullptr;
   if (len > 0) {
-    st = Cuda(cudaMallocAsync(reinterpret_cast<void**>(&d), AlignUp((size_t)len, 256), stream_), "cudaMallocAsync(stream)");
-    if (!st.ok()) return st;
+    const Status got =
+        Cuda(cudaMallocAsync(reinterpret_cast<void**>(&d), AlignUp((size_t)len, 256), stream_), "cudaMallocAsync(stream)");
+    if (!got.ok()) {  // a malformed stream, and one without rows, needs none
+      d = nullptr;
+      st = ParseStream(data, len, idx, &bs, &frames, &arena_bytes);
+      if (st.ok() && !bs.empty()) st = got;
+      if (!st.ok()) return st;
+    }
+  }
+  if (d != nullptr) {
     // the caller's bytes are read before the call returns, and while the host parses them: by the
     // device itself where it walks the host page tables, else by a copy
     if (direct_) {

@@ -174,3 +174,35 @@ def test_compressed_streams_are_read_with_memory_for_image_and_columns_only():
             r.close()
     for c in read:
         assert np.array_equal(np.asarray(c[2]).view(np.int64), want)
+
+
+def test_a_reader_without_device_memory_reads_streams_without_rows():
+    """With no byte left a reader is made, takes streams without record batches, reports a malformed one as that
+    and one with rows as out of memory; and reads it once there is memory."""
+    schema = [W.Field("k", "int64", False)]
+    rng = np.random.default_rng(4)
+    batch = W.Batch(5000, W._column(rng, schema[0], 5000, rng.integers(0, 50, size=5000), 0.0))
+    stream = S.split_batches(schema, [batch], 1, [0], writeSchema=True)[1]
+    eos = stream[-8:]
+    schema_only = stream[:8 + int.from_bytes(stream[4:8], "little")] + eos
+
+    def status(r, s):
+        try:
+            r.addStream(np.frombuffer(s, np.uint8))
+        except S.SplitterError as e:
+            return e.status
+        return S.GZ_OK
+
+    with pool(64 << 20) as p:
+        p.fill()
+        r = S.PartitionReader(schema)
+        assert [status(r, s) for s in (schema_only, eos, b"", stream[:-20], b"\1" * 64)] == [S.GZ_OK] * 3 + [S.GZ_INVALID] * 2
+        assert status(r, stream) == S.GZ_OOM
+        for q in p.held:
+            p._ok(p.cu.cuMemFreeAsync(q, None))
+        p.held = []
+        torch.cuda.synchronize()
+        assert status(r, stream) == S.GZ_OK
+        assert r.finish()[0] == 5000
+        assert np.array_equal(np.asarray(r.column_to_host(0)[2]).view(np.int64), batch.buffers[1].view(np.int64))
+        r.close()
