@@ -168,3 +168,69 @@ def test_gpu_large_file_gathered_by_the_cpu_into_a_full_file_system_is_an_io_err
             f"_stop({str(mnt / 'x.data')!r}, 0, 1, n=400, host_budget=1 << 40, localDirs={str(tmp_path)!r})")
     r = subprocess.run(mount + [sys.executable, "-c", call], cwd=ROOT, capture_output=True, text=True, timeout=300)
     assert r.returncode == 0 and "reported" in r.stdout, (r.returncode, r.stdout, r.stderr)
+
+
+SHIM = r"""
+#define _GNU_SOURCE
+#include <dlfcn.h>
+#include <errno.h>
+#include <stdio.h>
+#include <string.h>
+#include <sys/mman.h>
+#include <unistd.h>
+/* no shared mapping of a file named *.data, as of a file system that has none */
+void* mmap(void* a, size_t n, int prot, int flags, int fd, off_t off) {
+  static void* (*next)(void*, size_t, int, int, int, off_t);
+  if (!next) next = (void* (*)(void*, size_t, int, int, int, off_t))dlsym(RTLD_NEXT, "mmap");
+  if (fd >= 0 && (flags & MAP_SHARED) && (prot & PROT_WRITE)) {
+    char link[64], path[512];
+    snprintf(link, sizeof(link), "/proc/self/fd/%d", fd);
+    const ssize_t l = readlink(link, path, sizeof(path));
+    if (l > 5 && memcmp(path + l - 5, ".data", 5) == 0) {
+      fprintf(stderr, "no mapping\n");
+      errno = ENODEV;
+      return MAP_FAILED;
+    }
+  }
+  return next(a, n, prot, flags, fd, off);
+}
+void* mmap64(void* a, size_t n, int prot, int flags, int fd, off_t off) { return mmap(a, n, prot, flags, fd, off); }
+"""
+
+
+def _stop_unmapped(path, n, device, kw):
+    rng = np.random.default_rng(6)
+    batches = [W.c2_batch(rng, 4096) for _ in range(n)]
+    w = S.ShuffleSplitterJniWrapper()
+
+    def task(p):
+        h = w.make(S.NativePartitioning("hash", 200, None, W.C2_KEYS, list(W.C2_SCHEMA)), dataFile=p,
+                   keep_output_on_device=device, **kw)
+        for b in batches:
+            a, z = b.addrs_sizes()
+            w.split(h, b.num_rows, a, z)
+        w.stop(h)
+        data = open(p, "rb").read()
+        w.close(h)
+        return data
+
+    got = task(path + ".data")
+    if "codec" in kw:  # (the compressed bytes are the library's own: those of the mapped path)
+        assert got == task(path + ".mapped")
+    else:
+        assert got == O.run_oracle(W.C2_SCHEMA, batches, 200, W.C2_KEYS).data
+    print("equal")
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n,device,kw", [(9, 0, {}), (61, 1, {}), (61, 0, {"codec": "lz4"}),
+                                         (370, 0, {"host_budget": 1 << 40, "localDirs": "."})])
+def test_gpu_stop_into_a_file_that_cannot_be_mapped(tmp_path, n, device, kw):
+    """Files of two windows and of several with a ragged last one, through a block of host memory and write
+    calls; a large one that the CPU gathers."""
+    (tmp_path / "s.c").write_text(SHIM)
+    subprocess.run(["gcc", "-O1", "-shared", "-fPIC", str(tmp_path / "s.c"), "-o", str(tmp_path / "s.so"), "-ldl"], check=True)
+    call = f"from tests.test_data_file_space import _stop_unmapped as f; f({str(tmp_path / 'x')!r}, {n}, {device}, {kw!r})"
+    r = subprocess.run([sys.executable, "-c", call], cwd=ROOT, capture_output=True, text=True, timeout=300,
+                       env=dict(os.environ, LD_PRELOAD=str(tmp_path / "s.so")))
+    assert r.returncode == 0 and "equal" in r.stdout and "no mapping" in r.stderr, (r.returncode, r.stdout, r.stderr)
