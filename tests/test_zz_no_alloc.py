@@ -283,3 +283,39 @@ def test_static_ids_of_keys_of_one_kind(many_keys, keys, P, off):
         assert got[shift + n] == 0xFFFF
         assert np.array_equal(counts.cpu().numpy(), np.bincount(want_all[:n], minlength=P))
     del hold
+
+
+# Both sides of what the launch is cut by: a sweep of a block's threads (2048 rows of 512 threads up to 2048
+# partitions, 4096 of 1024 above), and the blocks that are resident at once (three an SM, or one: 933,888 and
+# 622,592 rows on 152 SMs), from which on a block takes several sweeps, the next one's first key on its way.
+@pytest.mark.parametrize("P,sizes", [(200, (2047, 2048, 2049, 933_888, 933_889, 1_000_003, 1_900_001)),
+                                     (2049, (4095, 4096, 4097, 622_592, 622_593, 700_001, 1_300_003)),
+                                     (5000, (4097, 800_003))])
+@pytest.mark.parametrize("keys", [[0], [1], [0, 1], [0, 2, 3]])
+def test_static_ids_of_blocks_with_several_sweeps(P, sizes, keys):
+    n = max(sizes)
+    rng = np.random.default_rng(P)
+    schema = [W.Field(f"k{i}", t) for i, t in enumerate(("int64", "int32", "int16", "bool"))]
+    bufs = []
+    for f in schema:
+        bufs += W._column(rng, f, n, rng.integers(0, 2 if f.type == "bool" else 30_000, n), 0.2)
+    want = _oracle_pids(schema, keys, P, W.Batch(n, bufs))
+    for shift in (0, 1):  # columns on their boundaries, and one element off them
+        cols, hold = (GzKeyColumn * len(keys))(), []
+        for j, k in enumerate(keys):
+            w = W.BYTE_WIDTH.get(schema[k].type, 1) * shift
+            t = torch.from_numpy(np.concatenate([np.zeros(w, np.uint8), bufs[2 * k + 1].view(np.uint8)])).cuda()
+            m = torch.from_numpy(bufs[2 * k].view(np.uint8).copy()).cuda()
+            hold += [t, m]
+            cols[j].type, cols[j].values, cols[j].validity = schema[k].code, t.data_ptr() + w, m.data_ptr()
+        for rows in sizes:
+            assert -(-rows // TILE_ROWS) * P <= MAX_COUNTERS
+            out = torch.full((rows + 2,), -1, dtype=torch.int16, device="cuda")
+            counts = torch.full((P,), -1, dtype=torch.int64, device="cuda")
+            st = _entry()(0, P, cols, len(keys), rows, out.data_ptr(), counts.data_ptr(), torch.cuda.current_stream().cuda_stream)
+            assert st == 0, _last_error()
+            got = out.cpu().numpy().view(np.uint16)
+            assert np.array_equal(got[:rows], want[:rows]), (rows, shift)
+            assert (got[rows:] == 0xFFFF).all()
+            assert np.array_equal(counts.cpu().numpy(), np.bincount(want[:rows], minlength=P)), (rows, shift)
+        del hold
