@@ -1349,7 +1349,7 @@ Status Splitter::Drain() {
 // Copies a flush's outputs into a pinned host block and releases the HBM copy (both stream
 // ordered); the host bytes are valid once the stream has reached this point.
 Status Splitter::MoveFlushToHost(FlushRec& f) {
-  if (f.on_host) return Status::OK();
+  if (f.on_host || f.d_out == nullptr) return Status::OK();  // (a Stop has put it in the data file)
   f.h_out = HostAlloc(f.out_bytes);
   if (!f.h_out) return Status::Error(GZ_OOM, "pinned host memory for partition data");
   // on its own stream, after the pass's kernels, so the copy overlaps the next pass

@@ -120,3 +120,32 @@ def test_emit_rewrites_a_longer_file_and_reports_a_bad_path(tmp_path):
         _run_null.split(h, b.num_rows, a, z)
     assert int(_run_null.stop(h).partitionLengths.sum()) == len(data)
     _run_null.close(h)
+
+
+@pytest.mark.parametrize("codec", ["uncompressed", "lz4"])
+@pytest.mark.parametrize("device", [False, True])
+def test_spill_after_stop(tmp_path, device, codec):
+    """A memory manager may ask a task that has stopped to spill: the policy's bytes, as of a task whose file the
+    host gathers, and nothing is moved any more."""
+    schema, keys, batches = _batches("c2", 40)
+    got = []
+    for kw in ({}, dict(host_budget=1 << 40, localDirs=str(tmp_path))):
+        w = S.ShuffleSplitterJniWrapper()
+        h = w.make(S.NativePartitioning("hash", 200, None, keys, list(schema)), dataFile=str(tmp_path / "x.data"), codec=codec,
+                   bufferSize=64, preferSpill=False, input_kind=S.GZ_INPUT_DEVICE_RETAINED if device else S.GZ_INPUT_HOST, **kw)
+        keep = []
+        for b in batches:
+            a, z = b.addrs_sizes()
+            if device:
+                t = [torch.from_numpy(x.view(np.uint8).copy()).cuda() if x.nbytes else None for x in b.buffers]
+                keep.append(t)
+                a = np.array([0 if x is None else x.data_ptr() for x in t], np.int64)
+                torch.cuda.synchronize()
+            w.split(h, b.num_rows, a, z)
+        w.stop(h)
+        moved = w.stats(h)[3]
+        got.append([w.nativeSpill(h, 1 << 40), w.nativeSpill(h, 1)])
+        assert w.stats(h)[3] == moved or kw
+        w.sync(h)
+        w.close(h)
+    assert got[0] == got[1] and got[0][0] > 0
