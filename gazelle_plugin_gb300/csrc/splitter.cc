@@ -2436,8 +2436,11 @@ void Splitter::ReleaseStaging() {
 Status Splitter::SpillFixedSize(int64_t size, int64_t* actual) {
   *actual = 0;
   if (opts_.prefer_spill) return Status::OK();  // every emitted batch was spilled already
-  // cached batches exist only without prefer_spill: make them visible on the host
-  Status st = Drain();
+  // cached batches exist only without prefer_spill: make them visible on the host.  (A memory manager calls
+  // from a thread of its own, with any device current)
+  Status st = Cuda(cudaSetDevice(device_), "cudaSetDevice");
+  if (!st.ok()) return st;
+  st = Drain();
   if (!st.ok()) return st;
   st = SyncAndCheck();
   if (!st.ok()) return st;
@@ -2602,7 +2605,9 @@ Status Splitter::CompressedSize(int32_t num_rows, const int64_t* addrs, const in
 }
 
 Status Splitter::LastPids(uint16_t* out, int32_t n) {
-  Status st = Drain();
+  Status st = Cuda(cudaSetDevice(device_), "cudaSetDevice");
+  if (!st.ok()) return st;
+  st = Drain();
   if (!st.ok()) return st;
   st = SyncAndCheck();
   if (!st.ok()) return st;
@@ -2655,7 +2660,9 @@ Status SyncGroup(const std::vector<Splitter*>& tasks, int* failed) {
 }
 
 Status Splitter::KernelTimes(double* out4) {
-  Status st = SyncAndCheck();
+  Status st = Cuda(cudaSetDevice(device_), "cudaSetDevice");
+  if (!st.ok()) return st;
+  st = SyncAndCheck();
   if (!st.ok()) return st;
   for (int i = 0; i < 4; i++) out4[i] = kernel_ms_[i];
   return Status::OK();

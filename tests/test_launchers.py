@@ -12,6 +12,8 @@ from gazelle_plugin_gb300 import build as B
 RUNTIME = r"""
 #include <cuda_runtime.h>
 #include <stdio.h>
+#include <stdlib.h>
+#include <string.h>
 #include <map>
 #include <string>
 #include <utility>
@@ -21,7 +23,10 @@ static std::vector<std::string> g_calls;
 static cudaError_t g_last = cudaSuccess;
 static std::map<std::pair<int, const void*>, int> g_limit;
 static struct { dim3 g, b; size_t sm; cudaStream_t st; } g_cfg;
-static cudaError_t launch(const void* f, size_t sm) {
+struct Owned { int dev; };  // a stream or an event
+static cudaError_t fail() { return g_last = cudaErrorInvalidResourceHandle; }
+static cudaError_t launch(const void* f, size_t sm, cudaStream_t st) {
+  if (st && ((Owned*)st)->dev != g_dev) return fail();
   auto it = g_limit.find({g_dev, f});
   if (sm > (size_t)(it == g_limit.end() ? 48 * 1024 : it->second)) return g_last = cudaErrorInvalidValue;
   g_launched[g_dev]++;
@@ -40,8 +45,12 @@ cudaError_t __cudaPopCallConfiguration(dim3* g, dim3* b, size_t* sm, void* st) {
   *g = g_cfg.g; *b = g_cfg.b; *sm = g_cfg.sm; *(cudaStream_t*)st = g_cfg.st;
   return cudaSuccess;
 }
-cudaError_t __cudaLaunchKernel(cudaKernel_t k, dim3, dim3, void**, size_t sm, cudaStream_t) { return launch((const void*)k, sm); }
-cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t* c, const void* f, void**) { return launch(f, c->dynamicSmemBytes); }
+cudaError_t __cudaLaunchKernel(cudaKernel_t k, dim3, dim3, void**, size_t sm, cudaStream_t st) {
+  return launch((const void*)k, sm, st);
+}
+cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t* c, const void* f, void**) {
+  return launch(f, c->dynamicSmemBytes, c->stream);
+}
 cudaError_t cudaGetLastError() { cudaError_t e = g_last; g_last = cudaSuccess; return e; }
 cudaError_t cudaPeekAtLastError() { return g_last; }
 const char* cudaGetErrorString(cudaError_t) { return "an error"; }
@@ -58,6 +67,31 @@ cudaError_t cudaFuncSetAttribute(const void* f, cudaFuncAttribute a, int v) {
   }
   return cudaSuccess;
 }
+// memory is the heap's, copies happen at once, kernels do nothing
+static cudaError_t make(void* out) { *(Owned**)out = new Owned{g_dev}; return cudaSuccess; }
+cudaError_t cudaStreamCreateWithFlags(cudaStream_t* s, unsigned) { return make(s); }
+cudaError_t cudaStreamCreateWithPriority(cudaStream_t* s, unsigned, int) { return make(s); }
+cudaError_t cudaStreamDestroy(cudaStream_t) { return cudaSuccess; }
+cudaError_t cudaStreamSynchronize(cudaStream_t) { return cudaSuccess; }
+cudaError_t cudaStreamQuery(cudaStream_t) { return cudaSuccess; }
+cudaError_t cudaStreamWaitEvent(cudaStream_t, cudaEvent_t, unsigned) { return cudaSuccess; }
+cudaError_t cudaEventCreate(cudaEvent_t* e) { return make(e); }
+cudaError_t cudaEventCreateWithFlags(cudaEvent_t* e, unsigned) { return make(e); }
+cudaError_t cudaEventDestroy(cudaEvent_t) { return cudaSuccess; }
+cudaError_t cudaEventElapsedTime(float* ms, cudaEvent_t, cudaEvent_t) { *ms = 0; return cudaSuccess; }
+cudaError_t cudaEventRecord(cudaEvent_t e, cudaStream_t s) { return ((Owned*)e)->dev == ((Owned*)s)->dev ? cudaSuccess : fail(); }
+cudaError_t cudaEventSynchronize(cudaEvent_t) { return cudaSuccess; }
+cudaError_t cudaDeviceGetDefaultMemPool(cudaMemPool_t*, int) { return cudaErrorNotSupported; }
+cudaError_t cudaMemPoolSetAttribute(cudaMemPool_t, cudaMemPoolAttr, void*) { return cudaSuccess; }
+cudaError_t cudaDeviceGetStreamPriorityRange(int* least, int* greatest) { *least = 0; *greatest = -5; return cudaSuccess; }
+cudaError_t cudaMalloc(void** p, size_t n) { *p = calloc(1, n); return cudaSuccess; }
+cudaError_t cudaMallocAsync(void** p, size_t n, cudaStream_t) { *p = calloc(1, n); return cudaSuccess; }
+cudaError_t cudaHostAlloc(void** p, size_t n, unsigned) { *p = calloc(1, n); return cudaSuccess; }
+cudaError_t cudaFree(void* p) { free(p); return cudaSuccess; }
+cudaError_t cudaFreeAsync(void* p, cudaStream_t) { free(p); return cudaSuccess; }
+cudaError_t cudaMemcpy(void* d, const void* s, size_t n, cudaMemcpyKind) { memcpy(d, s, n); return cudaSuccess; }
+cudaError_t cudaMemcpyAsync(void* d, const void* s, size_t n, cudaMemcpyKind, cudaStream_t) { memcpy(d, s, n); return cudaSuccess; }
+cudaError_t cudaMemsetAsync(void* d, int v, size_t n, cudaStream_t) { memset(d, v, n); return cudaSuccess; }
 }
 """
 
@@ -145,4 +179,39 @@ def test_partition_ids_make_the_device_s_primary_context_current(tmp_path):
       check(!g_calls.empty() && g_calls[0] == "device " + std::to_string(dev), "its device is made current first");
       check(g_dev == 0, "the caller's device is current again");
     }
+""")
+
+
+def test_calls_of_a_thread_on_another_device_use_the_task_s(tmp_path):
+    """A memory manager's thread asks a task of device 1 to spill with device 0 current; so does a thread that
+    reads the task's ids and times.  Streams, events and launches are the task's device's, and so is what later
+    tasks take over from it."""
+    _run(str(tmp_path), [s for s in B.SOURCES], r"""
+  GzField field{};
+  field.type = GZ_TYPE_INT64;
+  field.name = "k";
+  GzSplitOptions o;
+  gz_split_default_options(&o);
+  o.device = 1;
+  o.prefer_spill = 0;
+  const int32_t key = 0;
+  int64_t values[10] = {};
+  const int64_t addrs[2] = {0, (int64_t)values}, sizes[2] = {0, (int64_t)sizeof(values)};
+  for (int what = 0; what < 6; what++) {
+    int64_t h = 0, n = 0;
+    uint16_t ids[10];
+    double times[4];
+    check(gz_split_make_fields("hash", 4, &field, 1, &key, 1, &o, &h) == GZ_OK, "make");
+    check(gz_split_split(h, 10, addrs, sizes, 2, 0, &n) == GZ_OK, "split");
+    g_dev = 0;
+    GzStatus st = GZ_OK;
+    if (what % 3 == 0) st = gz_split_spill(h, 1 << 20, &n);
+    if (what % 3 == 1) st = gz_split_last_pids(h, ids, 10);
+    if (what % 3 == 2) st = gz_split_kernel_times(h, times);
+    if (st != GZ_OK) printf("call %d: %d\n", what % 3, (int)st);
+    check(st == GZ_OK, "a call of a thread with another device current");
+    check(gz_split_sync(h) == GZ_OK, "sync");
+    check(gz_split_close(h) == GZ_OK, "close");
+  }
+  check(cudaGetLastError() == cudaSuccess, "an error left behind");
 """)
