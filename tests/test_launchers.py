@@ -18,19 +18,19 @@ RUNTIME = r"""
 #include <string>
 #include <utility>
 #include <vector>
+static char g_primary[2], g_other;            // contexts: the devices' primary ones, one of the driver API's own
+static char* g_ctx = &g_primary[0];
 static int g_dev = 0, g_lowered = 0, g_launched[2] = {0, 0};
-static std::vector<std::string> g_calls;
 static cudaError_t g_last = cudaSuccess;
 static std::map<std::pair<int, const void*>, int> g_limit;
 static struct { dim3 g, b; size_t sm; cudaStream_t st; } g_cfg;
 struct Owned { int dev; };  // a stream or an event
 static cudaError_t fail() { return g_last = cudaErrorInvalidResourceHandle; }
 static cudaError_t launch(const void* f, size_t sm, cudaStream_t st) {
-  if (st && ((Owned*)st)->dev != g_dev) return fail();
+  if ((st && ((Owned*)st)->dev != g_dev) || g_ctx != &g_primary[g_dev]) return fail();
   auto it = g_limit.find({g_dev, f});
   if (sm > (size_t)(it == g_limit.end() ? 48 * 1024 : it->second)) return g_last = cudaErrorInvalidValue;
   g_launched[g_dev]++;
-  g_calls.push_back("launch");
   return cudaSuccess;
 }
 extern "C" {
@@ -55,10 +55,16 @@ cudaError_t cudaGetLastError() { cudaError_t e = g_last; g_last = cudaSuccess; r
 cudaError_t cudaPeekAtLastError() { return g_last; }
 const char* cudaGetErrorString(cudaError_t) { return "an error"; }
 cudaError_t cudaGetDevice(int* d) { *d = g_dev; return cudaSuccess; }
-cudaError_t cudaSetDevice(int d) { g_dev = d; g_calls.push_back("device " + std::to_string(d)); return cudaSuccess; }
+cudaError_t cudaSetDevice(int d) { g_dev = d; g_ctx = &g_primary[d]; return cudaSuccess; }
 cudaError_t cudaDeviceGetAttribute(int* v, cudaDeviceAttr, int d) { *v = d == 0 ? 152 : 100; return cudaSuccess; }
 cudaError_t cudaFuncGetAttributes(cudaFuncAttributes*, const void*) { return cudaSuccess; }
-cudaError_t cudaGetSymbolAddress(void** p, const void*) { static char mem[256]; *p = mem; g_calls.push_back("symbol"); return cudaSuccess; }
+cudaError_t cudaGetSymbolAddress(void** p, const void*) { static char mem[256]; *p = mem; return g_ctx == &g_primary[g_dev] ? cudaSuccess : fail(); }
+static int current(void** c) { *c = g_ctx; return 0; }
+cudaError_t cudaGetDriverEntryPointByVersion(const char*, void** f, unsigned, unsigned long long, cudaDriverEntryPointQueryResult* r) {
+  *f = (void*)current;
+  *r = cudaDriverEntryPointSuccess;
+  return cudaSuccess;
+}
 cudaError_t cudaFuncSetAttribute(const void* f, cudaFuncAttribute a, int v) {
   if (a == cudaFuncAttributeMaxDynamicSharedMemorySize) {
     int& have = g_limit[{g_dev, f}];
@@ -161,8 +167,8 @@ def test_every_device_allows_the_shared_memory_of_its_launches(tmp_path):
 
 
 def test_partition_ids_make_the_device_s_primary_context_current(tmp_path):
-    """cudaSetDevice before anything that belongs to a context, on every call and also when the device is
-    current already: a context of the driver API's own may be."""
+    """Also when the device is current already: a context of the driver API's own may be, in which neither the
+    scratch array nor the kernels are at hand."""
     _run(str(tmp_path), ["hash_static.cu"], r"""
   int64_t counts[8];
   uint16_t ids[8];
@@ -171,14 +177,16 @@ def test_partition_ids_make_the_device_s_primary_context_current(tmp_path):
   key.type = GZ_TYPE_INT32;
   key.values = reinterpret_cast<const uint8_t*>(values);
   std::string msg;
+  int launches = 0;
   for (int call = 0; call < 2; call++)
-    for (int dev = 0; dev < 2; dev++) {
-      g_dev = 0;
-      g_calls.clear();
-      check(gz::HashPartitionStatic(dev, 8, &key, 1, 8, ids, counts, 0, &msg) == GZ_OK, "the call");
-      check(!g_calls.empty() && g_calls[0] == "device " + std::to_string(dev), "its device is made current first");
-      check(g_dev == 0, "the caller's device is current again");
-    }
+    for (int dev = 0; dev < 2; dev++)
+      for (int own = 0; own < 2; own++) {
+        cudaSetDevice(0);
+        if (own) g_ctx = &g_other;
+        check(gz::HashPartitionStatic(dev, 8, &key, 1, 8, ids, counts, 0, &msg) == GZ_OK, "the call");
+        check(g_launched[0] + g_launched[1] == (launches += 2), "its launches");
+        check(g_dev == 0, "the caller's device is current again");
+      }
 """)
 
 
@@ -203,7 +211,7 @@ def test_calls_of_a_thread_on_another_device_use_the_task_s(tmp_path):
     double times[4];
     check(gz_split_make_fields("hash", 4, &field, 1, &key, 1, &o, &h) == GZ_OK, "make");
     check(gz_split_split(h, 10, addrs, sizes, 2, 0, &n) == GZ_OK, "split");
-    g_dev = 0;
+    cudaSetDevice(0);
     GzStatus st = GZ_OK;
     if (what % 3 == 0) st = gz_split_spill(h, 1 << 20, &n);
     if (what % 3 == 1) st = gz_split_last_pids(h, ids, 10);
