@@ -1,7 +1,7 @@
 // sm_103a kernels of the reduce-side read (PartitionReader): the record batches of a partition's
 // IPC streams, already in HBM, concatenated into one set of Arrow columns.  Three job lists, each
-// job at most 64 KB so that one CTA per job keeps every SM busy:
-//   byte jobs   values of fixed-width columns and characters of binary columns, copied
+// job small enough that one CTA per job keeps every SM busy:
+//   byte jobs   (64 KB) values of fixed-width columns and characters of binary columns, copied
 //   offset jobs binary offsets (int32, or int64 of the large types) rebased:
 //               out[i] = in[i] - in[0] + (the batch's first character)
 //   bit jobs    validity / bool bits moved to their row in the output (OR into zeroed words;

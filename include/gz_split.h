@@ -394,8 +394,8 @@ GzStatus gz_reader_make_fields(const GzField* fields, int32_t n_fields, int32_t 
 
 /* Adds one IPC stream of the partition (host bytes: a map output's partition_lengths[p] bytes of
  * its data file, with or without the schema message in front, ending with the end-of-stream
- * marker); the bytes are read before the call returns.  Compressed bodies return
- * GZ_NOT_IMPLEMENTED. */
+ * marker); the bytes are read before the call returns.  Bodies may be compressed with LZ4_FRAME (each buffer its
+ * length and one frame); other codecs return GZ_NOT_IMPLEMENTED. */
 GzStatus gz_reader_add_stream(int64_t handle, const uint8_t* stream, int64_t len);
 
 /* Concatenates the record batches of every stream added, in order, into device columns and

@@ -183,8 +183,8 @@ def many_keys():
     return schema, batch, pids
 
 
-# both sides of every line of the dispatch: rows of one cluster block, of a cluster, of two launches;
-# histograms of 512- and 1024-thread blocks, of one block per SM, in the scratch
+# both sides of the lines of the dispatch by partitions (histograms of blocks of 512 and of 1024 threads, histograms
+# counted in the scratch), over rows around the 1024 of the limit on a call and their multiples
 @pytest.mark.parametrize("P", [1, 8, 2048, 2049, 12288, 12289, 24577, 57344, 57345])
 @pytest.mark.parametrize("shift", [0, 1])
 def test_static_ids_and_counts_over_sizes(many_keys, P, shift):
